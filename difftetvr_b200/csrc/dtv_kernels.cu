@@ -1222,16 +1222,37 @@ void launch_scatter_grads(const float4* grad_rows, uint32_t V, float* grad_pos, 
 // L2 loss and its image adjoint (Data/Shaders/Optimizer/Loss.glsl:242-248;
 // torch.nn.MSELoss in pytests/train.py:321-326): adjoint = 2 * scale * (x - y),
 // loss += scale * sum (x - y)^2.
-__global__ void __launch_bounds__(256) k_loss_l2(const float* __restrict__ img, const float* __restrict__ tgt,
+// 16-byte loads and stores, two blocks per SM: memory bound (at 1024^2 48 MB,
+// L2-resident behind the composite).  Few blocks also mean few additions into
+// the loss: with 2,368 of them the FP32 sum's own rounding was the largest
+// error of the loss (up to 3e-6 relative); the per-thread sums of a few
+// hundred squares carry theirs along (two_sum).
+__global__ void __launch_bounds__(512) k_loss_l2(const float* __restrict__ img, const float* __restrict__ tgt,
                                                  uint64_t n, float scale, float* __restrict__ adj,
-                                                 float* __restrict__ loss) {
-    __shared__ float sm[8];
-    float acc = 0.f;
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
+                                                 float* __restrict__ loss, bool vec) {
+    __shared__ float sm[16];
+    float acc = 0.f, err = 0.f;
+    auto add = [&](float q) {
+        const F2 t = two_sum(acc, q);
+        acc = t.hi;
+        err += t.lo;
+    };
+    const uint64_t first = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x, stride = uint64_t(gridDim.x) * blockDim.x;
+    const uint64_t n4 = vec ? n / 4 : 0;
+    for (uint64_t i = first; i < n4; i += stride) {
+        const float4 a = reinterpret_cast<const float4*>(img)[i], b = reinterpret_cast<const float4*>(tgt)[i];
+        const float4 d = make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w);
+        if (adj)
+            reinterpret_cast<float4*>(adj)[i] =
+                make_float4(2.f * scale * d.x, 2.f * scale * d.y, 2.f * scale * d.z, 2.f * scale * d.w);
+        add((d.x * d.x + d.y * d.y) + (d.z * d.z + d.w * d.w));
+    }
+    for (uint64_t i = 4 * n4 + first; i < n; i += stride) {
         const float d = img[i] - tgt[i];
         if (adj) adj[i] = 2.f * scale * d;
-        acc += d * d;
+        add(d * d);
     }
+    acc += err;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
@@ -1247,9 +1268,11 @@ __global__ void __launch_bounds__(256) k_loss_l2(const float* __restrict__ img, 
 void launch_loss_l2(const float* image, const float* target, uint64_t n, float scale, float* adjoint,
                     float* loss_accum, cudaStream_t s) {
     if (n == 0) return;
-    uint64_t blocks = (n + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    k_loss_l2<<<unsigned(blocks), 256, 0, s>>>(image, target, n, scale, adjoint, loss_accum);
+    const bool vec = ((reinterpret_cast<uintptr_t>(image) | reinterpret_cast<uintptr_t>(target) |
+                       reinterpret_cast<uintptr_t>(adjoint)) & 15u) == 0;
+    uint64_t blocks = ((vec ? (n + 3) / 4 : n) + 511) / 512;
+    if (blocks > 148 * 2) blocks = 148 * 2;
+    k_loss_l2<<<unsigned(blocks), 512, 0, s>>>(image, target, n, scale, adjoint, loss_accum, vec);
 }
 
 // ---------------------------------------------------------------------------
