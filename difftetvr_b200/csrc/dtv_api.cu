@@ -69,6 +69,13 @@ struct dtv_mesh {
     uint4* d_bfaces = nullptr;         // Nb
     uint32_t* d_bf_global = nullptr;   // Nb
     std::vector<uint32_t> bf_global;   // host copy
+    // Tables of the list walk; `walkable`: the topology can be walked and at
+    // most three quarters of the faces are boundary faces (else the lists are
+    // filled by the rasteriser and sorted: with unconnected tets every face is
+    // the start or end of a chain of its own).
+    uint4* d_walk_links = nullptr;
+    uint4* d_walk_start = nullptr;
+    bool walkable = false;
 };
 
 struct dtv_renderer {
@@ -88,6 +95,8 @@ struct dtv_renderer {
     // fragment budget (each band's lists are rebuilt by the adjoint); empty
     // when the lists are stored whole.
     std::vector<std::pair<int, int>> bands;
+    bool band_walk = false;       // the bands' lists are walked
+    bool clipped_view = false;    // the last projection clipped a vertex
     bool cells = false;           // last render used per-cell colours
     dtv_tuning tuning{0, 0, dtv::kSortSurrogateDefault, dtv::kSortBucketDefault};
     u64* h_rowoff = nullptr;      // pinned row-start offsets (H+1)
@@ -96,7 +105,12 @@ struct dtv_renderer {
     DevBuf<uint32_t> band_scratch;  // band counts and cursors of fill_order
     DevBuf<uint32_t> wide_list;     // [0] = n, then the faces of the 64-bit raster path (count -> fill)
     DevBuf<uint4> wstate;         // ray-tet path: (last tet, its entry face, boundary entry index, segments)
-    u64* h_nf = nullptr;          // pinned
+    DevBuf<dtv::WalkVertRow> walk_verts;  // per-view vertex rows of the list walk
+    DevBuf<dtv::ListInfo> info;   // record total and redo counters of the lists
+    DevBuf<uint32_t> clipped;     // [0]: the projection met a vertex it does not project
+    cudaEvent_t ev_info = nullptr;  // the record total is on the host
+    DevBuf<uint32_t> redo;        // pixels the walk left to the rasteriser
+    dtv::ListInfo* h_info = nullptr;  // pinned
     // State of the last render.
     bool have_render = false;
     const dtv_mesh* mesh = nullptr;
@@ -111,6 +125,10 @@ struct dtv_renderer {
 };
 
 namespace {
+
+dtv::WalkMesh walk_mesh(const dtv_mesh* m) {
+    return dtv::WalkMesh{m->d_walk_links, m->d_walk_start, m->d_bfaces};
+}
 
 void rec_event(dtv_renderer* r, int idx, cudaStream_t s) {
     if (r->timing) DTV_CK(cudaEventRecord(r->ev[idx], s));
@@ -148,14 +166,73 @@ uint64_t plan_bands(dtv_renderer* r, int W, int H, uint64_t cap, cudaStream_t s)
     return largest;
 }
 
+// Lists of rows [y0, y1) by walking the mesh (guarded: nothing happens unless
+// the scan found that the records fit).  The boundary fragments of a pixel go
+// to the end of its range; the walk starts from them.
+void walk_rows(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& cam, int y0, int y1, bool guarded,
+               cudaStream_t s) {
+    dtv::launch_raster_fill(mesh->d_bfaces, uint32_t(mesh->bf_global.size()), r->vproj.ptr, r->vfix.ptr, cam.W, cam.H,
+                            r->counts.ptr, r->offsets.ptr, r->records.ptr, s, y0, y1, nullptr, nullptr,
+                            guarded ? &r->info.ptr->ok : nullptr);
+    check_launch("boundary fill");
+    dtv::launch_walk_lists(walk_mesh(mesh), r->offsets.ptr, r->records.ptr, r->counts.ptr, r->walk_verts.ptr, cam.W,
+                           y0, y1, r->info.ptr, r->redo.ptr, guarded, s);
+    check_launch("list walk");
+}
+
+// The pixels the walk left: lists filled by the rasteriser and sorted.  Few of
+// them (no vertex clipped) take kernels over fixed grids that return at once
+// when there are none, so the host does not wait to know; clipped vertices cut
+// many pixels' chains, which takes the rasteriser's own passes (fill_order
+// must be there).
+void rest_rows(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& cam, int y0, int y1, bool few,
+               cudaStream_t s) {
+    const uint32_t F = uint32_t(mesh->host.num_faces);
+    if (few) {
+        dtv::launch_rest_fill(r->info.ptr, mesh->d_faces, F, r->vproj.ptr, r->vfix.ptr, cam.W, y0, y1, r->counts.ptr,
+                              r->offsets.ptr, r->records.ptr, s);
+        dtv::launch_rest_sort(r->info.ptr, true, r->redo.ptr, r->offsets.ptr, r->records.ptr, s);
+    } else {
+        dtv::launch_raster_fill(mesh->d_faces, F, r->vproj.ptr, r->vfix.ptr, cam.W, cam.H, r->counts.ptr,
+                                r->offsets.ptr, r->records.ptr, s, y0, y1, r->fill_order.ptr, r->wide_list.ptr,
+                                nullptr, /*rest=*/true);
+        dtv::launch_sort(r->offsets.ptr, r->records.ptr, uint32_t(y1 - y0) * uint32_t(cam.W), r->long_list.ptr, s,
+                         nullptr, r->tuning.sort_surrogate_classes, r->tuning.sort_bucket_classes, r->redo.ptr,
+                         &r->info.ptr->n_redo);
+    }
+    check_launch("rest of the lists");
+}
+
+// Composite of rows [y0, y1) with the stored lists: per-vertex colours
+// (d_colors f32[4V]) or per-cell colours (f32[4T]).
+void composite_rows(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors, const dtv::CamDev& cam,
+                    const dtv::ShadeDev& sh, float* d_image, int y0, int y1, cudaStream_t s,
+                    const uint32_t* gate = nullptr) {
+    if (r->cells)
+        dtv::launch_composite_cells(r->offsets.ptr, r->records.ptr, mesh->d_faces, mesh->d_face_to_tet, r->vgeo.ptr,
+                                    reinterpret_cast<const float4*>(d_colors), cam.W, cam.H, sh,
+                                    reinterpret_cast<float4*>(d_image), r->tfinal.ptr, r->term.ptr, s, y0, y1, gate);
+    else
+        dtv::launch_composite(r->offsets.ptr, r->records.ptr, mesh->d_faces, r->vgeo.ptr,
+                              reinterpret_cast<const float4*>(d_colors), cam.W, cam.H, sh,
+                              reinterpret_cast<float4*>(d_image), r->tfinal.ptr, r->term.ptr, s, y0, y1,
+                              r->tuning.composite_tile, gate);
+}
+
 // Builds the sorted lists of rows [y0, y1) into the records buffer (band-local
-// offsets): scan of the band's counts, fill (faces in the render's fill_order),
-// per-pixel sort.  The band's counts must hold the rasterised counts; the fill
-// leaves them zero.
-void build_band_lists(dtv_renderer* r, const dtv_mesh* mesh, int W, int H, int y0, int y1, cudaStream_t s) {
+// offsets): scan of the band's counts, then the walk and what it leaves, or
+// fill (faces in the render's fill_order) and per-pixel sort.  The band's
+// counts must hold the rasterised counts; they end at zero.
+void build_band_lists(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& cam, int y0, int y1, cudaStream_t s) {
+    const int W = cam.W, H = cam.H;
     const uint64_t p0 = uint64_t(y0) * W, pb = uint64_t(y1 - y0) * W;
-    dtv::launch_scan(r->counts.ptr + p0, pb, r->offsets.ptr + p0, r->scan_scratch.ptr, s);
+    dtv::launch_scan(r->counts.ptr + p0, pb, r->offsets.ptr + p0, r->scan_scratch.ptr, s, r->info.ptr);
     check_launch("band scan");
+    if (r->band_walk) {
+        walk_rows(r, mesh, cam, y0, y1, false, s);
+        rest_rows(r, mesh, cam, y0, y1, !r->clipped_view, s);
+        return;
+    }
     dtv::launch_raster_fill(mesh->d_faces, uint32_t(mesh->host.num_faces), r->vproj.ptr, r->vfix.ptr, W, H,
                             r->counts.ptr, r->offsets.ptr, r->records.ptr, s, y0, y1, r->fill_order.ptr,
                             r->wide_list.ptr);
@@ -163,21 +240,6 @@ void build_band_lists(dtv_renderer* r, const dtv_mesh* mesh, int W, int H, int y
     dtv::launch_sort(r->offsets.ptr + p0, r->records.ptr, uint32_t(pb), r->long_list.ptr, s, nullptr,
                      r->tuning.sort_surrogate_classes, r->tuning.sort_bucket_classes);
     check_launch("band sort");
-}
-
-// Composite of rows [y0, y1) with the stored lists: per-vertex colours
-// (d_colors f32[4V]) or per-cell colours (f32[4T]).
-void composite_rows(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors, const dtv::CamDev& cam,
-                    const dtv::ShadeDev& sh, float* d_image, int y0, int y1, cudaStream_t s) {
-    if (r->cells)
-        dtv::launch_composite_cells(r->offsets.ptr, r->records.ptr, mesh->d_faces, mesh->d_face_to_tet, r->vgeo.ptr,
-                                    reinterpret_cast<const float4*>(d_colors), cam.W, cam.H, sh,
-                                    reinterpret_cast<float4*>(d_image), r->tfinal.ptr, r->term.ptr, s, y0, y1);
-    else
-        dtv::launch_composite(r->offsets.ptr, r->records.ptr, mesh->d_faces, r->vgeo.ptr,
-                              reinterpret_cast<const float4*>(d_colors), cam.W, cam.H, sh,
-                              reinterpret_cast<float4*>(d_image), r->tfinal.ptr, r->term.ptr, s, y0, y1,
-                              r->tuning.composite_tile);
 }
 
 // Adjoint of rows [y0, y1) into the gradient rows (per-cell: the cell colour
@@ -227,7 +289,7 @@ void render_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors,
     }
     rec_event(r, 3, s);
     for (const auto& b : r->bands) {
-        build_band_lists(r, mesh, W, H, b.first, b.second, s);
+        build_band_lists(r, mesh, cam, b.first, b.second, s);
         composite_rows(r, mesh, d_colors, cam, sh, d_image, b.first, b.second, s);
         check_launch("band composite");
     }
@@ -248,7 +310,7 @@ void adjoint_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors
         dtv::launch_raster_count(mesh->d_faces, uint32_t(mesh->host.num_faces), r->vproj.ptr, r->vfix.ptr, W, H,
                                  r->counts.ptr, s, b.first, b.second, r->wide_list.ptr);
         check_launch("band count");
-        build_band_lists(r, mesh, W, H, b.first, b.second, s);
+        build_band_lists(r, mesh, r->cam, b.first, b.second, s);
         adjoint_rows(r, mesh, d_colors, d_image_adjoint, sh, b.first, b.second, d_grad_colors, s);
         check_launch("band adjoint");
     }
@@ -338,8 +400,27 @@ int32_t dtv_mesh_create(const uint32_t* h_cells, uint64_t num_cells, uint64_t nu
             if (num_vertices)
                 DTV_CK(cudaMemcpy(m->d_vertex_boundary, m->host.vertex_boundary.data(),
                                   sizeof(uint32_t) * num_vertices, cudaMemcpyHostToDevice));
-            if (num_cells)
+            if (num_cells) {
                 DTV_CK(cudaMemcpy(m->d_cells, h_cells, sizeof(uint32_t) * 4 * num_cells, cudaMemcpyHostToDevice));
+                DTV_CK(cudaMalloc(&m->d_walk_links, sizeof(uint4) * 4 * num_cells));
+                DTV_CK(cudaMalloc(&m->d_walk_start, sizeof(uint4) * (Nb ? Nb : 1)));
+                DevBuf<uint32_t> bad;
+                uint32_t h_bad = 1;
+                try {
+                    bad.ensure(1, nullptr, /*zero_new=*/true);
+                    dtv::launch_build_walk(reinterpret_cast<const uint4*>(m->d_cells), uint32_t(num_cells),
+                                           reinterpret_cast<const uint4*>(m->d_tet_faces), m->d_faces,
+                                           reinterpret_cast<const uint2*>(m->d_face_to_tet), m->d_bf_global,
+                                           uint32_t(Nb), m->d_walk_links, m->d_walk_start, bad.ptr, nullptr);
+                    check_launch("walk tables");
+                    DTV_CK(cudaMemcpy(&h_bad, bad.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+                } catch (...) {
+                    bad.release();
+                    throw;
+                }
+                bad.release();
+                m->walkable = h_bad == 0 && 4 * Nb <= 3 * F;
+            }
         } catch (...) {
             dtv_mesh_destroy(m);
             throw;
@@ -358,6 +439,8 @@ int32_t dtv_mesh_destroy(dtv_mesh* m) {
     cudaFree(m->d_tet_flip);
     cudaFree(m->d_bfaces);
     cudaFree(m->d_bf_global);
+    cudaFree(m->d_walk_links);
+    cudaFree(m->d_walk_start);
     delete m;
     return DTV_OK;
 }
@@ -398,8 +481,9 @@ int32_t dtv_renderer_create(int32_t type, dtv_renderer** out) {
         auto* r = new dtv_renderer();
         r->type = type;
         try {
-            DTV_CK(cudaMallocHost(&r->h_nf, sizeof(u64)));
+            DTV_CK(cudaMallocHost(&r->h_info, sizeof(dtv::ListInfo)));
             for (auto& e : r->ev) DTV_CK(cudaEventCreate(&e));
+            DTV_CK(cudaEventCreateWithFlags(&r->ev_info, cudaEventDisableTiming));
         } catch (...) {
             dtv_renderer_destroy(r);
             throw;
@@ -426,7 +510,12 @@ int32_t dtv_renderer_destroy(dtv_renderer* r) {
     r->fill_order.release();
     r->band_scratch.release();
     r->wide_list.release();
-    if (r->h_nf) cudaFreeHost(r->h_nf);
+    r->info.release();
+    r->redo.release();
+    r->clipped.release();
+    if (r->ev_info) cudaEventDestroy(r->ev_info);
+    r->walk_verts.release();
+    if (r->h_info) cudaFreeHost(r->h_info);
     if (r->h_rowoff) cudaFreeHost(r->h_rowoff);
     for (auto& e : r->ev)
         if (e) cudaEventDestroy(e);
@@ -481,7 +570,14 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         r->long_list.ensure(dtv::sort_scratch_elems(P), s);
 
         rec_event(r, 0, s);
-        dtv::launch_project(d_positions, uint32_t(V), cam, r->vproj.ptr, r->vfix.ptr, r->vgeo.ptr, s);
+        const bool walk = !raytet && mesh->walkable;
+        if (walk) {
+            r->walk_verts.ensure(V ? V : 1, s);
+            r->clipped.ensure(1, s, /*zero_new=*/true);
+            r->redo.ensure(P, s);
+        }
+        dtv::launch_project(d_positions, uint32_t(V), cam, r->vproj.ptr, r->vfix.ptr, r->vgeo.ptr, s,
+                            walk ? r->walk_verts.ptr : nullptr, walk ? r->clipped.ptr : nullptr);
         check_launch("project");
         rec_event(r, 1, s);
         r->wide_list.ensure(size_t(F) + 1, s);
@@ -489,12 +585,40 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
                                  r->wide_list.ptr);
         check_launch("raster count");
         rec_event(r, 2, s);
-        dtv::launch_scan(r->counts.ptr, P, r->offsets.ptr, r->scan_scratch.ptr, s);
-        check_launch("scan");
-        DTV_CK(cudaMemcpyAsync(r->h_nf, r->offsets.ptr + P, sizeof(u64), cudaMemcpyDeviceToHost, s));
-        DTV_CK(cudaStreamSynchronize(s));
-        const uint64_t nf = *r->h_nf;
         const uint64_t budget = params->fragment_budget_bytes;
+        r->info.ensure(1, s);
+        // The walk and the composite are enqueued before the host knows the
+        // record total: they run if the records fit what is allocated already
+        // (and the budget).  The host waits for the total only.
+        const uint64_t room = std::min<uint64_t>(r->records.cap, budget ? budget / sizeof(u64) : ~0ull);
+        dtv::launch_scan(r->counts.ptr, P, r->offsets.ptr, r->scan_scratch.ptr, s, r->info.ptr, room,
+                         walk ? r->clipped.ptr : nullptr);
+        check_launch("scan");
+        DTV_CK(cudaMemcpyAsync(r->h_info, r->info.ptr, sizeof(dtv::ListInfo), cudaMemcpyDeviceToHost, s));
+        DTV_CK(cudaEventRecord(r->ev_info, s));
+        // Lists by the walk (few left), then the composite; events of the
+        // fill, sort and composite stages.
+        auto lists_and_composite = [&](bool guarded) {
+            rec_event(r, 3, s);
+            walk_rows(r, mesh, cam, 0, H, guarded, s);
+            rec_event(r, 4, s);
+            rest_rows(r, mesh, cam, 0, H, /*few=*/true, s);
+            rec_event(r, 5, s);
+            composite_rows(r, mesh, d_colors, cam, sh, d_image, 0, H, s, &r->info.ptr->whole);
+            check_launch("composite");
+        };
+        const bool early = walk && r->records.ptr;
+        if (early) lists_and_composite(true);
+        DTV_CK(cudaEventSynchronize(r->ev_info));
+        const uint64_t nf = r->h_info->nf;
+        const bool walked = early && r->h_info->ok != 0u, clipped = walk && r->h_info->clipped != 0u;
+        r->clipped_view = clipped;
+        // Faces in row-band order for the fill of whole lists.
+        auto order_faces = [&] {
+            r->fill_order.ensure(size_t(F), s);
+            r->band_scratch.ensure(2 * dtv::kFillBands, s);
+            dtv::launch_fill_order(rfaces, uint32_t(F), r->vfix.ptr, H, nf, r->fill_order.ptr, r->band_scratch.ptr, s);
+        };
         r->bands.clear();
         if (budget && nf * sizeof(u64) > budget) {
             if (params->over_budget != DTV_OVER_BUDGET_RECOMPUTE || raytet) {
@@ -505,10 +629,8 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
                                                    " bytes), over the budget of " + std::to_string(budget) +
                                                    " bytes");
             }
-            r->fill_order.ensure(size_t(F), s);
-            r->band_scratch.ensure(2 * dtv::kFillBands, s);
-            dtv::launch_fill_order(rfaces, uint32_t(F), r->vfix.ptr, H, nf, r->fill_order.ptr, r->band_scratch.ptr,
-                                   s);
+            r->band_walk = walk;
+            if (!walk || clipped) order_faces();
             render_banded(r, mesh, d_colors, cam, sh, d_image, budget / sizeof(u64), s);
             r->adjoint_timed = false;
             r->have_render = true;
@@ -520,24 +642,40 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
             r->nf = nf;
             return;
         }
-        try {
-            r->records.ensure(nf ? nf : 1, s, false, 1.25);
-        } catch (...) {
-            cudaMemsetAsync(r->counts.ptr, 0, P * sizeof(uint32_t), s);
-            throw;
+        if (!walked) {
+            try {
+                r->records.ensure(nf ? nf : 1, s, false, 1.25);
+            } catch (...) {
+                cudaMemsetAsync(r->counts.ptr, 0, P * sizeof(uint32_t), s);
+                throw;
+            }
+            if (walk) {
+                // The flags of the scan were taken against the old capacity.
+                r->h_info->ok = 1u;
+                r->h_info->whole = clipped ? 0u : 1u;
+                DTV_CK(cudaMemcpyAsync(r->info.ptr, r->h_info, sizeof(dtv::ListInfo), cudaMemcpyHostToDevice, s));
+                lists_and_composite(false);
+            }
         }
-        rec_event(r, 3, s);
-        r->fill_order.ensure(size_t(F), s);
-        r->band_scratch.ensure(2 * dtv::kFillBands, s);
-        dtv::launch_fill_order(rfaces, uint32_t(F), r->vfix.ptr, H, nf, r->fill_order.ptr, r->band_scratch.ptr, s);
-        dtv::launch_raster_fill(rfaces, uint32_t(F), r->vproj.ptr, r->vfix.ptr, W, H, r->counts.ptr,
-                                r->offsets.ptr, r->records.ptr, s, 0, -1, r->fill_order.ptr, r->wide_list.ptr);
-        check_launch("raster fill");
-        rec_event(r, 4, s);
-        dtv::launch_sort(r->offsets.ptr, r->records.ptr, uint32_t(P), r->long_list.ptr, s, nullptr,
-                         r->tuning.sort_surrogate_classes, r->tuning.sort_bucket_classes);
-        check_launch("sort");
-        rec_event(r, 5, s);
+        if (walk && clipped) {
+            order_faces();
+            rest_rows(r, mesh, cam, 0, H, /*few=*/false, s);
+            rec_event(r, 5, s);
+            composite_rows(r, mesh, d_colors, cam, sh, d_image, 0, H, s);
+            check_launch("composite");
+        }
+        if (!walk) {
+            rec_event(r, 3, s);
+            order_faces();
+            dtv::launch_raster_fill(rfaces, uint32_t(F), r->vproj.ptr, r->vfix.ptr, W, H, r->counts.ptr,
+                                    r->offsets.ptr, r->records.ptr, s, 0, -1, r->fill_order.ptr, r->wide_list.ptr);
+            check_launch("raster fill");
+            rec_event(r, 4, s);
+            dtv::launch_sort(r->offsets.ptr, r->records.ptr, uint32_t(P), r->long_list.ptr, s, nullptr,
+                             r->tuning.sort_surrogate_classes, r->tuning.sort_bucket_classes);
+            check_launch("sort");
+            rec_event(r, 5, s);
+        }
         if (raytet) {
             dtv::launch_walk_composite(r->offsets.ptr, r->records.ptr, mesh->d_bf_global, mesh->d_faces,
                                        mesh->d_face_to_tet, mesh->d_tet_faces, mesh->d_cells, mesh->d_tet_flip,
@@ -545,7 +683,7 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
                                        r->vfix.ptr, r->vgeo.ptr, reinterpret_cast<const float4*>(d_colors), cam, sh,
                                        reinterpret_cast<float4*>(d_image), r->tfinal.ptr, r->wstate.ptr, s);
             check_launch("ray-tet walk");
-        } else {
+        } else if (!walk) {
             composite_rows(r, mesh, d_colors, cam, sh, d_image, 0, H, s);
             check_launch("composite");
         }
@@ -770,7 +908,10 @@ int32_t dtv_adam_step(float* d_param, const float* d_grad, float* d_m, float* d_
 
 // Helpers for the allocation-free entry point (dtv_noalloc.cu).
 namespace dtv {
-MeshView mesh_view(const dtv_mesh* m) { return MeshView{m->d_faces, m->host.num_faces, m->host.num_vertices}; }
+MeshView mesh_view(const dtv_mesh* m) {
+    return MeshView{m->d_faces, m->host.num_faces, m->host.num_vertices, m->walkable ? walk_mesh(m) : WalkMesh{},
+                    uint32_t(m->bf_global.size())};
+}
 uint64_t mesh_num_cells(const dtv_mesh* m) { return m->host.num_cells; }
 const uint32_t* mesh_cells_device(const dtv_mesh* m) { return m->d_cells; }
 CamDev camera_constants(const dtv_camera& c) { return make_cam(c); }

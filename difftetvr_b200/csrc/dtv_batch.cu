@@ -29,6 +29,7 @@
 #include "dtv_host.h"
 #include "dtv_internal.h"
 #include "dtv_path.cuh"
+#include "dtv_walk.cuh"
 
 namespace dtv {
 
@@ -40,8 +41,9 @@ struct BatchView {
     float4* image;
     float4* dimage;            // image adjoint: read by the adjoint, written by the fused loss
     const float4* target;      // fused-loss target (nullable)
-    u64 vert_base, face_base, pix_base, tile_base, grad_base;
-    uint32_t V, F, W, H, tiles_x;
+    WalkMesh walk;             // walk tables of the mesh (null when it cannot be walked)
+    u64 vert_base, face_base, bface_base, pix_base, tile_base, grad_base;
+    uint32_t V, F, Nb, W, H, tiles_x;
     int32_t grad_slot;         // -1: no gradient for this view
     float loss_scale;          // 1 / (W * H * 4)  (torch.nn.MSELoss, mean)
 };
@@ -87,7 +89,8 @@ __device__ __forceinline__ int view_of_item(u64 g, u64 block_first, int n, Gette
 
 __global__ void __launch_bounds__(256) kb_project(const BatchView* __restrict__ views, int nviews, u64 total,
                                                   float4* __restrict__ vproj, int2* __restrict__ vfix,
-                                                  VGeo* __restrict__ vgeo) {
+                                                  VGeo* __restrict__ vgeo, WalkVertRow* __restrict__ rows,
+                                                  uint32_t* __restrict__ clipped) {
     const u64 first = u64(blockIdx.x) * blockDim.x;
     const u64 g = first + threadIdx.x;
     if (g < total) {
@@ -96,9 +99,13 @@ __global__ void __launch_bounds__(256) kb_project(const BatchView* __restrict__ 
         const u64 k = g - bv.vert_base;
         const float x = bv.positions[3 * k], y = bv.positions[3 * k + 1], z = bv.positions[3 * k + 2];
         int2 fx;
-        vproj[g] = project_vertex(bv.cam, x, y, z, fx);
+        const float4 pr = project_vertex(bv.cam, x, y, z, fx);
+        const VGeo ge = project_vertex_geo(bv.cam, x, y, z, fx);
+        vproj[g] = pr;
         vfix[g] = fx;
-        vgeo[g] = project_vertex_geo(bv.cam, x, y, z, fx);
+        vgeo[g] = ge;
+        if (rows) rows[g] = walk_row(pr, ge);
+        if (clipped && fx.x == kInvalidFix) *clipped = 1u;
     }
 }
 
@@ -162,26 +169,37 @@ __global__ void __launch_bounds__(256) kb_band_scatter(const BatchView* __restri
     if (g < total) order[base[band] + rank] = uint32_t(g);
 }
 
-template <bool FILL, bool WIDE>
+// Count or fill of every view's faces (kAllFaces), the fill of its boundary
+// faces (kBoundaryFaces: record face field = boundary face index), or the fill
+// of the pixels the walk left to the rasteriser (kRestFaces; see fill_pixels).
+// `ok`: the fill does nothing when *ok is zero.
+enum FaceSet { kAllFaces = 0, kBoundaryFaces = 1, kRestFaces = 2 };
+template <bool FILL, bool WIDE, int kSet = kAllFaces>
 __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ views, int nviews, u64 total,
                                                  const float4* __restrict__ vproj, const int2* __restrict__ vfix,
                                                  uint32_t* __restrict__ counts, const u64* __restrict__ offsets,
                                                  u64* __restrict__ records, const uint32_t* __restrict__ ok,
                                                  const uint32_t* __restrict__ order,
-                                                 uint32_t* __restrict__ wide_list) {
+                                                 uint32_t* __restrict__ wide_list, uint32_t per_warp) {
     if (FILL && !batch_ok(ok)) return;
     const u64 first = u64(blockIdx.x) * blockDim.x;
-    const u64 i = first + threadIdx.x;
+    u64 i = first + threadIdx.x;
+    bool mine = true;
+    if (FILL && per_warp != 32u) {
+        const uint32_t l = threadIdx.x & 31u;
+        i = (i >> 5) * per_warp + l;
+        mine = l < per_warp;
+    }
     bool set = false, live = false;
     RasterJob J;
     u64 g = 0;
-    if (i < total) {
+    if (mine && i < total) {
         g = order ? u64(order[i]) : i;
-        const int v = order ? find_index(g, nviews, [&](int k) { return views[k].face_base; })
-                            : view_of_item(g, first, nviews, [&](int k) { return views[k].face_base; });
+        auto base = [&](int k) { return kSet == kBoundaryFaces ? views[k].bface_base : views[k].face_base; };
+        const int v = (FILL || order) ? find_index(g, nviews, base) : view_of_item(g, first, nviews, base);
         const BatchView& bv = views[v];
-        set = raster_setup(uint32_t(g - bv.face_base), bv.faces, vfix + bv.vert_base, uint32_t(bv.vert_base),
-                           int(bv.W), 0, int(bv.H), bv.pix_base, J);
+        set = raster_setup(uint32_t(g - base(v)), kSet == kBoundaryFaces ? bv.walk.bfaces : bv.faces,
+                           vfix + bv.vert_base, uint32_t(bv.vert_base), int(bv.W), 0, int(bv.H), bv.pix_base, J);
         live = set && (J.wide != 0) == WIDE;
     }
     if constexpr (!FILL) {
@@ -203,13 +221,14 @@ __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ v
         __shared__ RasterJob jobs[4][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         if (live) jobs[w][lane] = J;
-        raster_warp<FILL, WIDE>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets, records);
+        raster_warp<FILL, WIDE, kSet == kRestFaces>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts,
+                                                    offsets, records);
     }
 }
 
 // The 64-bit items listed by the count (wide_list), 32 per warp and step over
 // a fixed grid: the count (one thread per face) or the fill (raster_warp).
-template <bool FILL>
+template <bool FILL, bool REST = false>
 __global__ void __launch_bounds__(128) kb_raster_listed(const BatchView* __restrict__ views, int nviews,
                                                         const float4* __restrict__ vproj,
                                                         const int2* __restrict__ vfix,
@@ -238,10 +257,40 @@ __global__ void __launch_bounds__(128) kb_raster_listed(const BatchView* __restr
             if (live) count_face<long long>(J, counts);
         } else {
             if (live) jobs[w][lane] = J;
-            raster_warp<FILL, true>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets,
-                                    records);
+            raster_warp<FILL, true, REST>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets,
+                                          records);
             __syncwarp();  // every lane is done with this step's jobs before the next step writes them
         }
+    }
+}
+
+// Fill of the few pixels the walk left to the rasteriser (k_rest_fill).
+__global__ void __launch_bounds__(128) kb_rest_fill(const BatchView* __restrict__ views, int nviews, u64 total,
+                                                    const ListInfo* __restrict__ info,
+                                                    const float4* __restrict__ vproj, const int2* __restrict__ vfix,
+                                                    uint32_t* __restrict__ counts, const u64* __restrict__ offsets,
+                                                    u64* __restrict__ records) {
+    if (info->n_redo == 0u) return;
+    __shared__ RasterJob jobs[4][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const u64 stride = u64(gridDim.x) * blockDim.x;
+    for (u64 base = u64(blockIdx.x) * blockDim.x + u64(w) * 32u; base < total; base += stride) {
+        const u64 g = base + u64(lane);
+        RasterJob J;
+        bool live = false;
+        if (g < total) {
+            const int v = find_index(g, nviews, [&](int k) { return views[k].face_base; });
+            const BatchView& bv = views[v];
+            live = raster_setup(uint32_t(g - bv.face_base), bv.faces, vfix + bv.vert_base, uint32_t(bv.vert_base),
+                                int(bv.W), 0, int(bv.H), bv.pix_base, J);
+        }
+        const bool wide = live && J.wide != 0;
+        if (live) jobs[w][lane] = J;
+        raster_warp<true, false, true>(jobs[w], __ballot_sync(0xffffffffu, live && !wide), lane, vproj, counts,
+                                       offsets, records);
+        raster_warp<true, true, true>(jobs[w], __ballot_sync(0xffffffffu, wide), lane, vproj, counts, offsets,
+                                      records);
+        __syncwarp();  // every lane is done with this step's jobs before the next step writes them
     }
 }
 
@@ -251,14 +300,6 @@ __global__ void __launch_bounds__(256) kb_row_prefix(const BatchView* __restrict
     const BatchView& bv = views[blockIdx.y];
     const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row < bv.H) row_prefix_warp(counts + bv.pix_base + size_t(row) * bv.W, int(bv.W), threadIdx.x & 31);
-}
-
-// ok = (records fit the buffer); *total_out = number of records.
-__global__ void kb_check_capacity(const u64* __restrict__ offsets_end, u64 capacity, uint32_t* __restrict__ ok,
-                                  u64* __restrict__ total_out) {
-    const u64 total = *offsets_end;
-    *ok = total <= capacity ? 1u : 0u;
-    *total_out = total;
 }
 
 // On overflow the fill does not run, so clear the counters it would have consumed.
@@ -290,6 +331,31 @@ __global__ void __launch_bounds__(kTile * kTile) kb_composite(const BatchView* _
     const BatchView& bv = views[v];
     composite_pixel(px, py, int(bv.W), offsets + bv.pix_base, records, bv.faces, vgeo + bv.vert_base, bv.colors, sh,
                     bv.image, tfinal + bv.pix_base, term + bv.pix_base);
+}
+
+// Lists of every view by walking its mesh (walk_pixel), in blocks of 16 x 8
+// pixels (half a tile, four warps of 8 x 4 pixels).
+constexpr int kWalkBatchThreads = 128;
+__global__ void __launch_bounds__(kWalkBatchThreads) kb_walk_lists(
+    const BatchView* __restrict__ views, int nviews, const u64* __restrict__ offsets, u64* __restrict__ records,
+    uint32_t* __restrict__ counts, const WalkVertRow* __restrict__ verts, ListInfo* __restrict__ info,
+    uint32_t* __restrict__ redo) {
+    constexpr int N = kWalkBatchThreads;
+    __shared__ u64 starts[kWalkStarts * N];
+    __shared__ u64 recs[4 * N];
+    if (info->ok == 0u) return;
+    const u64 tile = blockIdx.x >> 1;
+    const int v = find_index(tile, nviews, [&](int i) { return views[i].tile_base; });
+    const BatchView& bv = views[v];
+    const uint32_t tl = uint32_t(tile - bv.tile_base);
+    const int lane = int(threadIdx.x & 31u), w = int(threadIdx.x >> 5);
+    const int px = int(tl % bv.tiles_x) * kTile + (w & 1) * 8 + lane % 8;
+    const int py = int(tl / bv.tiles_x) * kTile + int(blockIdx.x & 1u) * 8 + (w >> 1) * 4 + lane / 8;
+    if (px >= int(bv.W) || py >= int(bv.H)) return;
+    const size_t p = size_t(py) * bv.W + px;
+    walk_pixel(px, py, p, offsets + bv.pix_base, records, counts + bv.pix_base, bv.walk, verts + bv.vert_base,
+               WalkSmem{starts + threadIdx.x, recs + threadIdx.x, N}, WalkRedo{&info->n_redo, redo},
+               uint32_t(bv.pix_base + p));
 }
 
 // Fused L2 loss of every view with a target: dimage = 2 s (image - target),
@@ -479,6 +545,8 @@ struct dtv_batch {
         float* col = nullptr;
         uint64_t V = 0, F = 0;
         const uint4* faces = nullptr;
+        dtv::WalkMesh walk{};        // links null: the mesh cannot be walked
+        uint32_t Nb = 0;
         const uint32_t* boundary = nullptr;
         // training state (allocated on the first train step)
         DevBuf<float> m_pos, v_pos;
@@ -502,8 +570,14 @@ struct dtv_batch {
     DevBuf<float> tfinal;
     DevBuf<uint32_t> term;
     DevBuf<uint32_t> long_list;
-    DevBuf<uint32_t> ok;
-    DevBuf<u64> total;
+    DevBuf<dtv::ListInfo> info;     // record total, whether it fits, pixels the walk left
+    DevBuf<uint32_t> redo;          // those pixels
+    DevBuf<uint32_t> clipped;       // [0]: the projection met a vertex it does not project
+    // The last batch had clipped vertices: they cut many pixels' chains, so
+    // the next batch's left-over pixels take the passes for many pixels.  The
+    // results do not depend on it.
+    bool many_left = false;
+    DevBuf<dtv::WalkVertRow> walk_verts;
     DevBuf<float4> grad_rows;
     DevBuf<uint32_t> fill_order;    // items (view faces) in row-band order for the fill
     DevBuf<uint32_t> band_scratch;  // band counts and cursors of fill_order
@@ -512,11 +586,11 @@ struct dtv_batch {
     DevBuf<float4> dimage_internal;
     DevBuf<float> loss;
     DevBuf<int> step;
-    uint32_t* h_ok = nullptr;        // pinned
-    u64* h_total = nullptr;
+    dtv::ListInfo* h_info = nullptr;  // pinned
     // shapes of the last render (for the adjoint)
     int nviews = 0;
-    u64 tot_verts = 0, tot_faces = 0, tot_pixels = 0, tot_tiles = 0, tot_rows = 0;
+    u64 tot_verts = 0, tot_faces = 0, tot_bfaces = 0, tot_pixels = 0, tot_tiles = 0, tot_rows = 0;
+    bool walk = false;        // every view's mesh can be walked
     uint32_t max_height = 0;  // tallest view (grid of the count's row prefix)
     dtv::ShadeDev sh{};
     bool have_render = false;
@@ -547,7 +621,8 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
     require(nviews > 0, "need at least one view");
     ensure_pinned(reinterpret_cast<void**>(&b->h_views), b->h_views_cap, sizeof(BatchView) * size_t(nviews));
     if (b->staging_free) DTV_CK(cudaEventSynchronize(b->staging_free));
-    u64 vb = 0, fb = 0, pb = 0, tb = 0;
+    u64 vb = 0, fb = 0, bb = 0, pb = 0, tb = 0;
+    bool walk = true;
     for (int i = 0; i < nviews; ++i) {
         const dtv_batch_view& in = views[i];
         require(in.mesh >= 0 && in.mesh < int(b->meshes.size()), "view mesh index out of range");
@@ -568,6 +643,11 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
         bv.dimage = reinterpret_cast<float4*>(in.d_image_adjoint);
         bv.V = uint32_t(me.V);
         bv.F = uint32_t(me.F);
+        bv.walk = me.walk;
+        bv.Nb = me.Nb;
+        bv.bface_base = bb;
+        bb += me.Nb;
+        walk = walk && me.walk.links != nullptr;
         bv.W = uint32_t(c.width);
         bv.H = uint32_t(c.height);
         bv.tiles_x = uint32_t((c.width + dtv::kTile - 1) / dtv::kTile);
@@ -589,6 +669,8 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
     b->nviews = nviews;
     b->tot_verts = vb;
     b->tot_faces = fb;
+    b->tot_bfaces = bb;
+    b->walk = walk;
     b->tot_pixels = pb;
     b->tot_tiles = tb;
     uint32_t mh = 0;
@@ -611,12 +693,15 @@ void ensure_scratch(dtv_batch* b, cudaStream_t s) {
     b->tfinal.ensure(b->tot_pixels, s);
     b->term.ensure(b->tot_pixels, s);
     b->long_list.ensure(dtv::sort_scratch_elems(b->tot_pixels), s);
-    b->ok.ensure(1, s);
-    b->total.ensure(1, s);
+    b->info.ensure(1, s);
+    b->clipped.ensure(1, s, /*zero_new=*/true);
+    if (b->walk) {
+        b->walk_verts.ensure(b->tot_verts ? b->tot_verts : 1, s);
+        b->redo.ensure(b->tot_pixels, s);
+    }
     b->loss.ensure(1, s);
-    if (!b->h_ok) {
-        DTV_CK(cudaMallocHost(&b->h_ok, sizeof(uint32_t)));
-        DTV_CK(cudaMallocHost(&b->h_total, sizeof(u64)));
+    if (!b->h_info) {
+        DTV_CK(cudaMallocHost(&b->h_info, sizeof(dtv::ListInfo)));
         DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
     }
 }
@@ -627,15 +712,30 @@ void upload_views(dtv_batch* b, cudaStream_t s) {
     DTV_CK(cudaEventRecord(b->staging_free, s));
 }
 
-// Count (FILL false) or fill pass over every view's faces: the 32-bit faces,
-// then the 64-bit ones (kb_raster); the count's difference arrays are then
-// summed along each view's rows (kb_row_prefix).
-template <bool FILL>
-void launch_kb_raster(dtv_batch* b, const uint32_t* okp, cudaStream_t s) {
+// Count pass over every view's faces: the 32-bit faces, then the 64-bit ones,
+// which the first kernel lists; the count's difference arrays are then summed
+// along each view's rows (kb_row_prefix).
+void launch_kb_count(dtv_batch* b, cudaStream_t s) {
+    using namespace dtv;
+    const unsigned blocks = grid_for(b->tot_faces, 128, 0x7fffffffu);
+    DTV_CK(cudaMemsetAsync(b->wide_list.ptr, 0, sizeof(uint32_t), s));
+    kb_raster<false, false><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr, b->vfix.ptr,
+                                                   b->counts.ptr, nullptr, nullptr, nullptr, nullptr,
+                                                   b->wide_list.ptr, 32u);
+    kb_raster_listed<false><<<148, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
+                                                nullptr, nullptr, nullptr, b->wide_list.ptr);
+    dim3 grid(unsigned(b->max_height + 7) / 8, unsigned(b->nviews));
+    kb_row_prefix<<<grid, 256, 0, s>>>(b->d_views.ptr, b->counts.ptr);
+}
+
+// Fill pass over every view's faces in row-band order (kRestFaces: of the
+// pixels the walk left).
+template <int kSet>
+void launch_kb_fill(dtv_batch* b, const uint32_t* okp, cudaStream_t s) {
     using namespace dtv;
     const unsigned blocks = grid_for(b->tot_faces, 128, 0x7fffffffu);
     const uint32_t* order = nullptr;
-    if (FILL && b->tot_faces) {
+    if (b->tot_faces) {
         const unsigned ob = grid_for(b->tot_faces, 256, 0x7fffffffu);
         DTV_CK(cudaMemsetAsync(b->band_scratch.ptr, 0, kFillBands * sizeof(uint32_t), s));
         kb_band_count<<<ob, 256, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vfix.ptr, b->offsets.ptr,
@@ -645,20 +745,54 @@ void launch_kb_raster(dtv_batch* b, const uint32_t* okp, cudaStream_t s) {
                                            b->tot_pixels, b->band_scratch.ptr + kFillBands, b->fill_order.ptr);
         order = b->fill_order.ptr;
     }
-    // The count lists the 64-bit items; the 64-bit count and the fill that
-    // follows walk that list instead of setting up every item again.
-    if (!FILL) DTV_CK(cudaMemsetAsync(b->wide_list.ptr, 0, sizeof(uint32_t), s));
-    kb_raster<FILL, false><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr,
-                                                  b->vfix.ptr, b->counts.ptr, FILL ? b->offsets.ptr : nullptr,
-                                                  FILL ? b->records.ptr : nullptr, okp, order,
-                                                  FILL ? nullptr : b->wide_list.ptr);
-    kb_raster_listed<FILL><<<148, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
-                                               FILL ? b->offsets.ptr : nullptr, FILL ? b->records.ptr : nullptr, okp,
-                                               b->wide_list.ptr);
-    if (!FILL) {
-        dim3 grid(unsigned(b->max_height + 7) / 8, unsigned(b->nviews));
-        kb_row_prefix<<<grid, 256, 0, s>>>(b->d_views.ptr, b->counts.ptr);
+    kb_raster<true, false, kSet><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr,
+                                                  b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr, okp, order, nullptr,
+                                                  32u);
+    kb_raster_listed<true, kSet == kRestFaces><<<148, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
+                                               b->offsets.ptr, b->records.ptr, okp, b->wide_list.ptr);
+}
+
+// Lists and composite of every view after the scan.  Meshes that can be
+// walked: the boundary fragments to the end of each pixel's range, the walk,
+// then fill and sort of the pixels it left (kernels that return at once when
+// there are none); otherwise fill and sort of all.
+void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaStream_t s) {
+    using namespace dtv;
+    const uint32_t* okp = guarded ? &b->info.ptr->ok : nullptr;
+    if (b->walk) {
+        if (b->tot_bfaces) {
+            // Few faces are spread over more warps (as launch_raster_fill).
+            const uint32_t per_warp = uint32_t(std::min<u64>(32, std::max<u64>(1, b->tot_bfaces / (148 * 32))));
+            const unsigned bb = grid_for(b->tot_bfaces, 4 * per_warp, 0x7fffffffu);
+            kb_raster<true, false, kBoundaryFaces><<<bb, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_bfaces,
+                                                                      b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
+                                                                      b->offsets.ptr, b->records.ptr, okp, nullptr,
+                                                                      nullptr, per_warp);
+            kb_raster<true, true, kBoundaryFaces><<<bb, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_bfaces,
+                                                                     b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
+                                                                     b->offsets.ptr, b->records.ptr, okp, nullptr,
+                                                                     nullptr, per_warp);
+        }
+        kb_walk_lists<<<unsigned(2 * b->tot_tiles), kWalkBatchThreads, 0, s>>>(
+            b->d_views.ptr, b->nviews, b->offsets.ptr, b->records.ptr, b->counts.ptr, b->walk_verts.ptr, b->info.ptr,
+            b->redo.ptr);
+        if (b->many_left) {
+            launch_kb_fill<kRestFaces>(b, okp, s);
+            launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, okp,
+                        b->sort_surrogate_classes, b->sort_bucket_classes, b->redo.ptr, &b->info.ptr->n_redo);
+        } else {
+            kb_rest_fill<<<148 * 6, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->info.ptr, b->vproj.ptr,
+                                                 b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr);
+            launch_rest_sort(b->info.ptr, false, b->redo.ptr, b->offsets.ptr, b->records.ptr, s);
+        }
+    } else {
+        launch_kb_fill<kAllFaces>(b, okp, s);
+        launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, okp,
+                    b->sort_surrogate_classes, b->sort_bucket_classes);
     }
+    kb_composite<<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(b->d_views.ptr, b->nviews, b->offsets.ptr,
+                                                                  b->records.ptr, b->vgeo.ptr, sh, b->tfinal.ptr,
+                                                                  b->term.ptr, okp);
 }
 
 // Adjoint of every view with a gradient slot into the slots' rows (which the
@@ -680,25 +814,26 @@ void enqueue_adjoint(dtv_batch* b, const dtv::ShadeDev& sh, const uint32_t* okp,
         b->d_views.ptr, b->nviews, b->tot_verts, b->vgeo.ptr, b->view_rows.ptr, b->grad_rows.ptr, okp);
 }
 
-// Enqueues project, count, scan, [capacity guard], fill, sort, composite.
-// With `guarded`, kernels after the scan run only if the records fit.
-void enqueue_forward(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaStream_t s) {
+// Enqueues project, count and scan; info gets the record total and whether it
+// is at most `capacity`.
+void enqueue_count(dtv_batch* b, u64 capacity, cudaStream_t s) {
     using namespace dtv;
-    const uint32_t* okp = guarded ? b->ok.ptr : nullptr;
     kb_project<<<grid_for(b->tot_verts, 256, 0x7fffffffu), 256, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_verts,
-                                                                        b->vproj.ptr, b->vfix.ptr, b->vgeo.ptr);
-    launch_kb_raster<false>(b, nullptr, s);
-    launch_scan(b->counts.ptr, b->tot_pixels, b->offsets.ptr, b->scan.ptr, s);
-    if (guarded) {
-        kb_check_capacity<<<1, 1, 0, s>>>(b->offsets.ptr + b->tot_pixels, b->capacity, b->ok.ptr, b->total.ptr);
-        kb_clear_counts<<<grid_for(b->tot_pixels, 256, 148 * 16), 256, 0, s>>>(b->counts.ptr, b->tot_pixels, okp);
-    }
-    launch_kb_raster<true>(b, okp, s);
-    launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, okp,
-                b->sort_surrogate_classes, b->sort_bucket_classes);
-    kb_composite<<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(b->d_views.ptr, b->nviews, b->offsets.ptr,
-                                                                  b->records.ptr, b->vgeo.ptr, sh, b->tfinal.ptr,
-                                                                  b->term.ptr, okp);
+                                                                        b->vproj.ptr, b->vfix.ptr, b->vgeo.ptr,
+                                                                        b->walk ? b->walk_verts.ptr : nullptr, b->clipped.ptr);
+    launch_kb_count(b, s);
+    launch_scan(b->counts.ptr, b->tot_pixels, b->offsets.ptr, b->scan.ptr, s, b->info.ptr, capacity, b->clipped.ptr);
+    check_launch("batch count");
+}
+
+// Enqueues the whole forward without a host read: kernels after the scan run
+// only if the records fit the capacity.
+void enqueue_forward(dtv_batch* b, const dtv::ShadeDev& sh, cudaStream_t s) {
+    using namespace dtv;
+    enqueue_count(b, b->capacity, s);
+    kb_clear_counts<<<grid_for(b->tot_pixels, 256, 148 * 16), 256, 0, s>>>(b->counts.ptr, b->tot_pixels,
+                                                                           &b->info.ptr->ok);
+    launch_kb_lists(b, sh, /*guarded=*/true, s);
     check_launch("batch forward");
 }
 
@@ -765,12 +900,13 @@ int32_t dtv_batch_reserve(dtv_batch* b, uint64_t max_views, uint64_t max_vertice
         b->long_list.ensure(dtv::sort_scratch_elems(P), s);
         b->records.ensure(max_fragments ? max_fragments : 1, s);
         b->grad_rows.ensure(2 * (max_grad_vertices ? max_grad_vertices : 1), s);
-        b->ok.ensure(1, s);
-        b->total.ensure(1, s);
+        b->info.ensure(1, s);
+        b->clipped.ensure(1, s, /*zero_new=*/true);
+        b->walk_verts.ensure(V, s);
+        b->redo.ensure(P, s);
         b->loss.ensure(1, s);
-        if (!b->h_ok) {
-            DTV_CK(cudaMallocHost(&b->h_ok, sizeof(uint32_t)));
-            DTV_CK(cudaMallocHost(&b->h_total, sizeof(u64)));
+        if (!b->h_info) {
+            DTV_CK(cudaMallocHost(&b->h_info, sizeof(dtv::ListInfo)));
             DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
         }
         DTV_CK(cudaStreamSynchronize(s));
@@ -799,8 +935,10 @@ int32_t dtv_batch_destroy(dtv_batch* b) {
     b->tfinal.release();
     b->term.release();
     b->long_list.release();
-    b->ok.release();
-    b->total.release();
+    b->info.release();
+    b->redo.release();
+    b->clipped.release();
+    b->walk_verts.release();
     b->grad_rows.release();
     b->view_rows.release();
     b->fill_order.release();
@@ -811,8 +949,7 @@ int32_t dtv_batch_destroy(dtv_batch* b) {
     b->step.release();
     if (b->h_views) cudaFreeHost(b->h_views);
     if (b->h_slots) cudaFreeHost(b->h_slots);
-    if (b->h_ok) cudaFreeHost(b->h_ok);
-    if (b->h_total) cudaFreeHost(b->h_total);
+    if (b->h_info) cudaFreeHost(b->h_info);
     if (b->staging_free) cudaEventDestroy(b->staging_free);
     delete b;
     return DTV_OK;
@@ -834,6 +971,8 @@ int32_t dtv_batch_set_meshes(dtv_batch* b, int32_t num_meshes, const dtv_mesh* c
             me[size_t(i)].V = mv.num_vertices;
             me[size_t(i)].F = mv.num_faces;
             me[size_t(i)].faces = mv.faces;
+            me[size_t(i)].walk = mv.walk;
+            me[size_t(i)].Nb = mv.num_boundary_faces;
             const uint32_t* vb = nullptr;
             dtv_mesh_vertex_boundary_device(meshes[i], &vb);
             me[size_t(i)].boundary = vb;
@@ -876,15 +1015,11 @@ int32_t dtv_batch_render(dtv_batch* b, int32_t num_views, const dtv_batch_view* 
         upload_views(b, s);
         // Count and scan, then size the record buffer exactly (one host sync).
         using namespace dtv;
-        kb_project<<<grid_for(b->tot_verts, 256, 0x7fffffffu), 256, 0, s>>>(b->d_views.ptr, b->nviews,
-                                                                            b->tot_verts, b->vproj.ptr, b->vfix.ptr,
-                                                                            b->vgeo.ptr);
-        launch_kb_raster<false>(b, nullptr, s);
-        launch_scan(b->counts.ptr, b->tot_pixels, b->offsets.ptr, b->scan.ptr, s);
-        check_launch("batch count");
-        DTV_CK(cudaMemcpyAsync(b->h_total, b->offsets.ptr + b->tot_pixels, sizeof(u64), cudaMemcpyDeviceToHost, s));
+        enqueue_count(b, ~0ull, s);
+        DTV_CK(cudaMemcpyAsync(b->h_info, b->info.ptr, sizeof(ListInfo), cudaMemcpyDeviceToHost, s));
         DTV_CK(cudaStreamSynchronize(s));
-        const u64 nf = *b->h_total;
+        const u64 nf = b->h_info->nf;
+        b->many_left = b->h_info->clipped != 0u;
         if (params->fragment_budget_bytes && nf * sizeof(u64) > params->fragment_budget_bytes) {
             DTV_CK(cudaMemsetAsync(b->counts.ptr, 0, sizeof(uint32_t) * b->tot_pixels, s));
             throw DtvError(DTV_ERR_BUDGET, "batch needs " + std::to_string(nf) + " fragments, over the budget");
@@ -895,11 +1030,7 @@ int32_t dtv_batch_render(dtv_batch* b, int32_t num_views, const dtv_batch_view* 
             cudaMemsetAsync(b->counts.ptr, 0, sizeof(uint32_t) * b->tot_pixels, s);
             throw;
         }
-        launch_kb_raster<true>(b, nullptr, s);
-        launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, nullptr, b->sort_surrogate_classes, b->sort_bucket_classes);
-        kb_composite<<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(b->d_views.ptr, b->nviews, b->offsets.ptr,
-                                                                      b->records.ptr, b->vgeo.ptr, b->sh,
-                                                                      b->tfinal.ptr, b->term.ptr, nullptr);
+        launch_kb_lists(b, b->sh, /*guarded=*/false, s);
         check_launch("batch render");
         b->last_fragments = nf;
         b->have_render = true;
@@ -920,21 +1051,22 @@ int32_t dtv_batch_render_async(dtv_batch* b, int32_t num_views, const dtv_batch_
         b->sh = dtv::shade_constants(*params);
         upload_views(b, s);
         b->capacity = b->records.cap;
-        enqueue_forward(b, b->sh, /*guarded=*/true, s);
-        DTV_CK(cudaMemcpyAsync(b->h_ok, b->ok.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        DTV_CK(cudaMemcpyAsync(b->h_total, b->total.ptr, sizeof(u64), cudaMemcpyDeviceToHost, s));
+        enqueue_forward(b, b->sh, s);
+        DTV_CK(cudaMemcpyAsync(b->h_info, b->info.ptr, sizeof(dtv::ListInfo), cudaMemcpyDeviceToHost, s));
         b->have_render = true;
         b->async_render = true;
     });
 }
 
-int32_t dtv_batch_render_status(const dtv_batch* b, int32_t* fits, uint64_t* num_fragments) {
+int32_t dtv_batch_render_status(const dtv_batch* cb, int32_t* fits, uint64_t* num_fragments) {
     return guarded([&] {
+        auto* b = const_cast<dtv_batch*>(cb);
         require(b && fits && num_fragments, "null pointer");
         if (!b->have_render || !b->async_render)
             throw DtvError(DTV_ERR_STATE, "no dtv_batch_render_async to report on");
-        *fits = *b->h_ok != 0u ? 1 : 0;
-        *num_fragments = *b->h_total;
+        b->many_left = b->h_info->clipped != 0u;
+        *fits = b->h_info->ok != 0u ? 1 : 0;
+        *num_fragments = b->h_info->nf;
     });
 }
 
@@ -991,7 +1123,7 @@ int32_t dtv_batch_render_adjoint(dtv_batch* b, int32_t num_views, const dtv_batc
         dtv::ShadeDev sh = b->sh;
         sh.use_abs_grad = use_abs_grad ? 1 : 0;
         using namespace dtv;
-        const uint32_t* okp = b->async_render ? b->ok.ptr : nullptr;
+        const uint32_t* okp = b->async_render ? &b->info.ptr->ok : nullptr;
         enqueue_adjoint(b, sh, okp, s);
         if (rows)
             kb_scatter<<<grid_for(rows, 256, 148 * 16), 256, 0, s>>>(b->d_slots.ptr, num_slots, rows,
@@ -1007,15 +1139,16 @@ namespace {
 
 void enqueue_train_body(dtv_batch* b, const dtv::AdamConst& ac, int nslots, cudaStream_t s) {
     using namespace dtv;
-    enqueue_forward(b, b->sh, /*guarded=*/true, s);
+    enqueue_forward(b, b->sh, s);
+    const uint32_t* okp = &b->info.ptr->ok;
     DTV_CK(cudaMemsetAsync(b->loss.ptr, 0, sizeof(float), s));
     kb_loss<<<grid_for(b->tot_pixels, 256, 148 * 8), 256, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_pixels,
-                                                                  b->loss.ptr, b->ok.ptr);
+                                                                  b->loss.ptr, okp);
     DTV_CK(cudaMemsetAsync(b->grad_rows.ptr, 0, sizeof(float4) * 2 * size_t(b->tot_rows), s));
-    enqueue_adjoint(b, b->sh, b->ok.ptr, s);
+    enqueue_adjoint(b, b->sh, okp, s);
     kb_adam_rows<<<grid_for(b->tot_rows, 256, 148 * 16), 256, 0, s>>>(b->d_slots.ptr, nslots, b->tot_rows,
-                                                                      b->grad_rows.ptr, ac, b->step.ptr, b->ok.ptr);
-    kb_step_increment<<<1, 1, 0, s>>>(b->step.ptr, b->ok.ptr);
+                                                                      b->grad_rows.ptr, ac, b->step.ptr, okp);
+    kb_step_increment<<<1, 1, 0, s>>>(b->step.ptr, okp);
     check_launch("batch train step");
 }
 
@@ -1024,7 +1157,9 @@ std::vector<u64> train_signature(const dtv_batch* b, const dtv::AdamConst& ac, i
                             u64(b->max_height),
                             b->capacity, u64(nslots), u64(uintptr_t(b->records.ptr)),
                             u64(uintptr_t(b->dimage_internal.ptr)), u64(uintptr_t(b->grad_rows.ptr)),
-                            u64(uintptr_t(b->view_rows.ptr)), u64(uintptr_t(b->wide_list.ptr))};
+                            u64(uintptr_t(b->view_rows.ptr)), u64(uintptr_t(b->wide_list.ptr)),
+                            u64(uintptr_t(b->counts.ptr)), u64(uintptr_t(b->walk_verts.ptr)),
+                            u64(uintptr_t(b->redo.ptr)), b->tot_bfaces, u64(b->walk), u64(b->many_left)};
     const uint32_t* shw = reinterpret_cast<const uint32_t*>(&b->sh);
     for (size_t i = 0; i < sizeof(b->sh) / 4; ++i) sig.push_back(shw[i]);
     const uint32_t* acw = reinterpret_cast<const uint32_t*>(&ac);
@@ -1145,15 +1280,15 @@ int32_t dtv_batch_train_step(dtv_batch* b, int32_t num_views, const dtv_batch_vi
             } else {
                 enqueue_train_body(b, ac, nslots, ws);
             }
-            DTV_CK(cudaMemcpyAsync(b->h_ok, b->ok.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, ws));
-            DTV_CK(cudaMemcpyAsync(b->h_total, b->total.ptr, sizeof(u64), cudaMemcpyDeviceToHost, ws));
+            DTV_CK(cudaMemcpyAsync(b->h_info, b->info.ptr, sizeof(dtv::ListInfo), cudaMemcpyDeviceToHost, ws));
             DTV_CK(cudaStreamSynchronize(ws));
-            return *b->h_ok != 0u;
+            b->many_left = b->h_info->clipped != 0u;
+            return b->h_info->ok != 0u;
         };
         bool done = run(true);
         if (!done) {
             // Records did not fit: grow, rerun this step uncaptured, recapture next time.
-            const u64 need = *b->h_total;
+            const u64 need = b->h_info->nf;
             b->capacity = u64(double(need) * 1.25) + 1024;
             b->records.ensure(b->capacity, ws);
             b->capacity = b->records.cap;
@@ -1166,7 +1301,7 @@ int32_t dtv_batch_train_step(dtv_batch* b, int32_t num_views, const dtv_batch_vi
             done = run(false);
             if (!done) throw DtvError(DTV_ERR_STATE, "batch records overflowed after resizing");
         }
-        b->last_fragments = *b->h_total;
+        b->last_fragments = b->h_info->nf;
         if (d_loss) DTV_CK(cudaMemcpyAsync(d_loss, b->loss.ptr, sizeof(float), cudaMemcpyDeviceToDevice, ws));
         DTV_CK(cudaEventRecord(ev_out, ws));
         DTV_CK(cudaStreamWaitEvent(user, ev_out, 0));

@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(kTile * kTile) k_composite_cells(
     const u64* __restrict__ offsets, const u64* __restrict__ records, const uint4* __restrict__ faces,
     const uint2* __restrict__ f2t, const VGeo* __restrict__ vgeo, const float4* __restrict__ cell_colors, int W,
     int row0, int row1, ShadeDev sh, float4* __restrict__ image, float* __restrict__ tfinal,
-    uint32_t* __restrict__ term) {
+    uint32_t* __restrict__ term, const uint32_t* __restrict__ gate) {
+    if (gate && *gate == 0u) return;
     const int px = blockIdx.x * kTile + (threadIdx.x % kTile);
     const int py = row0 + int(blockIdx.y) * kTile + int(threadIdx.x / kTile);
     if (px >= W || py >= row1) return;
@@ -276,13 +277,14 @@ __global__ void __launch_bounds__(256) k_scatter_positions(const float4* __restr
 
 void launch_composite_cells(const u64* offsets, const u64* records, const uint4* faces, const uint32_t* face_to_tet,
                             const VGeo* vgeo, const float4* cell_colors, int W, int H, const ShadeDev& sh,
-                            float4* image, float* tfinal, uint32_t* term, cudaStream_t s, int row0, int row1) {
+                            float4* image, float* tfinal, uint32_t* term, cudaStream_t s, int row0, int row1,
+                            const uint32_t* gate) {
     if (row1 < 0) row1 = H;
     if (row1 <= row0) return;
     dim3 grid((W + kTile - 1) / kTile, (row1 - row0 + kTile - 1) / kTile);
     k_composite_cells<<<grid, kTile * kTile, 0, s>>>(offsets, records, faces,
                                                      reinterpret_cast<const uint2*>(face_to_tet), vgeo, cell_colors, W,
-                                                     row0, row1, sh, image, tfinal, term);
+                                                     row0, row1, sh, image, tfinal, term, gate);
 }
 
 void launch_adjoint_cells_rows(const u64* offsets, const u64* records, const uint4* faces,

@@ -108,8 +108,10 @@ __device__ __forceinline__ VGeo project_vertex_geo(const CamDev& c, float x, flo
     const float sxl = __fadd_rn(sx.lo, mxl), syl = __fsub_rn(sy.lo, myl);
     VGeo g;
     const bool valid = fix.x != kInvalidFix;
-    g.sx = valid ? __fmul_rn(float(fix.x), 0.00390625f) : sx.hi;
-    g.sy = valid ? __fmul_rn(float(fix.y), 0.00390625f) : sy.hi;
+    // A vertex outside the valid range is on no fragment's face; its NaN stops
+    // a walk that meets it.
+    g.sx = valid ? __fmul_rn(float(fix.x), 0.00390625f) : __int_as_float(0x7fffffff);
+    g.sy = valid ? __fmul_rn(float(fix.y), 0.00390625f) : __int_as_float(0x7fffffff);
     g.rx = __fadd_rn(__fsub_rn(sx.hi, g.sx), sxl);  // the difference is exact (Sterbenz)
     g.ry = __fadd_rn(__fsub_rn(sy.hi, g.sy), syl);
     // 1 / ze with one Newton correction on the float-float depth.
@@ -120,6 +122,10 @@ __device__ __forceinline__ VGeo project_vertex_geo(const CamDev& c, float x, flo
     g.xv = xv.hi;
     g.yv = yv.hi;
     return g;
+}
+
+__device__ __forceinline__ WalkVertRow walk_row(const float4& pr, const VGeo& g) {
+    return WalkVertRow{make_float4(g.sx, g.sy, pr.x, pr.y), make_float2(pr.z, pr.w), make_float2(0.f, 0.f)};
 }
 
 __device__ __forceinline__ long long floor_div256(long long a) { return a >> 8; }  // arithmetic shift = floor

@@ -30,8 +30,12 @@ struct MeshHost {
 void build_faces(const uint32_t* cells, uint64_t T, uint64_t V, MeshHost& out);
 
 // Launch wrappers (dtv_kernels.cu).  All run on `s`.
+// rows (optional): the vertices' walk rows as well; clipped (optional): set to
+// 1 when a vertex is not projected.
 void launch_project(const float* pos, uint32_t V, const CamDev& cam, float4* vproj, int2* vfix, VGeo* vgeo,
-                    cudaStream_t s);
+                    cudaStream_t s, WalkVertRow* rows = nullptr, uint32_t* clipped = nullptr);
+// gate (optional, fill without a wide_list): the kernels do nothing when *gate
+// is zero; rest: the fill takes only pixels whose counter is not zero.
 // Pixel rows [row0, row1) only (row1 < 0: all rows).  wide_list (u32[F + 1],
 // optional): the count lists the faces of the 64-bit path there, and the
 // 64-bit count and the fill that follows (same rows) walk that list instead of
@@ -42,7 +46,17 @@ void launch_raster_count(const uint4* faces, uint32_t F, const float4* vproj, co
 void launch_raster_fill(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, int H,
                         uint32_t* counts, const unsigned long long* offsets, unsigned long long* records,
                         cudaStream_t s, int row0 = 0, int row1 = -1, const uint32_t* order = nullptr,
-                        const uint32_t* wide_list = nullptr);
+                        const uint32_t* wide_list = nullptr, const uint32_t* gate = nullptr, bool rest = false);
+struct ListInfo;
+// The few pixels the walk left to the rasteriser (nothing is done when there
+// are none, or when clipped vertices make them many: launch_raster_fill with
+// rest and launch_sort of the list then): fill from all faces, sort of the
+// listed pixels' lists.
+void launch_rest_fill(const ListInfo* info, const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W,
+                      int row0, int row1, uint32_t* counts, const unsigned long long* offsets,
+                      unsigned long long* records, cudaStream_t s);
+void launch_rest_sort(const ListInfo* info, bool few, const uint32_t* list, const unsigned long long* offsets,
+                      unsigned long long* records, cudaStream_t s);
 // Order of the faces for the fill, grouped by row bands of about
 // kFillBandBytes of records each (nf records over H rows; order: F entries;
 // band_scratch: 2 * kFillBands entries).
@@ -55,12 +69,23 @@ void launch_band_scan(const uint32_t* hist, uint32_t* cursor, cudaStream_t s);
 // Exclusive scan of counts[n] into offsets[n+1]; scratch must hold scan_scratch_elems(n) u64.
 constexpr uint64_t kScanTile = 4096;  // counts per scan block (1024 threads x 4)
 constexpr size_t scan_scratch_elems(uint64_t n) { return size_t((n + kScanTile - 1) / kScanTile) + 1; }
+// info (optional) gets the total, whether it is at most `capacity`, whether the
+// projection clipped a vertex (*clipped, which is reset), and a zeroed redo
+// counter.
+struct ListInfo {
+    unsigned long long nf;  // records of the lists
+    uint32_t ok;            // they fit
+    uint32_t clipped;
+    uint32_t whole;         // ok and not clipped: the walk and what follows it complete the lists
+    uint32_t n_redo;        // pixels the walk left to the rasteriser
+};
 void launch_scan(const uint32_t* counts, uint64_t n, unsigned long long* offsets, unsigned long long* scratch,
-                 cudaStream_t s);
+                 cudaStream_t s, ListInfo* info = nullptr, unsigned long long capacity = ~0ull,
+                 uint32_t* clipped = nullptr);
 // Per-pixel sort of the lists of P pixels, any length.  scratch holds
 // sort_scratch_elems(P) u32 (length-class counts and lists).  With a non-null
 // `ok`, the sort does nothing when *ok == 0 (batched steps whose records
-// overflowed the buffer).
+// overflowed the buffer).  list: only the *list_n listed pixels (at most P).
 constexpr int kSortClasses = 9;  // list-length classes (dtv_kernels.cu)
 constexpr size_t sort_scratch_elems(uint64_t P) { return 16 + size_t(kSortClasses) * size_t(P); }
 // surrogate_classes: bit c set = list-length class c (1..4: up to 64, 128,
@@ -70,14 +95,17 @@ constexpr uint32_t kSortSurrogateDefault = 0x1eu;
 constexpr uint32_t kSortBucketDefault = 0x3cu;  // classes sorted by distribution (bit c: class c, 2..5)
 void launch_sort(const unsigned long long* offsets, unsigned long long* records, uint32_t P, uint32_t* scratch,
                  cudaStream_t s, const uint32_t* ok = nullptr,
-                 uint32_t surrogate_classes = kSortSurrogateDefault, uint32_t bucket_classes = kSortBucketDefault);
+                 uint32_t surrogate_classes = kSortSurrogateDefault, uint32_t bucket_classes = kSortBucketDefault,
+                 const uint32_t* list = nullptr, const uint32_t* list_n = nullptr);
 constexpr uint32_t kSortWarpCap = 1024;    // elements per warp list sorted in shared memory
 constexpr uint32_t kSortBlockCap = 16384;  // elements per block-sorted list / chunk of a longer one (128 KiB shared memory)
 
+// gate (optional): nothing is done when *gate is zero.
 // tile: pixel tile of the 256-thread blocks (0: 16 x 16, 1: 32 x 8, 2: 8 x 32).
 void launch_composite(const unsigned long long* offsets, const unsigned long long* records, const uint4* faces,
                       const VGeo* vgeo, const float4* colors, int W, int H, const ShadeDev& sh, float4* image,
-                      float* tfinal, uint32_t* term, cudaStream_t s, int row0 = 0, int row1 = -1, int tile = 0);
+                      float* tfinal, uint32_t* term, cudaStream_t s, int row0 = 0, int row1 = -1, int tile = 0,
+                      const uint32_t* gate = nullptr);
 void launch_adjoint(const unsigned long long* offsets, const unsigned long long* records, const uint4* faces,
                     const VGeo* vgeo, const float4* colors, const CamDev& cam, const ShadeDev& sh,
                     const float4* dimage, const float* tfinal, const uint32_t* term, uint32_t V,
@@ -103,7 +131,7 @@ void launch_adam(float* param, const float* grad, float* m, float* v, uint64_t n
 void launch_composite_cells(const unsigned long long* offsets, const unsigned long long* records, const uint4* faces,
                             const uint32_t* face_to_tet, const VGeo* vgeo, const float4* cell_colors, int W, int H,
                             const ShadeDev& sh, float4* image, float* tfinal, uint32_t* term, cudaStream_t s,
-                            int row0, int row1);
+                            int row0, int row1, const uint32_t* gate = nullptr);
 void launch_adjoint_cells_rows(const unsigned long long* offsets, const unsigned long long* records,
                                const uint4* faces, const uint32_t* face_to_tet, const VGeo* vgeo,
                                const float4* cell_colors, const CamDev& cam, const ShadeDev& sh, const float4* dimage,
@@ -131,12 +159,28 @@ void launch_walk_adjoint(const unsigned long long* b_offsets, const unsigned lon
                          const float* tfinal, const uint4* wstate, uint32_t V, float4* grad_rows, float* grad_pos,
                          float4* grad_col, cudaStream_t s);
 
+// Fragment lists by walking the mesh (dtv_walk.cu).
+// Fills the tables (links: 4 T, start: one per boundary face) from the device
+// topology; *bad (device) is set to a non-zero value when the topology cannot
+// be walked (a tet with a vertex twice, a face of more than two tets).
+void launch_build_walk(const uint4* cells, uint32_t T, const uint4* tet_faces, const uint4* faces, const uint2* f2t,
+                       const uint32_t* bf_global, uint32_t Nb, uint4* links, uint4* start, uint32_t* bad,
+                       cudaStream_t s);
+// Lists of pixel rows [row0, row1) from the boundary fragments at the end of
+// each pixel's range.  Pixels it cannot finish are appended to `redo`
+// (info->n_redo of them).  guarded: nothing is done when info->ok is zero.
+void launch_walk_lists(const WalkMesh& wm, const unsigned long long* offsets, unsigned long long* records,
+                       uint32_t* counts, const WalkVertRow* verts, int W, int row0, int row1, ListInfo* info,
+                       uint32_t* redo, bool guarded, cudaStream_t s);
+
 // Accessors used by the allocation-free entry point (dtv_noalloc.cu); they
 // expose what dtv_renderer_render derives from its arguments.
 struct MeshView {
     const uint4* faces;
     uint64_t num_faces;
     uint64_t num_vertices;
+    WalkMesh walk;               // links null: the mesh cannot be walked
+    uint32_t num_boundary_faces;
 };
 
 }  // namespace dtv

@@ -18,27 +18,33 @@ constexpr unsigned kFull = 0xffffffffu;
 // transform + perspective divide; FP32 with fixed rounding).
 __global__ void __launch_bounds__(256) k_project(const float* __restrict__ pos, uint32_t V, CamDev cam,
                                                  float4* __restrict__ vproj, int2* __restrict__ vfix,
-                                                 VGeo* __restrict__ vgeo) {
+                                                 VGeo* __restrict__ vgeo, WalkVertRow* __restrict__ rows,
+                                                 uint32_t* __restrict__ clipped) {
     uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
     float x = pos[3 * size_t(v)], y = pos[3 * size_t(v) + 1], z = pos[3 * size_t(v) + 2];
     int2 fx;
-    vproj[v] = project_vertex(cam, x, y, z, fx);
+    const float4 pr = project_vertex(cam, x, y, z, fx);
+    const VGeo g = project_vertex_geo(cam, x, y, z, fx);
+    vproj[v] = pr;
     vfix[v] = fx;
-    vgeo[v] = project_vertex_geo(cam, x, y, z, fx);
+    vgeo[v] = g;
+    if (rows) rows[v] = walk_row(pr, g);
+    if (clipped && fx.x == kInvalidFix) *clipped = 1u;
 }
 
 void launch_project(const float* pos, uint32_t V, const CamDev& cam, float4* vproj, int2* vfix, VGeo* vgeo,
-                    cudaStream_t s) {
+                    cudaStream_t s, WalkVertRow* rows, uint32_t* clipped) {
     if (V == 0) return;
-    k_project<<<(V + 255) / 256, 256, 0, s>>>(pos, V, cam, vproj, vfix, vgeo);
+    k_project<<<(V + 255) / 256, 256, 0, s>>>(pos, V, cam, vproj, vfix, vgeo, rows, clipped);
 }
 
 // (a)+(b) face rasterisation: 32 faces per warp, the warp's lanes spread over
 // each face's pixels in turn (raster_warp, dtv_path.cuh).
 constexpr int kRasterWarps = 4;
 
-template <bool FILL, bool WIDE>
+// `gate` (optional): nothing is done when *gate is zero.  REST: see fill_pixels.
+template <bool FILL, bool WIDE, bool REST = false>
 __global__ void __launch_bounds__(32 * kRasterWarps) k_raster(const uint4* __restrict__ faces, uint32_t F,
                                                               const float4* __restrict__ vproj,
                                                               const int2* __restrict__ vfix, int W, int row0, int row1,
@@ -46,11 +52,22 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster(const uint4* __res
                                                               const u64* __restrict__ offsets,
                                                               u64* __restrict__ records,
                                                               const uint32_t* __restrict__ order,
-                                                              uint32_t* __restrict__ wide_list) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t f = (order && i < F) ? order[i] : i;
+                                                              uint32_t* __restrict__ wide_list,
+                                                              const uint32_t* __restrict__ gate,
+                                                              uint32_t per_warp) {
+    if (gate && *gate == 0u) return;
+    // The fill gives each warp per_warp <= 32 faces, which it takes one at a
+    // time; the count takes one face per thread.
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool mine = true;
+    if (FILL && per_warp != 32u) {
+        const uint32_t l = threadIdx.x & 31u;
+        i = (i >> 5) * per_warp + l;
+        mine = l < per_warp;
+    }
+    const uint32_t f = (order && mine && i < F) ? order[i] : i;
     RasterJob J;
-    const bool set = i < F && raster_setup(f, faces, vfix, 0u, W, row0, row1, 0ull, J);
+    const bool set = mine && i < F && raster_setup(f, faces, vfix, 0u, W, row0, row1, 0ull, J);
     const bool live = set && (J.wide != 0) == WIDE;
     if constexpr (!FILL) {
         if (live) count_face<typename std::conditional<WIDE, long long, int>::type>(J, counts);
@@ -71,13 +88,13 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster(const uint4* __res
         __shared__ RasterJob jobs[kRasterWarps][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         if (live) jobs[w][lane] = J;
-        raster_warp<FILL, WIDE>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets, records);
+        raster_warp<FILL, WIDE, REST>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets, records);
     }
 }
 
 // The 64-bit faces listed by the count (wide_list), 32 per warp and step over
 // a fixed grid: the count (one thread per face) or the fill (raster_warp).
-template <bool FILL>
+template <bool FILL, bool REST = false>
 __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_listed(const uint4* __restrict__ faces,
                                                                      const float4* __restrict__ vproj,
                                                                      const int2* __restrict__ vfix, int W, int row0,
@@ -98,10 +115,44 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_listed(const uint4
             if (live) count_face<long long>(J, counts);
         } else {
             if (live) jobs[w][lane] = J;
-            raster_warp<FILL, true>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets, records);
+            raster_warp<FILL, true, REST>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets,
+                                          records);
             __syncwarp();  // every lane is done with this step's jobs before the next step writes them
         }
     }
+}
+
+// Fill of the few pixels the walk left to the rasteriser (their counters hold
+// the list length, all others zero), 32 faces per warp and step over a fixed
+// grid; nothing is done unless few_left.
+__global__ void __launch_bounds__(32 * kRasterWarps) k_rest_fill(const ListInfo* __restrict__ info,
+                                                                 const uint4* __restrict__ faces, uint32_t F,
+                                                                 const float4* __restrict__ vproj,
+                                                                 const int2* __restrict__ vfix, int W, int row0,
+                                                                 int row1, uint32_t* __restrict__ counts,
+                                                                 const u64* __restrict__ offsets,
+                                                                 u64* __restrict__ records) {
+    if (!few_left(info)) return;
+    __shared__ RasterJob jobs[kRasterWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t base = blockIdx.x * blockDim.x + uint32_t(w) * 32u; base < F; base += stride) {
+        const uint32_t i = base + uint32_t(lane);
+        RasterJob J;
+        const bool live = i < F && raster_setup(i, faces, vfix, 0u, W, row0, row1, 0ull, J);
+        const bool wide = live && J.wide != 0;
+        if (live) jobs[w][lane] = J;
+        raster_warp<true, false, true>(jobs[w], __ballot_sync(kFull, live && !wide), lane, vproj, counts, offsets,
+                                       records);
+        raster_warp<true, true, true>(jobs[w], __ballot_sync(kFull, wide), lane, vproj, counts, offsets, records);
+        __syncwarp();  // every lane is done with this step's jobs before the next step writes them
+    }
+}
+
+void launch_rest_fill(const ListInfo* info, const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W,
+                      int row0, int row1, uint32_t* counts, const u64* offsets, u64* records, cudaStream_t s) {
+    if (F) k_rest_fill<<<148 * 6, 32 * kRasterWarps, 0, s>>>(info, faces, F, vproj, vfix, W, row0, row1, counts,
+                                                            offsets, records);
 }
 
 constexpr unsigned kListedBlocks = 148;
@@ -120,30 +171,47 @@ void launch_raster_count(const uint4* faces, uint32_t F, const float4* vproj, co
     const unsigned blocks = (F + 32 * kRasterWarps - 1) / (32 * kRasterWarps);
     if (wide_list) cudaMemsetAsync(wide_list, 0, sizeof(uint32_t), s);
     k_raster<false, false><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts, nullptr,
-                                                                nullptr, nullptr, wide_list);
+                                                                nullptr, nullptr, wide_list, nullptr, 32u);
     if (wide_list)
         k_raster_listed<false><<<kListedBlocks, 32 * kRasterWarps, 0, s>>>(faces, vproj, vfix, W, row0, row1, counts,
                                                                            nullptr, nullptr, wide_list);
     else
         k_raster<false, true><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts,
-                                                                   nullptr, nullptr, nullptr, nullptr);
+                                                                   nullptr, nullptr, nullptr, nullptr, nullptr, 32u);
     k_row_prefix<<<unsigned(row1 - row0 + 7) / 8, 256, 0, s>>>(counts, W, row0, row1);
+}
+
+constexpr uint32_t kFillMinWarps = 148 * 32;
+
+template <bool REST>
+static void raster_fill(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, uint32_t* counts,
+                        const u64* offsets, u64* records, cudaStream_t s, int row0, int row1, const uint32_t* order,
+                        const uint32_t* wide_list, const uint32_t* gate) {
+    // A warp fills its faces one after another: few faces (the boundary of a
+    // small mesh) are spread over more warps, down to one face each, until
+    // there are kFillMinWarps of them (8^3 at 64^2: 53 -> 13 us).
+    const uint32_t per_warp = std::min(32u, std::max(1u, F / kFillMinWarps));
+    const unsigned blocks = (F + per_warp * kRasterWarps - 1) / (per_warp * kRasterWarps);
+    k_raster<true, false, REST><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts,
+                                                                     offsets, records, order, nullptr, gate, per_warp);
+    if (wide_list)
+        k_raster_listed<true, REST><<<kListedBlocks, 32 * kRasterWarps, 0, s>>>(faces, vproj, vfix, W, row0, row1,
+                                                                                counts, offsets, records, wide_list);
+    else
+        k_raster<true, true, REST><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts,
+                                                                        offsets, records, order, nullptr, gate,
+                                                                        per_warp);
 }
 
 void launch_raster_fill(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, int H,
                         uint32_t* counts, const u64* offsets, u64* records, cudaStream_t s, int row0, int row1,
-                        const uint32_t* order, const uint32_t* wide_list) {
+                        const uint32_t* order, const uint32_t* wide_list, const uint32_t* gate, bool rest) {
     if (F == 0) return;
     if (row1 < 0) row1 = H;
-    const unsigned blocks = (F + 32 * kRasterWarps - 1) / (32 * kRasterWarps);
-    k_raster<true, false><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts, offsets,
-                                                               records, order, nullptr);
-    if (wide_list)
-        k_raster_listed<true><<<kListedBlocks, 32 * kRasterWarps, 0, s>>>(faces, vproj, vfix, W, row0, row1, counts,
-                                                                          offsets, records, wide_list);
+    if (rest)
+        raster_fill<true>(faces, F, vproj, vfix, W, counts, offsets, records, s, row0, row1, order, wide_list, gate);
     else
-        k_raster<true, true><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts,
-                                                                  offsets, records, order, nullptr);
+        raster_fill<false>(faces, F, vproj, vfix, W, counts, offsets, records, s, row0, row1, order, wide_list, gate);
 }
 
 // ---------------------------------------------------------------------------
@@ -286,7 +354,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* __
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_mid(u64* __restrict__ block_sums, uint64_t nb,
-                                                           u64* __restrict__ out_total) {
+                                                           u64* __restrict__ out_total, ListInfo* __restrict__ info,
+                                                           u64 capacity, uint32_t* __restrict__ clipped) {
     __shared__ u64 sm[32];
     u64 carry = 0;
     for (uint64_t start = 0; start < nb; start += kScanThreads) {
@@ -297,7 +366,15 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_mid(u64* __restrict__ blo
         if (i < nb) block_sums[i] = carry + ex;
         carry += total;
     }
-    if (threadIdx.x == 0) *out_total = carry;
+    if (threadIdx.x == 0) {
+        *out_total = carry;
+        if (info) {
+            const uint32_t cut = clipped ? *clipped : 0u;
+            const uint32_t fits = carry <= capacity ? 1u : 0u;
+            *info = ListInfo{carry, fits, cut, fits && cut == 0u ? 1u : 0u, 0u};
+            if (clipped) *clipped = 0u;  // for the next projection
+        }
+    }
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_final(const uint32_t* __restrict__ in, uint64_t n,
@@ -321,14 +398,15 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_final(const uint32_t* __r
     }
 }
 
-void launch_scan(const uint32_t* counts, uint64_t n, u64* offsets, u64* scratch, cudaStream_t s) {
+void launch_scan(const uint32_t* counts, uint64_t n, u64* offsets, u64* scratch, cudaStream_t s, ListInfo* info,
+                 u64 capacity, uint32_t* clipped) {
     const uint64_t nb = (n + kScanTile - 1) / kScanTile;
     if (nb == 0) {
         cudaMemsetAsync(offsets, 0, sizeof(u64), s);
         return;
     }
     k_scan_reduce<<<unsigned(nb), kScanThreads, 0, s>>>(counts, n, scratch);
-    k_scan_mid<<<1, kScanThreads, 0, s>>>(scratch, nb, offsets + n);
+    k_scan_mid<<<1, kScanThreads, 0, s>>>(scratch, nb, offsets + n, info, capacity, clipped);
     k_scan_final<<<unsigned(nb), kScanThreads, 0, s>>>(counts, n, scratch, offsets);
 }
 
@@ -577,13 +655,18 @@ __device__ __forceinline__ int sort_class(uint32_t n) {
     return 6;
 }
 
+// The pixels are 0 .. P - 1, or the *list_n <= P listed ones.
 __global__ void __launch_bounds__(256) k_sort_classify(const u64* __restrict__ offsets, uint32_t P,
                                                        uint32_t* __restrict__ scratch,
-                                                       const uint32_t* __restrict__ ok) {
+                                                       const uint32_t* __restrict__ ok,
+                                                       const uint32_t* __restrict__ list,
+                                                       const uint32_t* __restrict__ list_n) {
     if (ok && *ok == 0u) return;
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool any = i < (list ? *list_n : P);
+    const uint32_t p = any && list ? list[i] : i;
     int c = -1;
-    if (p < P) {
+    if (any) {
         const u64 n = offsets[p + 1] - offsets[p];
         if (n > kSortBlockCap)
             c = 7;
@@ -954,20 +1037,11 @@ __device__ __forceinline__ void cmpswap_global(u64* r, u64 i, u64 l) {
     }
 }
 
-__global__ void __launch_bounds__(1024) k_sort_class_long(const u64* __restrict__ offsets, u64* records,
-                                                          const uint32_t* __restrict__ items,
-                                                          const uint32_t* __restrict__ count,
-                                                          const uint32_t* __restrict__ ok) {
-    if (ok && *ok == 0u) return;
-    extern __shared__ u64 sm_sort[];
-    constexpr u64 C = kSortBlockCap;
-    const uint32_t num = *count;
+template <uint32_t kChunk>
+__device__ void sort_list_block(u64* r, u64 n, u64* sm_sort) {
+    constexpr u64 C = kChunk;
     const uint32_t tid = threadIdx.x, nthr = blockDim.x;
-    for (uint32_t it = blockIdx.x; it < num; it += gridDim.x) {
-        const uint32_t p = items[it];
-        const u64 beg = offsets[p];
-        const u64 n = offsets[p + 1] - beg;
-        u64* r = records + beg;
+    {
         u64 N = C;
         while (N < n) N <<= 1;
         // Stages k <= C: each chunk sorted in shared memory.
@@ -1018,6 +1092,52 @@ __global__ void __launch_bounds__(1024) k_sort_class_long(const u64* __restrict_
     }
 }
 
+__global__ void __launch_bounds__(1024) k_sort_class_long(const u64* __restrict__ offsets, u64* records,
+                                                          const uint32_t* __restrict__ items,
+                                                          const uint32_t* __restrict__ count,
+                                                          const uint32_t* __restrict__ ok) {
+    if (ok && *ok == 0u) return;
+    extern __shared__ u64 sm_sort[];
+    const uint32_t num = *count;
+    for (uint32_t it = blockIdx.x; it < num; it += gridDim.x) {
+        const uint32_t p = items[it];
+        const u64 beg = offsets[p];
+        sort_list_block<kSortBlockCap>(records + beg, offsets[p + 1] - beg, sm_sort);
+    }
+}
+
+// The lists of the listed pixels, one block per list over a fixed grid: up
+// to kRestCap records in shared memory, longer lists in place.  For the few
+// pixels the walk leaves to the rasteriser, whatever their length, in one
+// launch that costs next to nothing when there are none.
+constexpr uint32_t kRestCap = 2048;
+__global__ void __launch_bounds__(256) k_rest_sort(const ListInfo* __restrict__ info, bool few,
+                                                   const uint32_t* __restrict__ list,
+                                                   const u64* __restrict__ offsets, u64* records) {
+    __shared__ u64 sm[kRestCap];
+    const uint32_t num = few ? few_left(info) : info->n_redo;
+    for (uint32_t i = blockIdx.x; i < num; i += gridDim.x) {
+        const uint32_t p = list[i];
+        const u64 beg = offsets[p], n = offsets[p + 1] - beg;
+        u64* r = records + beg;
+        if (n > kRestCap) {
+            sort_list_block<kRestCap>(r, n, sm);
+        } else {
+            uint32_t N = 32;
+            while (N < n) N <<= 1;
+            for (uint32_t j = threadIdx.x; j < N; j += blockDim.x) sm[j] = j < n ? r[j] : ~0ull;
+            __syncthreads();
+            bitonic_smem<true>(sm, N, threadIdx.x, blockDim.x);
+            for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) r[j] = sm[j];
+        }
+        __syncthreads();
+    }
+}
+
+void launch_rest_sort(const ListInfo* info, bool few, const uint32_t* list, const u64* offsets, u64* records, cudaStream_t s) {
+    k_rest_sort<<<148 * 8, 256, 0, s>>>(info, few, list, offsets, records);
+}
+
 static_assert(kSortClasses == 9, "k_sort_classify assigns classes 0..8");
 
 template <int K>
@@ -1032,7 +1152,8 @@ void sort_class(int method, unsigned g, const u64* offsets, u64* records, const 
 }
 
 void launch_sort(const u64* offsets, u64* records, uint32_t P, uint32_t* scratch, cudaStream_t s,
-                 const uint32_t* ok, uint32_t surrogate_classes, uint32_t bucket_classes) {
+                 const uint32_t* ok, uint32_t surrogate_classes, uint32_t bucket_classes, const uint32_t* list,
+                 const uint32_t* list_n) {
     static bool attr_set = false;
     const size_t smem_warp = size_t(kSortWarps) * kSortWarpCap * sizeof(u64);
     const size_t smem_bucket = size_t(kSortBucketWarps) * (2 * kSortWarpCap + kSortWarpCap / 2) * sizeof(u64);
@@ -1047,7 +1168,7 @@ void launch_sort(const u64* offsets, u64* records, uint32_t P, uint32_t* scratch
     }
     if (P == 0) return;
     cudaMemsetAsync(scratch, 0, 16 * sizeof(uint32_t), s);
-    k_sort_classify<<<(P + 255) / 256, 256, 0, s>>>(offsets, P, scratch, ok);
+    k_sort_classify<<<(P + 255) / 256, 256, 0, s>>>(offsets, P, scratch, ok, list, list_n);
     auto items = [&](int c) { return scratch + 16 + size_t(c) * P; };
     const unsigned g = unsigned(std::min<uint64_t>(kSortGridBlocks, (uint64_t(P) + kSortWarps - 1) / kSortWarps));
     // Lists the register sorts leave unsettled join the block-sort class (6).
@@ -1083,7 +1204,9 @@ template <int TX>
 __global__ void __launch_bounds__(256) k_composite(
     const u64* __restrict__ offsets, const u64* __restrict__ records, const uint4* __restrict__ faces,
     const VGeo* __restrict__ vgeo, const float4* __restrict__ colors, int W, int row0, int row1, ShadeDev sh,
-    float4* __restrict__ image, float* __restrict__ tfinal, uint32_t* __restrict__ term) {
+    float4* __restrict__ image, float* __restrict__ tfinal, uint32_t* __restrict__ term,
+    const uint32_t* __restrict__ gate) {
+    if (gate && *gate == 0u) return;
     constexpr int TY = 256 / TX;
     const int px = blockIdx.x * TX + (threadIdx.x % TX);
     const int py = row0 + int(blockIdx.y) * TY + int(threadIdx.x / TX);
@@ -1094,24 +1217,24 @@ __global__ void __launch_bounds__(256) k_composite(
 template <int TX>
 void composite_tiles(const u64* offsets, const u64* records, const uint4* faces, const VGeo* vgeo,
                      const float4* colors, int W, int row0, int row1, const ShadeDev& sh, float4* image,
-                     float* tfinal, uint32_t* term, cudaStream_t s) {
+                     float* tfinal, uint32_t* term, const uint32_t* gate, cudaStream_t s) {
     constexpr int TY = 256 / TX;
     dim3 grid((W + TX - 1) / TX, (row1 - row0 + TY - 1) / TY);
     k_composite<TX><<<grid, 256, 0, s>>>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal,
-                                         term);
+                                         term, gate);
 }
 
 void launch_composite(const u64* offsets, const u64* records, const uint4* faces, const VGeo* vgeo,
                       const float4* colors, int W, int H, const ShadeDev& sh, float4* image, float* tfinal,
-                      uint32_t* term, cudaStream_t s, int row0, int row1, int tile) {
+                      uint32_t* term, cudaStream_t s, int row0, int row1, int tile, const uint32_t* gate) {
     if (row1 < 0) row1 = H;
     if (row1 <= row0) return;
     if (tile == 1)
-        composite_tiles<32>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, s);
+        composite_tiles<32>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate, s);
     else if (tile == 2)
-        composite_tiles<8>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, s);
+        composite_tiles<8>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate, s);
     else
-        composite_tiles<16>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, s);
+        composite_tiles<16>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate, s);
 }
 
 // ---------------------------------------------------------------------------

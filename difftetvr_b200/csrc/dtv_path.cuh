@@ -3,6 +3,7 @@
 #pragma once
 #include <type_traits>
 #include "dtv_device.cuh"
+#include "dtv_internal.h"
 #include "dtv_segment.cuh"
 
 namespace dtv {
@@ -211,8 +212,9 @@ __device__ __forceinline__ void row_prefix_warp(uint32_t* row, int W, int lane) 
 // Fill of U covered pixels per lane per step: offset loads, counter atomics
 // and depth keys of all U before the stores.  A counter already at zero
 // (which matching count and fill spans never leave) skips the store, so a
-// record is never written outside its list.
-template <typename I, int U>
+// record is never written outside its list.  REST: only the pixels whose list
+// the walk left to the rasteriser (the others' counters are zero).
+template <bool REST, typename I, int U>
 __device__ __forceinline__ void fill_pixels(const RasterJob& J, const int (&c)[U], const int (&r)[U],
                                             const bool (&valid)[U], u64 pbase, const float4& va, const float4& vb,
                                             const float4& vc, uint32_t* __restrict__ counts,
@@ -224,6 +226,8 @@ __device__ __forceinline__ void fill_pixels(const RasterJob& J, const int (&c)[U
     for (int k = 0; k < U; ++k) {
         if (valid[k]) {
             const u64 p = pbase + uint32_t(r[k] * J.W + c[k]);
+            slot[k] = 0u;
+            if (REST && *reinterpret_cast<volatile uint32_t*>(&counts[p]) == 0u) continue;
             off[k] = offsets[p];
             slot[k] = atomicSub(&counts[p], 1u);
             z[k] = depth_key(va, vb, vc, float(J.px0 + c[k]) + 0.5f, float(J.py0 + r[k]) + 0.5f);
@@ -238,7 +242,7 @@ __device__ __forceinline__ void fill_pixels(const RasterJob& J, const int (&c)[U
 // row), finds each row's exact span, and spreads the concatenated spans over
 // its lanes (slot s -> row by a binary search of the spans' exclusive prefix
 // sums), so every lane slot is a covered pixel.
-template <bool FILL, typename I>
+template <bool FILL, bool REST, typename I>
 __device__ __forceinline__ void raster_job(const RasterJob& J, int lane, const float4* __restrict__ vproj,
                                            uint32_t* __restrict__ counts, const u64* __restrict__ offsets,
                                            u64* __restrict__ records) {
@@ -276,7 +280,7 @@ __device__ __forceinline__ void raster_job(const RasterJob& J, int lane, const f
                     rr[k] = r0 + i;
                     c[k] = __shfl_sync(0xffffffffu, xl, i) + (sl - __shfl_sync(0xffffffffu, excl, i));
                 }
-                fill_pixels<I, U>(J, c, rr, valid, pbase, va, vb, vc, counts, offsets, records);
+                fill_pixels<REST, I, U>(J, c, rr, valid, pbase, va, vb, vc, counts, offsets, records);
             }
         }
     }
@@ -285,7 +289,7 @@ __device__ __forceinline__ void raster_job(const RasterJob& J, int lane, const f
 // The warp's jobs (one per lane that has one, `live` the ballot), one at a time.
 // The 32-bit and 64-bit faces go to separate launches (WIDE), so that the
 // common 32-bit kernel keeps the register count of its own path.
-template <bool FILL, bool WIDE>
+template <bool FILL, bool WIDE, bool REST = false>
 __device__ __forceinline__ void raster_warp(const RasterJob* jobs, uint32_t live, int lane,
                                             const float4* __restrict__ vproj, uint32_t* __restrict__ counts,
                                             const u64* __restrict__ offsets, u64* __restrict__ records) {
@@ -294,10 +298,15 @@ __device__ __forceinline__ void raster_warp(const RasterJob* jobs, uint32_t live
         const int k = __ffs(live) - 1;
         live &= live - 1;
         const RasterJob J = jobs[k];
-        raster_job<FILL, typename std::conditional<WIDE, long long, int>::type>(J, lane, vproj, counts, offsets,
-                                                                                records);
+        raster_job<FILL, REST, typename std::conditional<WIDE, long long, int>::type>(J, lane, vproj, counts,
+                                                                                      offsets, records);
     }
 }
+
+// Pixels the walk left to the rasteriser when that are few (rounding cannot
+// make any; loops of inverted tets and far vertices do).  With clipped
+// vertices many pixels' chains are cut: the launches for many pixels follow.
+__device__ __forceinline__ uint32_t few_left(const ListInfo* info) { return info->clipped ? 0u : info->n_redo; }
 
 // ---------------------------------------------------------------------------
 // Fragment evaluation shared by composite and adjoint.

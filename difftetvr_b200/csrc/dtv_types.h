@@ -2,6 +2,7 @@
 #pragma once
 #include <cstdint>
 #include <climits>
+#include <vector_types.h>
 
 namespace dtv {
 
@@ -32,6 +33,33 @@ struct alignas(16) VGeo {
     float sx, sy;   // snapped position (px)
     float rx, ry;   // exact projected position - snapped position (px)
     float iz, ze, xv, yv;
+};
+
+// Per-view vertex row of the list walk, 32 bytes (one sector): what a step
+// needs of a new vertex.
+struct alignas(32) WalkVertRow {
+    float4 pos;    // VGeo sx, sy (NaN when not projected); vproj x, y
+    float2 depth;  // vproj 1 / ze, ze
+    float2 pad;
+};
+
+// Walk tables of a mesh.  links[4 t + k] belongs to the face opposite tet t's
+// local vertex k:
+//   x  bits 0..27 the tet across the face (0x0fffffff: none), 28..29 the local
+//      vertex that is the face's third stored vertex, 31 whether the two tets'
+//      vertex orders wind the face alike
+//   y  face << 2 | boundary << 1 | whether the stored winding is odd against
+//      the tet's own vertex order
+//   z  the vertex of the tet across that is not on the face
+//   w  byte l: the local index in the tet across of t's local vertex l, byte k
+//      that of z
+// and per boundary face k (vertices bfaces[k]) start[k] = its tet, that tet's
+// vertex off the face, the local indices of the face's three vertices and of
+// that one (a byte each), the face id.
+struct WalkMesh {
+    const uint4* links;
+    const uint4* start;
+    const uint4* bfaces;
 };
 
 // Per-render settings that the kernels read.
