@@ -313,8 +313,8 @@ __device__ __forceinline__ bool tile_pixel(const BatchView* views, int nviews, i
     v = find_index(blockIdx.x, nviews, [&](int i) { return views[i].tile_base; });
     const BatchView& bv = views[v];
     const uint32_t t = uint32_t(blockIdx.x - bv.tile_base);
-    px = int((t % bv.tiles_x) * kTile + threadIdx.x % kTile);
-    py = int((t / bv.tiles_x) * kTile + threadIdx.x / kTile);
+    px = int((t % bv.tiles_x) * kTile + tile_x<kTile>(threadIdx.x));
+    py = int((t / bv.tiles_x) * kTile + tile_y<kTile>(threadIdx.x));
     return px < int(bv.W) && py < int(bv.H);
 }
 

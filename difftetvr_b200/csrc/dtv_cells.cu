@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(kTile * kTile) k_composite_cells(
     int row0, int row1, ShadeDev sh, float4* __restrict__ image, float* __restrict__ tfinal,
     uint32_t* __restrict__ term, const uint32_t* __restrict__ gate) {
     if (gate && *gate == 0u) return;
-    const int px = blockIdx.x * kTile + (threadIdx.x % kTile);
-    const int py = row0 + int(blockIdx.y) * kTile + int(threadIdx.x / kTile);
+    const int px = blockIdx.x * kTile + tile_x<kTile>(threadIdx.x);
+    const int py = row0 + int(blockIdx.y) * kTile + tile_y<kTile>(threadIdx.x);
     if (px >= W || py >= row1) return;
     const size_t p = size_t(py) * W + px;
     const u64 beg = offsets[p];
@@ -108,7 +108,7 @@ __device__ __forceinline__ FragP load_frag_p(const uint32_t (&v)[3], uint32_t ke
         f.dx[j] = fi.dx[j];
         f.dy[j] = fi.dy[j];
     }
-    f.invA = __fdividef(1.0f, fi.A);
+    f.invA = rcp_approx(fi.A);
     f.zz = fi.clamped ? 0.f : fi.zb * fi.zb;
     return f;
 }
@@ -191,8 +191,8 @@ __global__ void __launch_bounds__(kTile * kCellRows, SCREEN ? 5 : 4) k_adjoint_c
     const uint2* __restrict__ f2t, const VGeo* __restrict__ vgeo, const float4* __restrict__ cell_colors, int W,
     int row0, int row1, CamDev cam, ShadeDev sh, const float4* __restrict__ dimage, const float* __restrict__ tfinal,
     const uint32_t* __restrict__ term, float4* __restrict__ grad_rows, float4* __restrict__ grad_cells) {
-    const int px = blockIdx.x * kTile + (threadIdx.x % kTile);
-    const int py = row0 + int(blockIdx.y) * kCellRows + int(threadIdx.x / kTile);
+    const int px = blockIdx.x * kTile + tile_x<kTile>(threadIdx.x);
+    const int py = row0 + int(blockIdx.y) * kCellRows + tile_y<kTile>(threadIdx.x);
     if (px >= W || py >= row1) return;
     const size_t p = size_t(py) * W + px;
     const u64 beg = offsets[p];

@@ -192,6 +192,12 @@ __device__ __forceinline__ float cross_res(float ax, float ay, float arx, float 
     return __fadd_rn(f, __fadd_rn(e, t));
 }
 
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 __device__ __forceinline__ void face_interp(const VGeo& a, const VGeo& b, const VGeo& c, float qx, float qy,
                                             FaceInterp& fi) {
     // Snapped differences: multiples of 1/256 px below 2^16 px, exact (x and
@@ -204,7 +210,7 @@ __device__ __forceinline__ void face_interp(const VGeo& a, const VGeo& b, const 
     const float E1 = cross_res(d2x, d2y, c.rx, c.ry, d0x, d0y, a.rx, a.ry);
     const float E2 = cross_res(d0x, d0y, a.rx, a.ry, d1x, d1y, b.rx, b.ry);
     fi.A = E0 + E1 + E2;
-    const float iA = __fdividef(1.0f, fi.A);
+    const float iA = rcp_approx(fi.A);
     fi.lam[0] = E0 * iA;
     fi.lam[1] = E1 * iA;
     fi.lam[2] = E2 * iA;
@@ -213,7 +219,7 @@ __device__ __forceinline__ void face_interp(const VGeo& a, const VGeo& b, const 
     fi.dx[0] = e0.x; fi.dx[1] = e1.x; fi.dx[2] = e2.x;
     fi.dy[0] = e0.y; fi.dy[1] = e1.y; fi.dy[2] = e2.y;
     const float u0 = fi.lam[0] * a.iz, u1 = fi.lam[1] * b.iz, u2 = fi.lam[2] * c.iz;
-    fi.zb = __fdividef(1.0f, u0 + u1 + u2);
+    fi.zb = rcp_approx(u0 + u1 + u2);
     fi.bary[0] = u0 * fi.zb;
     fi.bary[1] = u1 * fi.zb;
     fi.bary[2] = u2 * fi.zb;

@@ -1208,8 +1208,8 @@ __global__ void __launch_bounds__(256) k_composite(
     const uint32_t* __restrict__ gate) {
     if (gate && *gate == 0u) return;
     constexpr int TY = 256 / TX;
-    const int px = blockIdx.x * TX + (threadIdx.x % TX);
-    const int py = row0 + int(blockIdx.y) * TY + int(threadIdx.x / TX);
+    const int px = blockIdx.x * TX + tile_x<TX>(threadIdx.x);
+    const int py = row0 + int(blockIdx.y) * TY + tile_y<TX>(threadIdx.x);
     if (px < W && py < row1)
         composite_pixel(px, py, W, offsets, records, faces, vgeo, colors, sh, image, tfinal, term);
 }
@@ -1251,8 +1251,8 @@ __global__ void __launch_bounds__(kAdjThreads, 2 * 256 / kAdjThreads) k_adjoint(
     __shared__ float4 vcache4[3 * kAdjThreads];
     __shared__ float vcache1[3 * kAdjThreads];
     constexpr int TY = kAdjThreads / TX;
-    const int px = blockIdx.x * TX + (threadIdx.x % TX);
-    const int py = row0 + int(blockIdx.y) * TY + int(threadIdx.x / TX);
+    const int px = blockIdx.x * TX + tile_x<TX>(threadIdx.x);
+    const int py = row0 + int(blockIdx.y) * TY + tile_y<TX>(threadIdx.x);
     if (px >= W || py >= row1) return;
     // Screen-space rows: the ordered register cache (order_like); world-space
     // rows (absolute gradients): the shared-memory cache.

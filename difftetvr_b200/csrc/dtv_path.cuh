@@ -11,6 +11,12 @@ namespace dtv {
 using u64 = unsigned long long;
 constexpr int kTile = 16;  // composite / adjoint pixel tile (16 x 16 threads)
 
+// Pixel of thread t in a block TX pixels wide: its warps are 8 x 4 pixels.
+template <int TX>
+__device__ __forceinline__ int tile_x(uint32_t t) { return int((t >> 5) % (TX / 8) * 8 + (t & 7u)); }
+template <int TX>
+__device__ __forceinline__ int tile_y(uint32_t t) { return int((t >> 5) / (TX / 8) * 4 + ((t >> 3) & 3u)); }
+
 // ---------------------------------------------------------------------------
 // (a)+(b) face rasterisation, warp-cooperative.  Each lane of a warp sets up
 // one face (projected fixed-point vertices, orientation, clipped bounding box)
@@ -732,7 +738,7 @@ __device__ __forceinline__ void frag_vertex_grads(const FragV& fr, float qx, flo
         giz[j] = gu * fi.lam[j];
         sl += glam[j] * fi.lam[j];
     }
-    const float invA = __fdividef(1.0f, fi.A);
+    const float invA = rcp_approx(fi.A);
     float gE[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j) gE[j] = (glam[j] - sl) * invA;
@@ -948,7 +954,7 @@ __device__ __forceinline__ void frag_position_grads(const uint4& fc, float qx, f
         giz[j] = -gzz * fi.lam[j];
         sl += glam[j] * fi.lam[j];
     }
-    const float invA = __fdividef(1.0f, fi.A);
+    const float invA = rcp_approx(fi.A);
     float gE[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j) gE[j] = (glam[j] - sl) * invA;
@@ -1034,7 +1040,7 @@ __device__ __forceinline__ FragG load_frag_g(uint32_t lo, uint32_t v0, uint32_t 
         f.dx[j] = fi.dx[j];
         f.dy[j] = fi.dy[j];
     }
-    f.invA = __fdividef(1.0f, fi.A);
+    f.invA = rcp_approx(fi.A);
     f.zb = fi.zb;
     f.zz = fi.clamped ? 0.f : fi.zb * fi.zb;
     f.pc[0] = gC0 * c0.x + gC1 * c0.y + gC2 * c0.z;

@@ -185,8 +185,8 @@ __global__ void __launch_bounds__(kWalkThreads, 5) k_walk_composite(
     const uint4* __restrict__ faces, const uint32_t* __restrict__ f2t, TetTopo tt, uint32_t num_tets, const int2* __restrict__ vfix, const VGeo* __restrict__ vgeo,
     const float4* __restrict__ colors, CamDev cam, ShadeDev sh, float4* __restrict__ image,
     float* __restrict__ tfinal, uint4* __restrict__ wstate) {
-    const int px = blockIdx.x * kTile + (threadIdx.x % kTile);
-    const int py = blockIdx.y * kWalkRows + (threadIdx.x / kTile);
+    const int px = blockIdx.x * kTile + tile_x<kTile>(threadIdx.x);
+    const int py = blockIdx.y * kWalkRows + tile_y<kTile>(threadIdx.x);
     if (px >= cam.W || py >= cam.H) return;
     const size_t p = size_t(py) * cam.W + px;
     const u64 beg = b_offsets[p];
@@ -315,8 +315,8 @@ __global__ void __launch_bounds__(kTile * kTile, 2) k_walk_adjoint(
     const uint4* __restrict__ faces, const uint32_t* __restrict__ f2t, TetTopo tt, uint32_t num_tets, const int2* __restrict__ vfix, const VGeo* __restrict__ vgeo,
     const float4* __restrict__ colors, CamDev cam, ShadeDev sh, const float4* __restrict__ dimage,
     const float* __restrict__ tfinal, const uint4* __restrict__ wstate, float4* __restrict__ grad_rows) {
-    const int px = blockIdx.x * kTile + (threadIdx.x % kTile);
-    const int py = blockIdx.y * kTile + (threadIdx.x / kTile);
+    const int px = blockIdx.x * kTile + tile_x<kTile>(threadIdx.x);
+    const int py = blockIdx.y * kTile + tile_y<kTile>(threadIdx.x);
     if (px >= cam.W || py >= cam.H) return;
     const size_t p = size_t(py) * cam.W + px;
     const uint4 ws = wstate[p];
