@@ -90,7 +90,8 @@ struct dtv_renderer {
     DevBuf<float> tfinal;
     DevBuf<uint32_t> term;
     DevBuf<uint32_t> long_list;     // sort scratch (length classes)
-    DevBuf<float4> grad_rows;     // [V][2] interleaved vertex gradient accumulator
+    DevBuf<float4> grad_rows;     // [copies][V][2] interleaved vertex gradient accumulator (grad_copies)
+    DevBuf<float4> cell_rows;     // [copies][T] cell gradients of a mesh with few cells
     // Row bands [row0, row1) of the last render when its lists exceeded the
     // fragment budget (each band's lists are rebuilt by the adjoint); empty
     // when the lists are stored whole.
@@ -242,6 +243,24 @@ void build_band_lists(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& 
     check_launch("band sort");
 }
 
+// Gradient rows of an adjoint, cleared: the copies of the vertices' rows, and
+// with few cells those of the cells'.
+void clear_rows(dtv_renderer* r, const dtv_mesh* mesh, cudaStream_t s) {
+    const uint64_t V = r->V ? r->V : 1, T = mesh->host.num_cells;
+    const size_t n = 2 * size_t(V) * dtv::grad_copies(r->V, r->P);
+    r->grad_rows.ensure(n, s);
+    DTV_CK(cudaMemsetAsync(r->grad_rows.ptr, 0, sizeof(float4) * n, s));
+    if (r->cells && dtv::grad_copies(T, r->P) > 1) {
+        r->cell_rows.ensure(size_t(T) * dtv::grad_copies(T, r->P), s);
+        DTV_CK(cudaMemsetAsync(r->cell_rows.ptr, 0, sizeof(float4) * size_t(T) * dtv::grad_copies(T, r->P), s));
+    }
+}
+
+// Where the per-cell adjoint adds the cell gradients.
+float4* cell_target(dtv_renderer* r, const dtv_mesh* mesh, float* d_grad_colors) {
+    return dtv::grad_copies(mesh->host.num_cells, r->P) > 1 ? r->cell_rows.ptr : reinterpret_cast<float4*>(d_grad_colors);
+}
+
 // Adjoint of rows [y0, y1) into the gradient rows (per-cell: the cell colour
 // gradients go straight into d_grad_colors f32[4T]).
 void adjoint_rows(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors, const float* d_image_adjoint,
@@ -250,23 +269,29 @@ void adjoint_rows(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors, 
         dtv::launch_adjoint_cells_rows(r->offsets.ptr, r->records.ptr, mesh->d_faces, mesh->d_face_to_tet,
                                        r->vgeo.ptr, reinterpret_cast<const float4*>(d_colors), r->cam, sh,
                                        reinterpret_cast<const float4*>(d_image_adjoint), r->tfinal.ptr, r->term.ptr,
-                                       y0, y1, r->grad_rows.ptr, reinterpret_cast<float4*>(d_grad_colors), s);
+                                       y0, y1, r->grad_rows.ptr, uint32_t(r->V), dtv::grad_copies(r->V, r->P),
+                                       cell_target(r, mesh, d_grad_colors), uint32_t(mesh->host.num_cells),
+                                       dtv::grad_copies(mesh->host.num_cells, r->P), s);
     else
         dtv::launch_adjoint_rows(r->offsets.ptr, r->records.ptr, mesh->d_faces, r->vgeo.ptr,
                                  reinterpret_cast<const float4*>(d_colors), r->cam, sh,
                                  reinterpret_cast<const float4*>(d_image_adjoint), r->tfinal.ptr, r->term.ptr, y0, y1,
-                                 r->grad_rows.ptr, s, r->tuning.adjoint_tile);
+                                 r->grad_rows.ptr, uint32_t(r->V), dtv::grad_copies(r->V, r->P), s, r->tuning.adjoint_tile);
 }
 
 // The list adjoint (launch_adjoint_rows) leaves screen-space position rows
 // unless absolute gradients were asked for.
-void scatter_rows(dtv_renderer* r, const dtv::ShadeDev& sh, float* d_grad_positions, float* d_grad_colors,
-                  cudaStream_t s) {
+void scatter_rows(dtv_renderer* r, const dtv_mesh* mesh, const dtv::ShadeDev& sh, float* d_grad_positions,
+                  float* d_grad_colors, cudaStream_t s) {
+    const uint64_t T = mesh->host.num_cells;
+    if (r->cells && dtv::grad_copies(T, r->P) > 1)
+        dtv::launch_add_cell_copies(r->cell_rows.ptr, uint32_t(T), dtv::grad_copies(T, r->P),
+                                    reinterpret_cast<float4*>(d_grad_colors), s);
     if (r->cells)
-        dtv::launch_scatter_positions(r->grad_rows.ptr, uint32_t(r->V), d_grad_positions, s,
+        dtv::launch_scatter_positions(r->grad_rows.ptr, uint32_t(r->V), dtv::grad_copies(r->V, r->P), d_grad_positions, s,
                                       sh.use_abs_grad ? nullptr : r->vgeo.ptr, &r->cam);
     else
-        dtv::launch_scatter_grads(r->grad_rows.ptr, uint32_t(r->V), d_grad_positions,
+        dtv::launch_scatter_grads(r->grad_rows.ptr, uint32_t(r->V), dtv::grad_copies(r->V, r->P), d_grad_positions,
                                   reinterpret_cast<float4*>(d_grad_colors), s,
                                   sh.use_abs_grad ? nullptr : r->vgeo.ptr, &r->cam);
 }
@@ -304,7 +329,7 @@ void render_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors,
 void adjoint_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors, const float* d_image_adjoint,
                     const dtv::ShadeDev& sh, float* d_grad_positions, float* d_grad_colors, cudaStream_t s) {
     const int W = r->cam.W, H = r->cam.H;
-    DTV_CK(cudaMemsetAsync(r->grad_rows.ptr, 0, sizeof(float4) * 2 * size_t(r->V ? r->V : 1), s));
+    clear_rows(r, mesh, s);
     r->wide_list.ensure(size_t(mesh->host.num_faces) + 1, s);
     for (const auto& b : r->bands) {
         dtv::launch_raster_count(mesh->d_faces, uint32_t(mesh->host.num_faces), r->vproj.ptr, r->vfix.ptr, W, H,
@@ -314,7 +339,7 @@ void adjoint_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors
         adjoint_rows(r, mesh, d_colors, d_image_adjoint, sh, b.first, b.second, d_grad_colors, s);
         check_launch("band adjoint");
     }
-    scatter_rows(r, sh, d_grad_positions, d_grad_colors, s);
+    scatter_rows(r, mesh, sh, d_grad_positions, d_grad_colors, s);
     check_launch("scatter gradients");
 }
 
@@ -506,6 +531,7 @@ int32_t dtv_renderer_destroy(dtv_renderer* r) {
     r->term.release();
     r->long_list.release();
     r->grad_rows.release();
+    r->cell_rows.release();
     r->wstate.release();
     r->fill_order.release();
     r->band_scratch.release();
@@ -718,24 +744,24 @@ int32_t adjoint_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_pos
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         dtv::ShadeDev sh = r->sh;
         sh.use_abs_grad = use_abs_grad ? 1 : 0;
-        r->grad_rows.ensure(2 * (r->V ? r->V : 1), s);
         rec_event(r, 7, s);
         if (!r->bands.empty()) {
             adjoint_banded(r, mesh, d_colors, d_image_adjoint, sh, d_grad_positions, d_grad_colors, s);
         } else if (r->type == DTV_RENDERER_INTERSECTION) {
+            r->grad_rows.ensure(2 * size_t(r->V ? r->V : 1) * dtv::grad_copies(r->V, r->P), s);
             dtv::launch_walk_adjoint(r->offsets.ptr, r->records.ptr, mesh->d_bf_global, mesh->d_faces,
                                      mesh->d_face_to_tet, mesh->d_tet_faces, mesh->d_cells, mesh->d_tet_flip,
                                      uint32_t(mesh->host.num_cells),
                                      r->vfix.ptr, r->vgeo.ptr, reinterpret_cast<const float4*>(d_colors), r->cam, sh,
                                      reinterpret_cast<const float4*>(d_image_adjoint), r->tfinal.ptr,
-                                     r->wstate.ptr, uint32_t(r->V), r->grad_rows.ptr, d_grad_positions,
+                                     r->wstate.ptr, uint32_t(r->V), r->grad_rows.ptr, dtv::grad_copies(r->V, r->P), d_grad_positions,
                                      reinterpret_cast<float4*>(d_grad_colors), s);
             check_launch("ray-tet adjoint walk");
         } else {
-            DTV_CK(cudaMemsetAsync(r->grad_rows.ptr, 0, sizeof(float4) * 2 * size_t(r->V ? r->V : 1), s));
+            clear_rows(r, mesh, s);
             adjoint_rows(r, mesh, d_colors, d_image_adjoint, sh, 0, r->cam.H, d_grad_colors, s);
             check_launch("adjoint");
-            scatter_rows(r, sh, d_grad_positions, d_grad_colors, s);
+            scatter_rows(r, mesh, sh, d_grad_positions, d_grad_colors, s);
             check_launch("scatter gradients");
         }
         rec_event(r, 8, s);

@@ -400,8 +400,8 @@ __global__ void __launch_bounds__(kTile * kTile, 2) kb_adjoint(const BatchView* 
                                                             const float* __restrict__ tfinal,
                                                             const uint32_t* __restrict__ term,
                                                             float4* __restrict__ grad_rows,
-                                                            float4* __restrict__ view_rows,
-                                                            const uint32_t* __restrict__ ok) {
+                                                            float4* __restrict__ view_rows, size_t copy_stride,
+                                                            uint32_t copies, const uint32_t* __restrict__ ok) {
     __shared__ float4 vcache4[3 * kTile * kTile];
     __shared__ float vcache1[3 * kTile * kTile];
     if (!batch_ok(ok)) return;
@@ -409,7 +409,8 @@ __global__ void __launch_bounds__(kTile * kTile, 2) kb_adjoint(const BatchView* 
     if (!tile_pixel(views, nviews, v, px, py)) return;
     const BatchView& bv = views[v];
     if (bv.grad_slot < 0 || bv.dimage == nullptr) return;
-    float4* rows = SCREEN ? view_rows + 2 * bv.vert_base : grad_rows + 2 * bv.grad_base;
+    float4* rows = SCREEN ? block_rows(view_rows, copies, copy_stride) + 2 * bv.vert_base
+                          : grad_rows + 2 * bv.grad_base;
     if constexpr (SCREEN) {
         OrderedRowsSmem acc{rows, vcache4 + threadIdx.x, vcache1 + threadIdx.x, kTile * kTile};
         adjoint_pixel<OrderedRowsSmem, SCREEN>(px, py, offsets + bv.pix_base, records, bv.faces, vgeo + bv.vert_base,
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(kTile * kTile, 2) kb_adjoint(const BatchView* 
 // of the slot (one thread per view vertex; untouched vertices skipped).
 __global__ void __launch_bounds__(256) kb_view_rows(const BatchView* __restrict__ views, int nviews, u64 total,
                                                     const VGeo* __restrict__ vgeo,
-                                                    const float4* __restrict__ view_rows,
+                                                    const float4* __restrict__ view_rows, uint32_t copies,
                                                     float4* __restrict__ grad_rows, const uint32_t* __restrict__ ok) {
     if (!batch_ok(ok)) return;
     const u64 first = u64(blockIdx.x) * blockDim.x;
@@ -436,7 +437,8 @@ __global__ void __launch_bounds__(256) kb_view_rows(const BatchView* __restrict_
     const int v = view_of_item(g, first, nviews, [&](int i) { return views[i].vert_base; });
     const BatchView& bv = views[v];
     if (bv.grad_slot < 0 || bv.dimage == nullptr) return;
-    const float4 a = view_rows[2 * g], c = view_rows[2 * g + 1];
+    const float4 a = sum_copies(view_rows + 2 * g, copies, 2 * size_t(total)),
+                 c = sum_copies(view_rows + 2 * g + 1, copies, 2 * size_t(total));
     if (a.x == 0.f && a.y == 0.f && a.z == 0.f && c.x == 0.f && c.y == 0.f && c.z == 0.f && c.w == 0.f) return;
     const float3 w = screen_to_world(a, vgeo[g], bv.cam);
     float4* row = grad_rows + 2 * (bv.grad_base + (g - bv.vert_base));
@@ -582,7 +584,9 @@ struct dtv_batch {
     DevBuf<uint32_t> fill_order;    // items (view faces) in row-band order for the fill
     DevBuf<uint32_t> band_scratch;  // band counts and cursors of fill_order
     DevBuf<uint32_t> wide_list;     // [0] = n, then the items of the 64-bit raster path (count -> fill)
-    DevBuf<float4> view_rows;  // [tot_verts][2]: screen-space adjoint rows of each view (at its vert_base)
+    // [copies][tot_verts][2]: screen-space adjoint rows of each view (at its
+    // vert_base), in view_copies copies.
+    DevBuf<float4> view_rows;
     DevBuf<float4> dimage_internal;
     DevBuf<float> loss;
     DevBuf<int> step;
@@ -678,12 +682,18 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
     b->max_height = mh;
 }
 
+// Copies of the views' gradient rows (grad_copies on the mean view).
+uint32_t view_copies(const dtv_batch* b) {
+    const uint64_t n = b->nviews > 0 ? uint64_t(b->nviews) : 1;
+    return dtv::grad_copies((b->tot_verts + n - 1) / n, b->tot_pixels / n);
+}
+
 void ensure_scratch(dtv_batch* b, cudaStream_t s) {
     b->d_views.ensure(size_t(b->nviews), s);
     b->vproj.ensure(b->tot_verts ? b->tot_verts : 1, s);
     b->vfix.ensure(b->tot_verts ? b->tot_verts : 1, s);
     b->vgeo.ensure(b->tot_verts ? b->tot_verts : 1, s);
-    b->view_rows.ensure(2 * (b->tot_verts ? b->tot_verts : 1), s);
+    b->view_rows.ensure(2 * size_t(b->tot_verts ? b->tot_verts : 1) * view_copies(b), s);
     b->fill_order.ensure(b->tot_faces ? b->tot_faces : 1, s);
     b->band_scratch.ensure(2 * dtv::kFillBands, s);
     b->wide_list.ensure(b->tot_faces + 1, s);
@@ -803,15 +813,17 @@ void enqueue_adjoint(dtv_batch* b, const dtv::ShadeDev& sh, const uint32_t* okp,
     if (sh.use_abs_grad) {
         kb_adjoint<false><<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(
             b->d_views.ptr, b->nviews, b->offsets.ptr, b->records.ptr, b->vgeo.ptr, sh, b->tfinal.ptr, b->term.ptr,
-            b->grad_rows.ptr, b->view_rows.ptr, okp);
+            b->grad_rows.ptr, b->view_rows.ptr, 0, 1, okp);
         return;
     }
-    DTV_CK(cudaMemsetAsync(b->view_rows.ptr, 0, sizeof(float4) * 2 * size_t(b->tot_verts), s));
+    const uint32_t copies = view_copies(b);
+    const size_t stride = 2 * size_t(b->tot_verts);
+    DTV_CK(cudaMemsetAsync(b->view_rows.ptr, 0, sizeof(float4) * stride * copies, s));
     kb_adjoint<true><<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(
         b->d_views.ptr, b->nviews, b->offsets.ptr, b->records.ptr, b->vgeo.ptr, sh, b->tfinal.ptr, b->term.ptr,
-        b->grad_rows.ptr, b->view_rows.ptr, okp);
+        b->grad_rows.ptr, b->view_rows.ptr, stride, copies, okp);
     kb_view_rows<<<grid_for(b->tot_verts, 256, 0x7fffffffu), 256, 0, s>>>(
-        b->d_views.ptr, b->nviews, b->tot_verts, b->vgeo.ptr, b->view_rows.ptr, b->grad_rows.ptr, okp);
+        b->d_views.ptr, b->nviews, b->tot_verts, b->vgeo.ptr, b->view_rows.ptr, copies, b->grad_rows.ptr, okp);
 }
 
 // Enqueues project, count and scan; info gets the record total and whether it
@@ -886,6 +898,8 @@ int32_t dtv_batch_reserve(dtv_batch* b, uint64_t max_views, uint64_t max_vertice
         b->vproj.ensure(V, s);
         b->vfix.ensure(V, s);
         b->vgeo.ensure(V, s);
+        // Batches of small meshes hold copies of their rows: at most kGradRows
+        // rows per view, grown at the first such batch.
         b->view_rows.ensure(2 * V, s);
         // Fill order: a Kuhn-grid tet mesh has about 12 faces per vertex; a
         // batch with more faces grows it at its first render.

@@ -190,7 +190,8 @@ __global__ void __launch_bounds__(kTile * kCellRows, SCREEN ? 5 : 4) k_adjoint_c
     const u64* __restrict__ offsets, const u64* __restrict__ records, const uint4* __restrict__ faces,
     const uint2* __restrict__ f2t, const VGeo* __restrict__ vgeo, const float4* __restrict__ cell_colors, int W,
     int row0, int row1, CamDev cam, ShadeDev sh, const float4* __restrict__ dimage, const float* __restrict__ tfinal,
-    const uint32_t* __restrict__ term, float4* __restrict__ grad_rows, float4* __restrict__ grad_cells) {
+    const uint32_t* __restrict__ term, float4* __restrict__ row_copies, uint32_t V, uint32_t copies,
+    float4* __restrict__ cell_copies, uint32_t T, uint32_t ncell_copies) {
     const int px = blockIdx.x * kTile + tile_x<kTile>(threadIdx.x);
     const int py = row0 + int(blockIdx.y) * kCellRows + tile_y<kTile>(threadIdx.x);
     if (px >= W || py >= row1) return;
@@ -204,9 +205,11 @@ __global__ void __launch_bounds__(kTile * kCellRows, SCREEN ? 5 : 4) k_adjoint_c
     const float qx = float(px) + 0.5f, qy = float(py) + 0.5f;
     const bool use_abs = sh.use_abs_grad != 0;
     const float atten = sh.atten;
+    float4* grad_rows = block_rows(row_copies, copies, 2 * size_t(V));
+    float4* grad_cells = block_rows(cell_copies, ncell_copies, T);
     // Float-float transmittance and its adjoint (dtv_segment.cuh).
     TransF gT{g.x * sh.clear[0] + g.y * sh.clear[1] + g.z * sh.clear[2] + g.w * (sh.clear[3] - 1.f), 0.f};
-    TransF T{tfinal[p], 0.f};
+    TransF Tr{tfinal[p], 0.f};
     if constexpr (SCREEN) {
         // Dependent loads record -> face -> vertex rows one step ahead, as in
         // adjoint_pixel_carried.
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__(kTile * kCellRows, SCREEN ? 5 : 4) k_adjoint_c
                 pf_f = f2t[fni];
                 if (i >= 3) fni = uint32_t(records[beg + i - 3]) >> 2;
             }
-            const float g_t = cell_segment_adjoint(ff.tets, fb.tets, ff.z, fb.z, cell_colors, atten, false, g, T, gT,
+            const float g_t = cell_segment_adjoint(ff.tets, fb.tets, ff.z, fb.z, cell_colors, atten, false, g, Tr, gT,
                                                    grad_cells);
             frag_pos_carried(fb, gz_b + g_t, ff.keep, acc);
             fb = ff;
@@ -247,7 +250,7 @@ __global__ void __launch_bounds__(kTile * kCellRows, SCREEN ? 5 : 4) k_adjoint_c
         const uint4 ff = faces[ffi];
         const uint2 pf = f2t[ffi];
         const float zf = face_depth(ff, vgeo, qx, qy);
-        const float g_t = cell_segment_adjoint(pf, pb, zf, zb, cell_colors, atten, use_abs, g, T, gT, grad_cells);
+        const float g_t = cell_segment_adjoint(pf, pb, zf, zb, cell_colors, atten, use_abs, g, Tr, gT, grad_cells);
         gz_b += g_t;
         frag_position_grads(fb, qx, qy, vgeo, cam, gz_b, use_abs, grad_rows);
         fb = ff;
@@ -260,11 +263,12 @@ __global__ void __launch_bounds__(kTile * kCellRows, SCREEN ? 5 : 4) k_adjoint_c
 
 template <bool SCREEN>
 __global__ void __launch_bounds__(256) k_scatter_positions(const float4* __restrict__ rows, uint32_t V,
+                                                           uint32_t copies,
                                                            float* __restrict__ grad_pos,
                                                            const VGeo* __restrict__ vgeo, CamDev cam) {
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
-    float4 a = rows[2 * size_t(v)];
+    float4 a = sum_copies(rows + 2 * size_t(v), copies, 2 * size_t(V));
     if (SCREEN) {
         const float3 w = screen_to_world(a, vgeo[v], cam);
         a = make_float4(w.x, w.y, w.z, 0.f);
@@ -290,7 +294,8 @@ void launch_composite_cells(const u64* offsets, const u64* records, const uint4*
 void launch_adjoint_cells_rows(const u64* offsets, const u64* records, const uint4* faces,
                                const uint32_t* face_to_tet, const VGeo* vgeo, const float4* cell_colors,
                                const CamDev& cam, const ShadeDev& sh, const float4* dimage, const float* tfinal,
-                               const uint32_t* term, int row0, int row1, float4* grad_rows, float4* grad_cells,
+                               const uint32_t* term, int row0, int row1, float4* grad_rows, uint32_t V,
+                               uint32_t copies, float4* grad_cells, uint32_t T, uint32_t cell_copies,
                                cudaStream_t s) {
     if (row1 <= row0) return;
     dim3 grid((cam.W + kTile - 1) / kTile, (row1 - row0 + kCellRows - 1) / kCellRows);
@@ -298,21 +303,34 @@ void launch_adjoint_cells_rows(const u64* offsets, const u64* records, const uin
         k_adjoint_cells<false><<<grid, kTile * kCellRows, 0, s>>>(offsets, records, faces,
                                                               reinterpret_cast<const uint2*>(face_to_tet), vgeo,
                                                               cell_colors, cam.W, row0, row1, cam, sh, dimage, tfinal,
-                                                              term, grad_rows, grad_cells);
+                                                              term, grad_rows, V, copies, grad_cells, T, cell_copies);
     else
         k_adjoint_cells<true><<<grid, kTile * kCellRows, 0, s>>>(offsets, records, faces,
                                                              reinterpret_cast<const uint2*>(face_to_tet), vgeo,
                                                              cell_colors, cam.W, row0, row1, cam, sh, dimage, tfinal,
-                                                             term, grad_rows, grad_cells);
+                                                             term, grad_rows, V, copies, grad_cells, T, cell_copies);
 }
 
-void launch_scatter_positions(const float4* grad_rows, uint32_t V, float* grad_pos, cudaStream_t s,
+__global__ void __launch_bounds__(128) k_add_cell_copies(const float4* __restrict__ base, uint32_t T, uint32_t copies,
+                                                         float4* __restrict__ grad_cells) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= T) return;
+    const float4 a = sum_copies(base + t, copies, T), c = grad_cells[t];
+    grad_cells[t] = make_float4(c.x + a.x, c.y + a.y, c.z + a.z, c.w + a.w);
+}
+
+void launch_add_cell_copies(const float4* copies_base, uint32_t T, uint32_t copies, float4* grad_cells,
+                            cudaStream_t s) {
+    if (T) k_add_cell_copies<<<(T + 127) / 128, 128, 0, s>>>(copies_base, T, copies, grad_cells);
+}
+
+void launch_scatter_positions(const float4* grad_rows, uint32_t V, uint32_t copies, float* grad_pos, cudaStream_t s,
                               const VGeo* vgeo, const CamDev* cam) {
     if (V == 0) return;
     if (vgeo)
-        k_scatter_positions<true><<<(V + 255) / 256, 256, 0, s>>>(grad_rows, V, grad_pos, vgeo, *cam);
+        k_scatter_positions<true><<<(V + 255) / 256, 256, 0, s>>>(grad_rows, V, copies, grad_pos, vgeo, *cam);
     else
-        k_scatter_positions<false><<<(V + 255) / 256, 256, 0, s>>>(grad_rows, V, grad_pos, nullptr, CamDev{});
+        k_scatter_positions<false><<<(V + 255) / 256, 256, 0, s>>>(grad_rows, V, copies, grad_pos, nullptr, CamDev{});
 }
 
 }  // namespace dtv

@@ -106,19 +106,30 @@ void launch_composite(const unsigned long long* offsets, const unsigned long lon
                       const VGeo* vgeo, const float4* colors, int W, int H, const ShadeDev& sh, float4* image,
                       float* tfinal, uint32_t* term, cudaStream_t s, int row0 = 0, int row1 = -1, int tile = 0,
                       const uint32_t* gate = nullptr);
-void launch_adjoint(const unsigned long long* offsets, const unsigned long long* records, const uint4* faces,
-                    const VGeo* vgeo, const float4* colors, const CamDev& cam, const ShadeDev& sh,
-                    const float4* dimage, const float* tfinal, const uint32_t* term, uint32_t V,
-                    float4* grad_rows, float* grad_pos, float4* grad_col, cudaStream_t s);
-// Adjoint of pixel rows [row0, row1) into grad_rows (no clearing, no scatter).
+// Copies of the gradient rows of a mesh with few vertices (or cells): all
+// pixels' atomics on a few thousand rows wait for one another in L2, so the
+// blocks are spread over a power of two of copies with up to kGradRows rows in
+// all, which the scatter sums.  Measured (adjoint, us, one copy -> copies):
+// 8^3 at 800^2 1,326 -> 337, 16^3 at 1000^2 1,890 -> 969, 32^3 at 700^2 992 ->
+// 954, per-cell 10^3 at 600^2 440 -> 207; 2^15, 2^16 and 2^18 rows gave 1,117,
+// 983 and 975 at 16^3.  One copy per 8192 pixels at most: a small image has no
+// contention to spread, and clearing and summing 64 copies cost 12 us.
+constexpr uint64_t kGradRows = 1u << 17;
+inline uint32_t grad_copies(uint64_t rows, uint64_t pixels) {
+    uint32_t c = 1;
+    while (c < 64 && 2 * uint64_t(c) * rows <= kGradRows && 2 * uint64_t(c) * 8192 <= pixels) c *= 2;
+    return c;
+}
+// Adjoint of pixel rows [row0, row1) into the copies of grad_rows ([copies][V][2];
+// no clearing, no scatter).
 void launch_adjoint_rows(const unsigned long long* offsets, const unsigned long long* records, const uint4* faces,
                          const VGeo* vgeo, const float4* colors, const CamDev& cam, const ShadeDev& sh,
                          const float4* dimage, const float* tfinal, const uint32_t* term, int row0, int row1,
-                         float4* grad_rows, cudaStream_t s, int tile = 0);
+                         float4* grad_rows, uint32_t V, uint32_t copies, cudaStream_t s, int tile = 0);
 // Adds the interleaved [V][2] gradient rows into grad_pos [V,3] / grad_col [V,4].
 // screen_vgeo / cam: rows hold screen-space position adjoints of that camera
 // (the list adjoint without absolute gradients); nullptr: world-space rows.
-void launch_scatter_grads(const float4* grad_rows, uint32_t V, float* grad_pos, float4* grad_col, cudaStream_t s,
+void launch_scatter_grads(const float4* grad_rows, uint32_t V, uint32_t copies, float* grad_pos, float4* grad_col, cudaStream_t s,
                           const VGeo* screen_vgeo = nullptr, const CamDev* cam = nullptr);
 
 void launch_loss_l2(const float* image, const float* target, uint64_t n, float scale, float* adjoint,
@@ -136,12 +147,16 @@ void launch_adjoint_cells_rows(const unsigned long long* offsets, const unsigned
                                const uint4* faces, const uint32_t* face_to_tet, const VGeo* vgeo,
                                const float4* cell_colors, const CamDev& cam, const ShadeDev& sh, const float4* dimage,
                                const float* tfinal, const uint32_t* term, int row0, int row1, float4* grad_rows,
-                               float4* grad_cells, cudaStream_t s);
+                               uint32_t V, uint32_t copies, float4* grad_cells, uint32_t T, uint32_t cell_copies,
+                               cudaStream_t s);
+// grad_cells[T] += the sum of the copies.
+void launch_add_cell_copies(const float4* copies_base, uint32_t T, uint32_t copies, float4* grad_cells,
+                            cudaStream_t s);
 // Adds the position part of the [V][2] gradient rows into grad_pos [V,3]
 // (vgeo non-null: the rows hold screen-space adjoints, converted per vertex
 // with the render's camera, as the per-cell adjoint leaves them without
 // absolute gradients).
-void launch_scatter_positions(const float4* grad_rows, uint32_t V, float* grad_pos, cudaStream_t s,
+void launch_scatter_positions(const float4* grad_rows, uint32_t V, uint32_t copies, float* grad_pos, cudaStream_t s,
                               const VGeo* vgeo = nullptr, const CamDev* cam = nullptr);
 
 // Ray-tet path (dtv_raytet.cu).
@@ -156,7 +171,7 @@ void launch_walk_adjoint(const unsigned long long* b_offsets, const unsigned lon
                          const uint32_t* tet_faces, const uint32_t* cells, const uint8_t* tet_flip,
                          uint32_t num_tets, const int2* vfix, const VGeo* vgeo,
                          const float4* colors, const CamDev& cam, const ShadeDev& sh, const float4* dimage,
-                         const float* tfinal, const uint4* wstate, uint32_t V, float4* grad_rows, float* grad_pos,
+                         const float* tfinal, const uint4* wstate, uint32_t V, float4* grad_rows, uint32_t copies, float* grad_pos,
                          float4* grad_col, cudaStream_t s);
 
 // Fragment lists by walking the mesh (dtv_walk.cu).

@@ -1242,12 +1242,14 @@ void launch_composite(const u64* offsets, const u64* records, const uint4* faces
 // blocks per SM at 128 registers): measured 1.5 % faster than 256-thread blocks
 // at two per SM, the same occupancy with finer scheduling of uneven lists.
 constexpr int kAdjThreads = 128;
-template <int TX, bool SCREEN>
+// COPIES: more than one copy of the gradient rows (with one, the rows' address
+// stays a kernel parameter: the screen-space variant has no register left).
+template <int TX, bool SCREEN, bool COPIES>
 __global__ void __launch_bounds__(kAdjThreads, 2 * 256 / kAdjThreads) k_adjoint(
     const u64* __restrict__ offsets, const u64* __restrict__ records, const uint4* __restrict__ faces,
     const VGeo* __restrict__ vgeo, const float4* __restrict__ colors, int W, int row0, int row1, CamDev cam,
     ShadeDev sh, const float4* __restrict__ dimage, const float* __restrict__ tfinal,
-    const uint32_t* __restrict__ term, float4* __restrict__ grad_rows) {
+    const uint32_t* __restrict__ term, float4* __restrict__ grad_rows, uint32_t V, uint32_t copies) {
     __shared__ float4 vcache4[3 * kAdjThreads];
     __shared__ float vcache1[3 * kAdjThreads];
     constexpr int TY = kAdjThreads / TX;
@@ -1257,11 +1259,11 @@ __global__ void __launch_bounds__(kAdjThreads, 2 * 256 / kAdjThreads) k_adjoint(
     // Screen-space rows: the ordered register cache (order_like); world-space
     // rows (absolute gradients): the shared-memory cache.
     if constexpr (SCREEN) {
-        OrderedRows acc{grad_rows};
+        OrderedRows acc{COPIES ? block_rows(grad_rows, copies, 2 * size_t(V)) : grad_rows};
         adjoint_pixel<OrderedRows, SCREEN>(px, py, offsets, records, faces, vgeo, colors, W, cam, sh, dimage, tfinal,
                                            term, acc);
     } else {
-        VertCache acc{grad_rows, vcache4 + threadIdx.x, vcache1 + threadIdx.x, kAdjThreads};
+        VertCache acc{COPIES ? block_rows(grad_rows, copies, 2 * size_t(V)) : grad_rows, vcache4 + threadIdx.x, vcache1 + threadIdx.x, kAdjThreads};
         adjoint_pixel<VertCache, SCREEN>(px, py, offsets, records, faces, vgeo, colors, W, cam, sh, dimage, tfinal,
                                          term, acc);
     }
@@ -1270,14 +1272,14 @@ __global__ void __launch_bounds__(kAdjThreads, 2 * 256 / kAdjThreads) k_adjoint(
 // Adds the interleaved rows into the caller's gradient buffers (SCREEN: the
 // position rows hold screen-space adjoints, converted here per vertex).
 template <bool SCREEN>
-__global__ void __launch_bounds__(256) k_scatter_grads(const float4* __restrict__ rows, uint32_t V,
+__global__ void __launch_bounds__(128) k_scatter_grads(const float4* __restrict__ rows, uint32_t V, uint32_t copies,
                                                        float* __restrict__ grad_pos,
                                                        float4* __restrict__ grad_col,
                                                        const VGeo* __restrict__ vgeo, CamDev cam) {
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
-    float4 a = rows[2 * size_t(v)];
-    const float4 b = rows[2 * size_t(v) + 1];
+    float4 a = sum_copies(rows + 2 * size_t(v), copies, 2 * size_t(V));
+    const float4 b = sum_copies(rows + 2 * size_t(v) + 1, copies, 2 * size_t(V));
     if (SCREEN) {
         const float3 w = screen_to_world(a, vgeo[v], cam);
         a = make_float4(w.x, w.y, w.z, 0.f);
@@ -1290,55 +1292,48 @@ __global__ void __launch_bounds__(256) k_scatter_grads(const float4* __restrict_
     grad_col[v] = make_float4(c.x + b.x, c.y + b.y, c.z + b.z, c.w + b.w);
 }
 
-void launch_adjoint(const u64* offsets, const u64* records, const uint4* faces, const VGeo* vgeo,
-                    const float4* colors, const CamDev& cam, const ShadeDev& sh, const float4* dimage,
-                    const float* tfinal, const uint32_t* term, uint32_t V, float4* grad_rows, float* grad_pos,
-                    float4* grad_col, cudaStream_t s) {
-    cudaMemsetAsync(grad_rows, 0, sizeof(float4) * 2 * size_t(V), s);
-    launch_adjoint_rows(offsets, records, faces, vgeo, colors, cam, sh, dimage, tfinal, term, 0, cam.H, grad_rows,
-                        s);
-    launch_scatter_grads(grad_rows, V, grad_pos, grad_col, s, sh.use_abs_grad ? nullptr : vgeo, &cam);
-}
-
 template <int TX>
 void adjoint_tiles(const u64* offsets, const u64* records, const uint4* faces, const VGeo* vgeo,
                    const float4* colors, const CamDev& cam, const ShadeDev& sh, const float4* dimage,
-                   const float* tfinal, const uint32_t* term, int row0, int row1, float4* grad_rows, cudaStream_t s) {
+                   const float* tfinal, const uint32_t* term, int row0, int row1, float4* grad_rows, uint32_t V,
+                   uint32_t copies, cudaStream_t s) {
     constexpr int TY = kAdjThreads / TX;
     dim3 grid((cam.W + TX - 1) / TX, (row1 - row0 + TY - 1) / TY);
     // Rows in screen space unless absolute gradients are asked for (see
     // frag_vertex_grads); launch_scatter_grads converts with the same rule.
+    auto go = [&](auto k) {
+        k<<<grid, kAdjThreads, 0, s>>>(offsets, records, faces, vgeo, colors, cam.W, row0, row1, cam, sh, dimage, tfinal,
+                                       term, grad_rows, V, copies);
+    };
     if (sh.use_abs_grad)
-        k_adjoint<TX, false><<<grid, kAdjThreads, 0, s>>>(offsets, records, faces, vgeo, colors, cam.W, row0, row1, cam, sh,
-                                                  dimage, tfinal, term, grad_rows);
+        copies > 1 ? go(k_adjoint<TX, false, true>) : go(k_adjoint<TX, false, false>);
     else
-        k_adjoint<TX, true><<<grid, kAdjThreads, 0, s>>>(offsets, records, faces, vgeo, colors, cam.W, row0, row1, cam, sh,
-                                                 dimage, tfinal, term, grad_rows);
+        copies > 1 ? go(k_adjoint<TX, true, true>) : go(k_adjoint<TX, true, false>);
 }
 
 void launch_adjoint_rows(const u64* offsets, const u64* records, const uint4* faces, const VGeo* vgeo,
                          const float4* colors, const CamDev& cam, const ShadeDev& sh, const float4* dimage,
-                         const float* tfinal, const uint32_t* term, int row0, int row1, float4* grad_rows,
-                         cudaStream_t s, int tile) {
+                         const float* tfinal, const uint32_t* term, int row0, int row1, float4* grad_rows, uint32_t V,
+                         uint32_t copies, cudaStream_t s, int tile) {
     if (row1 <= row0) return;
     if (tile == 1)
         adjoint_tiles<32>(offsets, records, faces, vgeo, colors, cam, sh, dimage, tfinal, term, row0, row1, grad_rows,
-                          s);
+                          V, copies, s);
     else if (tile == 2)
         adjoint_tiles<8>(offsets, records, faces, vgeo, colors, cam, sh, dimage, tfinal, term, row0, row1, grad_rows,
-                         s);
+                          V, copies, s);
     else
         adjoint_tiles<16>(offsets, records, faces, vgeo, colors, cam, sh, dimage, tfinal, term, row0, row1, grad_rows,
-                          s);
+                          V, copies, s);
 }
 
-void launch_scatter_grads(const float4* grad_rows, uint32_t V, float* grad_pos, float4* grad_col, cudaStream_t s,
-                          const VGeo* screen_vgeo, const CamDev* cam) {
+void launch_scatter_grads(const float4* grad_rows, uint32_t V, uint32_t copies, float* grad_pos, float4* grad_col,
+                          cudaStream_t s, const VGeo* screen_vgeo, const CamDev* cam) {
     if (!V) return;
     if (screen_vgeo)
-        k_scatter_grads<true><<<(V + 255) / 256, 256, 0, s>>>(grad_rows, V, grad_pos, grad_col, screen_vgeo, *cam);
+        k_scatter_grads<true><<<(V + 127) / 128, 128, 0, s>>>(grad_rows, V, copies, grad_pos, grad_col, screen_vgeo, *cam);
     else
-        k_scatter_grads<false><<<(V + 255) / 256, 256, 0, s>>>(grad_rows, V, grad_pos, grad_col, nullptr, CamDev{});
+        k_scatter_grads<false><<<(V + 127) / 128, 128, 0, s>>>(grad_rows, V, copies, grad_pos, grad_col, nullptr, CamDev{});
 }
 
 // ---------------------------------------------------------------------------

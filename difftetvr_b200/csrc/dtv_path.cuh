@@ -17,6 +17,24 @@ __device__ __forceinline__ int tile_x(uint32_t t) { return int((t >> 5) % (TX / 
 template <int TX>
 __device__ __forceinline__ int tile_y(uint32_t t) { return int((t >> 5) / (TX / 8) * 4 + ((t >> 3) & 3u)); }
 
+// The copy of the gradient rows (`rows` float4 each) that this block adds into
+// (grad_copies, a power of two).
+__device__ __forceinline__ float4* block_rows(float4* base, uint32_t copies, size_t rows) {
+    const uint32_t b = blockIdx.x + blockIdx.y * gridDim.x;
+    return base + size_t(b & (copies - 1u)) * rows;
+}
+
+// Sum of a row's copies, `stride` float4 apart.
+__device__ __forceinline__ float4 sum_copies(const float4* __restrict__ p, uint32_t copies, size_t stride) {
+    float4 s = p[0];
+#pragma unroll 8
+    for (uint32_t k = 1; k < copies; ++k) {
+        const float4 q = p[k * stride];
+        s = make_float4(s.x + q.x, s.y + q.y, s.z + q.z, s.w + q.w);
+    }
+    return s;
+}
+
 // ---------------------------------------------------------------------------
 // (a)+(b) face rasterisation, warp-cooperative.  Each lane of a warp sets up
 // one face (projected fixed-point vertices, orientation, clipped bounding box)

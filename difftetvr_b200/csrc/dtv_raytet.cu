@@ -314,7 +314,8 @@ __global__ void __launch_bounds__(kTile * kTile, 2) k_walk_adjoint(
     const u64* __restrict__ b_offsets, const u64* __restrict__ b_records, const uint32_t* __restrict__ bf_global,
     const uint4* __restrict__ faces, const uint32_t* __restrict__ f2t, TetTopo tt, uint32_t num_tets, const int2* __restrict__ vfix, const VGeo* __restrict__ vgeo,
     const float4* __restrict__ colors, CamDev cam, ShadeDev sh, const float4* __restrict__ dimage,
-    const float* __restrict__ tfinal, const uint4* __restrict__ wstate, float4* __restrict__ grad_rows) {
+    const float* __restrict__ tfinal, const uint4* __restrict__ wstate, float4* __restrict__ row_copies, uint32_t V,
+    uint32_t copies) {
     const int px = blockIdx.x * kTile + tile_x<kTile>(threadIdx.x);
     const int py = blockIdx.y * kTile + tile_y<kTile>(threadIdx.x);
     if (px >= cam.W || py >= cam.H) return;
@@ -335,6 +336,7 @@ __global__ void __launch_bounds__(kTile * kTile, 2) k_walk_adjoint(
     int b = int(ws.z);
     uint32_t fx = tet_face_at(tt, vfix, t, fe, false, px, py);
     if (fx == kNoTet) return;
+    float4* grad_rows = block_rows(row_copies, copies, 2 * size_t(V));
     if constexpr (SCREEN) {
         __shared__ float4 vcache4[3 * kTile * kTile];
         __shared__ float vcache1[3 * kTile * kTile];
@@ -413,8 +415,9 @@ void launch_walk_adjoint(const u64* b_offsets, const u64* b_records, const uint3
                          const uint8_t* tet_flip, uint32_t num_tets,
                          const int2* vfix, const VGeo* vgeo, const float4* colors, const CamDev& cam,
                          const ShadeDev& sh, const float4* dimage, const float* tfinal, const uint4* wstate,
-                         uint32_t V, float4* grad_rows, float* grad_pos, float4* grad_col, cudaStream_t s) {
-    cudaMemsetAsync(grad_rows, 0, sizeof(float4) * 2 * size_t(V), s);
+                         uint32_t V, float4* grad_rows, uint32_t copies, float* grad_pos, float4* grad_col,
+                         cudaStream_t s) {
+    cudaMemsetAsync(grad_rows, 0, sizeof(float4) * 2 * size_t(V) * copies, s);
     dim3 grid((cam.W + kTile - 1) / kTile, (cam.H + kTile - 1) / kTile);
     const TetTopo tt{reinterpret_cast<const uint4*>(tet_faces), reinterpret_cast<const uint4*>(cells), tet_flip};
     // Screen-space position rows unless absolute gradients are asked for
@@ -422,12 +425,12 @@ void launch_walk_adjoint(const u64* b_offsets, const u64* b_records, const uint3
     if (sh.use_abs_grad)
         k_walk_adjoint<false><<<grid, kTile * kTile, 0, s>>>(b_offsets, b_records, bf_global, faces, face_to_tet,
                                                              tt, num_tets, vfix, vgeo, colors, cam, sh, dimage,
-                                                             tfinal, wstate, grad_rows);
+                                                             tfinal, wstate, grad_rows, V, copies);
     else
         k_walk_adjoint<true><<<grid, kTile * kTile, 0, s>>>(b_offsets, b_records, bf_global, faces, face_to_tet,
                                                             tt, num_tets, vfix, vgeo, colors, cam, sh, dimage,
-                                                            tfinal, wstate, grad_rows);
-    launch_scatter_grads(grad_rows, V, grad_pos, grad_col, s, sh.use_abs_grad ? nullptr : vgeo, &cam);
+                                                            tfinal, wstate, grad_rows, V, copies);
+    launch_scatter_grads(grad_rows, V, copies, grad_pos, grad_col, s, sh.use_abs_grad ? nullptr : vgeo, &cam);
 }
 
 }  // namespace dtv
