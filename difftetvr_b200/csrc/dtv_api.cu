@@ -692,9 +692,10 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         }
         if (!walk) {
             rec_event(r, 3, s);
-            order_faces();
+            if (!raytet) order_faces();
             dtv::launch_raster_fill(rfaces, uint32_t(F), r->vproj.ptr, r->vfix.ptr, W, H, r->counts.ptr,
-                                    r->offsets.ptr, r->records.ptr, s, 0, -1, r->fill_order.ptr, r->wide_list.ptr);
+                                    r->offsets.ptr, r->records.ptr, s, 0, -1, raytet ? nullptr : r->fill_order.ptr,
+                                    raytet ? nullptr : r->wide_list.ptr);
             check_launch("raster fill");
             rec_event(r, 4, s);
             dtv::launch_sort(r->offsets.ptr, r->records.ptr, uint32_t(P), r->long_list.ptr, s, nullptr,

@@ -185,7 +185,11 @@ __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ v
     const u64 first = u64(blockIdx.x) * blockDim.x;
     u64 i = first + threadIdx.x;
     bool mine = true;
-    if (FILL && per_warp != 32u) {
+    // As k_raster: faces per warp of the fill, threads per face of the count.
+    const uint32_t per_face = 32u / per_warp, sub = FILL ? 0u : uint32_t(i) & (per_face - 1u);
+    if (!FILL) {
+        i /= per_face;
+    } else if (per_warp != 32u) {
         const uint32_t l = threadIdx.x & 31u;
         i = (i >> 5) * per_warp + l;
         mine = l < per_warp;
@@ -196,18 +200,19 @@ __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ v
     if (mine && i < total) {
         g = order ? u64(order[i]) : i;
         auto base = [&](int k) { return kSet == kBoundaryFaces ? views[k].bface_base : views[k].face_base; };
-        const int v = (FILL || order) ? find_index(g, nviews, base) : view_of_item(g, first, nviews, base);
+        const int v = (FILL || order) ? find_index(g, nviews, base) : view_of_item(g, first / per_face, nviews, base);
         const BatchView& bv = views[v];
         set = raster_setup(uint32_t(g - base(v)), kSet == kBoundaryFaces ? bv.walk.bfaces : bv.faces,
                            vfix + bv.vert_base, uint32_t(bv.vert_base), int(bv.W), 0, int(bv.H), bv.pix_base, J);
         live = set && (J.wide != 0) == WIDE;
     }
     if constexpr (!FILL) {
-        if (live) count_face<typename std::conditional<WIDE, long long, int>::type>(J, counts);
+        if (live)
+            count_face<typename std::conditional<WIDE, long long, int>::type>(J, counts, int(sub), int(per_face));
         if (!WIDE && wide_list) {
             // The items of the 64-bit path, for its count and fill launches
             // (wide_list[0] = how many, then the items).
-            const bool wide = set && J.wide != 0;
+            const bool wide = set && J.wide != 0 && sub == 0u;
             const unsigned m = __ballot_sync(0xffffffffu, wide);
             if (m) {
                 const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
@@ -222,12 +227,12 @@ __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ v
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         if (live) jobs[w][lane] = J;
         raster_warp<FILL, WIDE, kSet == kRestFaces>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts,
-                                                    offsets, records);
+                                                    offsets, records, int(blockIdx.y), int(gridDim.y));
     }
 }
 
-// The 64-bit items listed by the count (wide_list), 32 per warp and step over
-// a fixed grid: the count (one thread per face) or the fill (raster_warp).
+// The 64-bit items listed by the count (wide_list) over a fixed grid: the count
+// (one item per warp) or the fill (32 per warp and step, raster_warp).
 template <bool FILL, bool REST = false>
 __global__ void __launch_bounds__(128) kb_raster_listed(const BatchView* __restrict__ views, int nviews,
                                                         const float4* __restrict__ vproj,
@@ -240,22 +245,25 @@ __global__ void __launch_bounds__(128) kb_raster_listed(const BatchView* __restr
     __shared__ RasterJob jobs[4][32];
     const uint32_t n = wide_list[0];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x + uint32_t(w) * 32u; base < n; base += stride) {
-        const uint32_t i = base + uint32_t(lane);
-        RasterJob J;
-        bool live = false;
-        if (i < n) {
-            const u64 g = wide_list[1 + i];
-            const int v = find_index(g, nviews, [&](int k) { return views[k].face_base; });
-            const BatchView& bv = views[v];
-            live = raster_setup(uint32_t(g - bv.face_base), bv.faces, vfix + bv.vert_base, uint32_t(bv.vert_base),
-                                int(bv.W), 0, int(bv.H), bv.pix_base, J) &&
-                   J.wide != 0;
+    auto setup = [&](uint32_t i, RasterJob& J) {
+        const u64 g = wide_list[1 + i];
+        const int v = find_index(g, nviews, [&](int k) { return views[k].face_base; });
+        const BatchView& bv = views[v];
+        return raster_setup(uint32_t(g - bv.face_base), bv.faces, vfix + bv.vert_base, uint32_t(bv.vert_base),
+                            int(bv.W), 0, int(bv.H), bv.pix_base, J) &&
+               J.wide != 0;
+    };
+    if constexpr (!FILL) {
+        for (uint32_t i = blockIdx.x * 4 + uint32_t(w); i < n; i += gridDim.x * 4) {
+            RasterJob J;
+            if (setup(i, J)) count_face<long long>(J, counts, lane, 32);
         }
-        if constexpr (!FILL) {
-            if (live) count_face<long long>(J, counts);
-        } else {
+    } else {
+        const uint32_t stride = gridDim.x * blockDim.x;
+        for (uint32_t base = blockIdx.x * blockDim.x + uint32_t(w) * 32u; base < n; base += stride) {
+            const uint32_t i = base + uint32_t(lane);
+            RasterJob J;
+            const bool live = i < n && setup(i, J);
             if (live) jobs[w][lane] = J;
             raster_warp<FILL, true, REST>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets,
                                           records);
@@ -727,12 +735,13 @@ void upload_views(dtv_batch* b, cudaStream_t s) {
 // along each view's rows (kb_row_prefix).
 void launch_kb_count(dtv_batch* b, cudaStream_t s) {
     using namespace dtv;
-    const unsigned blocks = grid_for(b->tot_faces, 128, 0x7fffffffu);
+    const uint32_t per_face = count_threads_per_face(b->tot_faces);
+    const unsigned blocks = grid_for(b->tot_faces * per_face, 128, 0x7fffffffu);
     DTV_CK(cudaMemsetAsync(b->wide_list.ptr, 0, sizeof(uint32_t), s));
     kb_raster<false, false><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr, b->vfix.ptr,
                                                    b->counts.ptr, nullptr, nullptr, nullptr, nullptr,
-                                                   b->wide_list.ptr, 32u);
-    kb_raster_listed<false><<<148, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
+                                                   b->wide_list.ptr, 32u / per_face);
+    kb_raster_listed<false><<<148 * 8, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
                                                 nullptr, nullptr, nullptr, b->wide_list.ptr);
     dim3 grid(unsigned(b->max_height + 7) / 8, unsigned(b->nviews));
     kb_row_prefix<<<grid, 256, 0, s>>>(b->d_views.ptr, b->counts.ptr);
@@ -771,9 +780,9 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
     const uint32_t* okp = guarded ? &b->info.ptr->ok : nullptr;
     if (b->walk) {
         if (b->tot_bfaces) {
-            // Few faces are spread over more warps (as launch_raster_fill).
-            const uint32_t per_warp = uint32_t(std::min<u64>(32, std::max<u64>(1, b->tot_bfaces / (148 * 32))));
-            const unsigned bb = grid_for(b->tot_bfaces, 4 * per_warp, 0x7fffffffu);
+            const FillSplit sp = fill_split(b->tot_bfaces, b->max_height);
+            const uint32_t per_warp = sp.per_warp;
+            const dim3 bb(grid_for(b->tot_bfaces, 4 * per_warp, 0x7fffffffu), sp.parts);
             kb_raster<true, false, kBoundaryFaces><<<bb, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_bfaces,
                                                                       b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
                                                                       b->offsets.ptr, b->records.ptr, okp, nullptr,

@@ -29,6 +29,31 @@ struct MeshHost {
 // Builds faces from cells (restates buildFacesSlim, TetMesh.cpp:1218-1268).
 void build_faces(const uint32_t* cells, uint64_t T, uint64_t V, MeshHost& out);
 
+// Split of the raster passes over few faces (a small mesh, or the boundary
+// faces alone), which one thread (count) or 32 faces per warp (fill) would
+// leave to a few warps, row after row.  Measured (us): count of 6^3 at 200^2
+// (64-bit boxes) 49 -> 18, of 8^3 at 800^2 125 -> 36, of 16^3 at 1000^2 131 ->
+// 55; fill of the boundary faces 12^3 at 600^2 904 -> 56, 8^3 at 64^2 53 -> 13,
+// 64^3 at 1024^2 (10 -> 5 faces per warp) 96 -> 88.
+// Count: threads per face (a power of two), each taking every so many rows.
+inline uint32_t count_threads_per_face(uint64_t F) {
+    uint32_t n = 1;
+    while (n < 32 && F * n * 2 <= 148 * 2048) n *= 2;
+    return n;
+}
+// Fill: faces that a warp takes one after another, and, with one face per warp
+// and still few warps, the warps that share a face's groups of 32 rows (images
+// of few rows have none to share).
+struct FillSplit {
+    uint32_t per_warp, parts;
+};
+inline FillSplit fill_split(uint64_t F, uint64_t image_rows) {
+    if (F == 0) F = 1;
+    uint64_t w = F / (148 * 64), p = 148 * 64 / F;
+    if (p > 1 + image_rows / 128) p = 1 + image_rows / 128;
+    return FillSplit{uint32_t(w < 1 ? 1 : (w > 32 ? 32 : w)), uint32_t(p < 1 ? 1 : (p > 16 ? 16 : p))};
+}
+
 // Launch wrappers (dtv_kernels.cu).  All run on `s`.
 // rows (optional): the vertices' walk rows as well; clipped (optional): set to
 // 1 when a vertex is not projected.

@@ -57,10 +57,14 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster(const uint4* __res
                                                               uint32_t per_warp) {
     if (gate && *gate == 0u) return;
     // The fill gives each warp per_warp <= 32 faces, which it takes one at a
-    // time; the count takes one face per thread.
+    // time; the count takes 32 / per_warp threads per face (a power of two),
+    // each every so many rows.
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     bool mine = true;
-    if (FILL && per_warp != 32u) {
+    const uint32_t per_face = 32u / per_warp, sub = FILL ? 0u : i & (per_face - 1u);
+    if (!FILL) {
+        i /= per_face;
+    } else if (per_warp != 32u) {
         const uint32_t l = threadIdx.x & 31u;
         i = (i >> 5) * per_warp + l;
         mine = l < per_warp;
@@ -70,11 +74,12 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster(const uint4* __res
     const bool set = mine && i < F && raster_setup(f, faces, vfix, 0u, W, row0, row1, 0ull, J);
     const bool live = set && (J.wide != 0) == WIDE;
     if constexpr (!FILL) {
-        if (live) count_face<typename std::conditional<WIDE, long long, int>::type>(J, counts);
+        if (live)
+            count_face<typename std::conditional<WIDE, long long, int>::type>(J, counts, int(sub), int(per_face));
         if (!WIDE && wide_list) {
             // The faces of the 64-bit path, for its count and fill launches
             // (wide_list[0] = how many, then the face ids).
-            const bool wide = set && J.wide != 0;
+            const bool wide = set && J.wide != 0 && sub == 0u;
             const unsigned m = __ballot_sync(kFull, wide);
             if (m) {
                 const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
@@ -88,12 +93,14 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster(const uint4* __res
         __shared__ RasterJob jobs[kRasterWarps][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         if (live) jobs[w][lane] = J;
-        raster_warp<FILL, WIDE, REST>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets, records);
+        raster_warp<FILL, WIDE, REST>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets, records,
+                                      int(blockIdx.y), int(gridDim.y));
     }
 }
 
-// The 64-bit faces listed by the count (wide_list), 32 per warp and step over
-// a fixed grid: the count (one thread per face) or the fill (raster_warp).
+// The 64-bit faces listed by the count (wide_list) over a fixed grid: the count
+// of one face per warp (its rows over the lanes: a listed face has a side of
+// more than 64 px), or the fill (32 faces per warp and step, raster_warp).
 template <bool FILL, bool REST = false>
 __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_listed(const uint4* __restrict__ faces,
                                                                      const float4* __restrict__ vproj,
@@ -105,18 +112,21 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_listed(const uint4
     __shared__ RasterJob jobs[kRasterWarps][32];
     const uint32_t n = wide_list[0];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x + uint32_t(w) * 32u; base < n; base += stride) {
-        const uint32_t i = base + uint32_t(lane);
-        RasterJob J;
-        const bool live = i < n && raster_setup(wide_list[1 + i], faces, vfix, 0u, W, row0, row1, 0ull, J) &&
-                          J.wide != 0;
-        if constexpr (!FILL) {
-            if (live) count_face<long long>(J, counts);
-        } else {
+    if constexpr (!FILL) {
+        for (uint32_t i = blockIdx.x * kRasterWarps + uint32_t(w); i < n; i += gridDim.x * kRasterWarps) {
+            RasterJob J;
+            if (raster_setup(wide_list[1 + i], faces, vfix, 0u, W, row0, row1, 0ull, J) && J.wide != 0)
+                count_face<long long>(J, counts, lane, 32);
+        }
+    } else {
+        const uint32_t stride = gridDim.x * blockDim.x;
+        for (uint32_t base = blockIdx.x * blockDim.x + uint32_t(w) * 32u; base < n; base += stride) {
+            const uint32_t i = base + uint32_t(lane);
+            RasterJob J;
+            const bool live = i < n && raster_setup(wide_list[1 + i], faces, vfix, 0u, W, row0, row1, 0ull, J) &&
+                              J.wide != 0;
             if (live) jobs[w][lane] = J;
-            raster_warp<FILL, true, REST>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets,
-                                          records);
+            raster_warp<FILL, true, REST>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets, records);
             __syncwarp();  // every lane is done with this step's jobs before the next step writes them
         }
     }
@@ -155,7 +165,7 @@ void launch_rest_fill(const ListInfo* info, const uint4* faces, uint32_t F, cons
                                                             offsets, records);
 }
 
-constexpr unsigned kListedBlocks = 148;
+constexpr unsigned kListedBlocks = 148, kListedCountBlocks = 148 * 8;
 
 // Difference array of the count pass -> per-pixel counts, rows [row0, row1).
 __global__ void __launch_bounds__(256) k_row_prefix(uint32_t* __restrict__ counts, int W, int row0, int row1) {
@@ -168,30 +178,30 @@ void launch_raster_count(const uint4* faces, uint32_t F, const float4* vproj, co
     if (F == 0) return;
     if (row1 < 0) row1 = H;
     if (row1 <= row0) return;
-    const unsigned blocks = (F + 32 * kRasterWarps - 1) / (32 * kRasterWarps);
+    const uint32_t per_face = count_threads_per_face(F);
+    const unsigned blocks = unsigned((uint64_t(F) * per_face + 32 * kRasterWarps - 1) / (32 * kRasterWarps));
+    const uint32_t per_warp = 32u / per_face;
     if (wide_list) cudaMemsetAsync(wide_list, 0, sizeof(uint32_t), s);
     k_raster<false, false><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts, nullptr,
-                                                                nullptr, nullptr, wide_list, nullptr, 32u);
+                                                                nullptr, nullptr, wide_list, nullptr, per_warp);
     if (wide_list)
-        k_raster_listed<false><<<kListedBlocks, 32 * kRasterWarps, 0, s>>>(faces, vproj, vfix, W, row0, row1, counts,
-                                                                           nullptr, nullptr, wide_list);
+        k_raster_listed<false><<<kListedCountBlocks, 32 * kRasterWarps, 0, s>>>(faces, vproj, vfix, W, row0, row1,
+                                                                                counts, nullptr, nullptr, wide_list);
     else
         k_raster<false, true><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts,
-                                                                   nullptr, nullptr, nullptr, nullptr, nullptr, 32u);
+                                                                   nullptr, nullptr, nullptr, nullptr, nullptr,
+                                                                   per_warp);
     k_row_prefix<<<unsigned(row1 - row0 + 7) / 8, 256, 0, s>>>(counts, W, row0, row1);
 }
 
-constexpr uint32_t kFillMinWarps = 148 * 32;
 
 template <bool REST>
 static void raster_fill(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, uint32_t* counts,
                         const u64* offsets, u64* records, cudaStream_t s, int row0, int row1, const uint32_t* order,
                         const uint32_t* wide_list, const uint32_t* gate) {
-    // A warp fills its faces one after another: few faces (the boundary of a
-    // small mesh) are spread over more warps, down to one face each, until
-    // there are kFillMinWarps of them (8^3 at 64^2: 53 -> 13 us).
-    const uint32_t per_warp = std::min(32u, std::max(1u, F / kFillMinWarps));
-    const unsigned blocks = (F + per_warp * kRasterWarps - 1) / (per_warp * kRasterWarps);
+    const FillSplit sp = fill_split(F, uint64_t(row1 - row0));
+    const uint32_t per_warp = sp.per_warp;
+    const dim3 blocks((F + per_warp * kRasterWarps - 1) / (per_warp * kRasterWarps), sp.parts);
     k_raster<true, false, REST><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts,
                                                                      offsets, records, order, nullptr, gate, per_warp);
     if (wide_list)

@@ -198,13 +198,15 @@ struct FaceEdges {
 // row_prefix_warp turns it into per-pixel counts.  Two atomics per face row
 // instead of one per covered pixel, and no per-face warp work: a face has
 // about eleven rows at the path's sizes.
+// `first`, `step`: the rows taken by this thread (several threads per face).
 template <typename I>
-__device__ __forceinline__ void count_face(const RasterJob& J, uint32_t* __restrict__ counts) {
+__device__ __forceinline__ void count_face(const RasterJob& J, uint32_t* __restrict__ counts, int first = 0,
+                                           int step = 1) {
     EdgeT<I> e0, e1, e2;
     float i0, i1, i2;
     FaceEdges::make(J, e0, e1, e2, i0, i1, i2);
-    uint32_t* row = counts + J.pix_base + u64(J.py0) * u64(J.W) + u64(J.px0);
-    for (int r = 0; r < J.bh; ++r, row += J.W) {
+    uint32_t* row = counts + J.pix_base + u64(J.py0 + first) * u64(J.W) + u64(J.px0);
+    for (int r = first; r < J.bh; r += step, row += size_t(step) * size_t(J.W)) {
         int xl;
         const int len = row_span(e0, e1, e2, i0, i1, i2, r, J.bw, xl);
         if (len > 0) {
@@ -269,7 +271,7 @@ __device__ __forceinline__ void fill_pixels(const RasterJob& J, const int (&c)[U
 template <bool FILL, bool REST, typename I>
 __device__ __forceinline__ void raster_job(const RasterJob& J, int lane, const float4* __restrict__ vproj,
                                            uint32_t* __restrict__ counts, const u64* __restrict__ offsets,
-                                           u64* __restrict__ records) {
+                                           u64* __restrict__ records, int part, int parts) {
     static_assert(FILL, "the count pass runs one face per thread (count_face)");
     {
         constexpr int U = sizeof(I) == 4 ? 2 : 1;  // one pixel per step on the rare 64-bit path
@@ -278,7 +280,7 @@ __device__ __forceinline__ void raster_job(const RasterJob& J, int lane, const f
         FaceEdges::make(J, e0, e1, e2, i0, i1, i2);
         const u64 pbase = J.pix_base + u64(J.py0) * u64(J.W) + u64(J.px0);
         const float4 va = vproj[J.v0], vb = vproj[J.v1], vc = vproj[J.v2];
-        for (int r0 = 0; r0 < J.bh; r0 += 32) {
+        for (int r0 = 32 * part; r0 < J.bh; r0 += 32 * parts) {
             const int r = r0 + lane;
             int xl = 0, len = 0;
             if (r < J.bh) len = row_span(e0, e1, e2, i0, i1, i2, r, J.bw, xl);
@@ -310,20 +312,22 @@ __device__ __forceinline__ void raster_job(const RasterJob& J, int lane, const f
     }
 }
 
-// The warp's jobs (one per lane that has one, `live` the ballot), one at a time.
+// The warp's jobs (one per lane that has one, `live` the ballot), one at a time;
+// of each the row groups (32 rows) part, part + parts, ...
 // The 32-bit and 64-bit faces go to separate launches (WIDE), so that the
 // common 32-bit kernel keeps the register count of its own path.
 template <bool FILL, bool WIDE, bool REST = false>
 __device__ __forceinline__ void raster_warp(const RasterJob* jobs, uint32_t live, int lane,
                                             const float4* __restrict__ vproj, uint32_t* __restrict__ counts,
-                                            const u64* __restrict__ offsets, u64* __restrict__ records) {
+                                            const u64* __restrict__ offsets, u64* __restrict__ records,
+                                            int part = 0, int parts = 1) {
     __syncwarp();
     while (live) {
         const int k = __ffs(live) - 1;
         live &= live - 1;
         const RasterJob J = jobs[k];
-        raster_job<FILL, REST, typename std::conditional<WIDE, long long, int>::type>(J, lane, vproj, counts,
-                                                                                      offsets, records);
+        raster_job<FILL, REST, typename std::conditional<WIDE, long long, int>::type>(
+            J, lane, vproj, counts, offsets, records, part, parts);
     }
 }
 
