@@ -215,7 +215,7 @@ void composite_rows(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors
                                     reinterpret_cast<float4*>(d_image), r->tfinal.ptr, r->term.ptr, s, y0, y1, gate);
     else
         dtv::launch_composite(r->offsets.ptr, r->records.ptr, mesh->d_faces, r->vgeo.ptr,
-                              reinterpret_cast<const float4*>(d_colors), cam.W, cam.H, sh,
+                              reinterpret_cast<const float4*>(d_colors), uint32_t(mesh->host.num_vertices), cam.W, cam.H, sh,
                               reinterpret_cast<float4*>(d_image), r->tfinal.ptr, r->term.ptr, s, y0, y1,
                               r->tuning.composite_tile, gate);
 }

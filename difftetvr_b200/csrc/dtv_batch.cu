@@ -326,6 +326,7 @@ __device__ __forceinline__ bool tile_pixel(const BatchView* views, int nviews, i
     return px < int(bv.W) && py < int(bv.H);
 }
 
+template <bool AHEAD>
 __global__ void __launch_bounds__(kTile * kTile) kb_composite(const BatchView* __restrict__ views, int nviews,
                                                               const u64* __restrict__ offsets,
                                                               const u64* __restrict__ records,
@@ -337,8 +338,8 @@ __global__ void __launch_bounds__(kTile * kTile) kb_composite(const BatchView* _
     int v, px, py;
     if (!tile_pixel(views, nviews, v, px, py)) return;
     const BatchView& bv = views[v];
-    composite_pixel(px, py, int(bv.W), offsets + bv.pix_base, records, bv.faces, vgeo + bv.vert_base, bv.colors, sh,
-                    bv.image, tfinal + bv.pix_base, term + bv.pix_base);
+    composite_pixel<AHEAD>(px, py, int(bv.W), offsets + bv.pix_base, records, bv.faces, vgeo + bv.vert_base,
+                           bv.colors, sh, bv.image, tfinal + bv.pix_base, term + bv.pix_base);
 }
 
 // Lists of every view by walking its mesh (walk_pixel), in blocks of 16 x 8
@@ -809,9 +810,12 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
         launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, okp,
                     b->sort_surrogate_classes, b->sort_bucket_classes);
     }
-    kb_composite<<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(b->d_views.ptr, b->nviews, b->offsets.ptr,
-                                                                  b->records.ptr, b->vgeo.ptr, sh, b->tfinal.ptr,
-                                                                  b->term.ptr, okp);
+    const u64 n = b->nviews > 0 ? u64(b->nviews) : 1;
+    const auto composite = composite_ahead(b->tot_verts / n, b->tot_pixels / n, b->tot_pixels) ? kb_composite<true>
+                                                                                               : kb_composite<false>;
+    composite<<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(b->d_views.ptr, b->nviews, b->offsets.ptr,
+                                                               b->records.ptr, b->vgeo.ptr, sh, b->tfinal.ptr,
+                                                               b->term.ptr, okp);
 }
 
 // Adjoint of every view with a gradient slot into the slots' rows (which the

@@ -127,9 +127,21 @@ constexpr uint32_t kSortBlockCap = 16384;  // elements per block-sorted list / c
 
 // gate (optional): nothing is done when *gate is zero.
 // tile: pixel tile of the 256-thread blocks (0: 16 x 16, 1: 32 x 8, 2: 8 x 32).
+// Whether the composite loads ahead (composite_pixel): a pixel's list is a chain
+// of dependent loads, and running ahead of it is worth half the warps when the
+// pixels do not fill the GPU with plain ones anyway, and later only while the
+// vertices are too many to mostly hit L1.  pixels and V of one view, `all`
+// pixels of the launch.  Measured (us, plain -> ahead): 64^3 at 128^2 583 ->
+// 282, 16^3 at 256^2 75 -> 58, 33^3 at 721 x 479 330 -> 303, 64^3 at 512^2 586
+// -> 517, at 1024^2 1,545 -> 1,526; 40^3 at 1000^2 850 -> 888, 16^3 at 1000^2
+// 338 -> 362, 8^3 at 800^2 121 -> 129.
+inline bool composite_ahead(uint64_t V, uint64_t pixels, uint64_t all) {
+    if (all < 148 * 1280) return true;
+    return pixels < (pixels < 148 * 2560 ? 64 : 6) * V;
+}
 void launch_composite(const unsigned long long* offsets, const unsigned long long* records, const uint4* faces,
-                      const VGeo* vgeo, const float4* colors, int W, int H, const ShadeDev& sh, float4* image,
-                      float* tfinal, uint32_t* term, cudaStream_t s, int row0 = 0, int row1 = -1, int tile = 0,
+                      const VGeo* vgeo, const float4* colors, uint32_t V, int W, int H, const ShadeDev& sh,
+                      float4* image, float* tfinal, uint32_t* term, cudaStream_t s, int row0 = 0, int row1 = -1, int tile = 0,
                       const uint32_t* gate = nullptr);
 // Copies of the gradient rows of a mesh with few vertices (or cells): all
 // pixels' atomics on a few thousand rows wait for one another in L2, so the

@@ -1210,7 +1210,7 @@ void launch_sort(const u64* offsets, u64* records, uint32_t P, uint32_t* scratch
 // (d) front-to-back compositing, one thread per pixel (composite_pixel).
 // Pixel tiles of 256 threads: TX x (256 / TX) pixels (tile index 0: 16 x 16,
 // 1: 32 x 8, 2: 8 x 32; chosen by the renderer's tuning).
-template <int TX>
+template <int TX, bool PIPE>
 __global__ void __launch_bounds__(256) k_composite(
     const u64* __restrict__ offsets, const u64* __restrict__ records, const uint4* __restrict__ faces,
     const VGeo* __restrict__ vgeo, const float4* __restrict__ colors, int W, int row0, int row1, ShadeDev sh,
@@ -1221,30 +1221,36 @@ __global__ void __launch_bounds__(256) k_composite(
     const int px = blockIdx.x * TX + tile_x<TX>(threadIdx.x);
     const int py = row0 + int(blockIdx.y) * TY + tile_y<TX>(threadIdx.x);
     if (px < W && py < row1)
-        composite_pixel(px, py, W, offsets, records, faces, vgeo, colors, sh, image, tfinal, term);
+        composite_pixel<PIPE>(px, py, W, offsets, records, faces, vgeo, colors, sh, image, tfinal, term);
 }
 
 template <int TX>
-void composite_tiles(const u64* offsets, const u64* records, const uint4* faces, const VGeo* vgeo,
-                     const float4* colors, int W, int row0, int row1, const ShadeDev& sh, float4* image,
-                     float* tfinal, uint32_t* term, const uint32_t* gate, cudaStream_t s) {
+static void composite_tiles(const u64* offsets, const u64* records, const uint4* faces, const VGeo* vgeo,
+                            const float4* colors, int W, int row0, int row1, const ShadeDev& sh, float4* image,
+                            float* tfinal, uint32_t* term, const uint32_t* gate, bool pipe, cudaStream_t s) {
     constexpr int TY = 256 / TX;
     dim3 grid((W + TX - 1) / TX, (row1 - row0 + TY - 1) / TY);
-    k_composite<TX><<<grid, 256, 0, s>>>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal,
-                                         term, gate);
+    (pipe ? k_composite<TX, true> : k_composite<TX, false>)<<<grid, 256, 0, s>>>(
+        offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate);
 }
 
 void launch_composite(const u64* offsets, const u64* records, const uint4* faces, const VGeo* vgeo,
-                      const float4* colors, int W, int H, const ShadeDev& sh, float4* image, float* tfinal,
-                      uint32_t* term, cudaStream_t s, int row0, int row1, int tile, const uint32_t* gate) {
+                      const float4* colors, uint32_t V, int W, int H, const ShadeDev& sh, float4* image,
+                      float* tfinal, uint32_t* term, cudaStream_t s, int row0, int row1, int tile,
+                      const uint32_t* gate) {
     if (row1 < 0) row1 = H;
     if (row1 <= row0) return;
+    const uint64_t pixels = uint64_t(row1 - row0) * uint64_t(W);
+    const bool pipe = composite_ahead(V, pixels, pixels);
     if (tile == 1)
-        composite_tiles<32>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate, s);
+        composite_tiles<32>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate, pipe,
+                            s);
     else if (tile == 2)
-        composite_tiles<8>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate, s);
+        composite_tiles<8>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate, pipe,
+                           s);
     else
-        composite_tiles<16>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate, s);
+        composite_tiles<16>(offsets, records, faces, vgeo, colors, W, row0, row1, sh, image, tfinal, term, gate, pipe,
+                            s);
 }
 
 // ---------------------------------------------------------------------------

@@ -152,7 +152,8 @@ extern "C" int32_t dtv_render_noalloc(const dtv_mesh* mesh, const float* d_posit
             throw NaError(DTV_ERR_BUDGET, "dtv_render_noalloc: fragments exceed fragment_budget_bytes");
         dtv::launch_raster_fill(mv.faces, uint32_t(mv.num_faces), vproj, vfix, W, H, counts, offsets, records, s);
         dtv::launch_sort(offsets, records, uint32_t(P), long_list, s);
-        dtv::launch_composite(offsets, records, mv.faces, vgeo, reinterpret_cast<const float4*>(d_colors), W, H, sh,
+        dtv::launch_composite(offsets, records, mv.faces, vgeo, reinterpret_cast<const float4*>(d_colors),
+                              uint32_t(mv.num_vertices), W, H, sh,
                               reinterpret_cast<float4*>(d_image), tfinal, term, s);
         NA_CK(cudaGetLastError());
         return DTV_OK;

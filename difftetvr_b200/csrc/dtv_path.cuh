@@ -346,20 +346,26 @@ struct FragV {
     uint32_t v0, v1, v2;
 };
 
+// What a fragment reads of its face's vertices.
+struct FragRaw {
+    VGeo g[3];
+    float4 c[3];
+};
+
+__device__ __forceinline__ FragRaw load_raw(const uint4& fc, const VGeo* __restrict__ vgeo,
+                                            const float4* __restrict__ colors) {
+    return FragRaw{{vgeo[fc.x], vgeo[fc.y], vgeo[fc.z]}, {colors[fc.x], colors[fc.y], colors[fc.z]}};
+}
+
 // Fragment values from the record's low word (face << 2 | bits) and the
-// face's vertex indices.
-__device__ __forceinline__ FragV load_frag_face(uint32_t lo, const uint4& fc, float qx, float qy,
-                                                const VGeo* __restrict__ vgeo, const float4* __restrict__ colors) {
+// face's vertices.
+__device__ __forceinline__ FragV frag_of_raw(uint32_t lo, const FragRaw& r, float qx, float qy) {
     FragV fr;
     fr.face = lo >> 2;
     fr.bits = lo & 3u;
-    fr.v0 = fc.x;
-    fr.v1 = fc.y;
-    fr.v2 = fc.z;
-    const VGeo a = vgeo[fc.x], b = vgeo[fc.y], c = vgeo[fc.z];
     float bary[3];
-    face_bary(a, b, c, qx, qy, bary, fr.z);  // depth and colour from the same weights
-    const float4 c0 = colors[fc.x], c1 = colors[fc.y], c2 = colors[fc.z];
+    face_bary(r.g[0], r.g[1], r.g[2], qx, qy, bary, fr.z);  // depth and colour from the same weights
+    const float4 c0 = r.c[0], c1 = r.c[1], c2 = r.c[2];
     // (r, g) and (b, a) as FP32 pairs.
     const float2 b0 = bc2(bary[0]), b1 = bc2(bary[1]), b2 = bc2(bary[2]);
     const float2 rg = fma2(b2, make_float2(c2.x, c2.y),
@@ -367,6 +373,15 @@ __device__ __forceinline__ FragV load_frag_face(uint32_t lo, const uint4& fc, fl
     const float2 ba = fma2(b2, make_float2(c2.z, c2.w),
                            fma2(b1, make_float2(c1.z, c1.w), mul2(b0, make_float2(c0.z, c0.w))));
     fr.col = make_float4(rg.x, rg.y, ba.x, ba.y);
+    return fr;
+}
+
+__device__ __forceinline__ FragV load_frag_face(uint32_t lo, const uint4& fc, float qx, float qy,
+                                                const VGeo* __restrict__ vgeo, const float4* __restrict__ colors) {
+    FragV fr = frag_of_raw(lo, load_raw(fc, vgeo, colors), qx, qy);
+    fr.v0 = fc.x;
+    fr.v1 = fc.y;
+    fr.v2 = fc.z;
     return fr;
 }
 
@@ -471,6 +486,10 @@ __device__ __forceinline__ void write_pixel(float4* __restrict__ image, float* _
 // (d) front-to-back compositing, one thread per pixel (16x16 pixel tiles).
 // Forward.glsl:159-211 with early ray termination (:169-173) and the
 // termination index (:256-259); final transmittance is kept for the adjoint.
+// PIPE: the dependent loads record -> face -> vertices run ahead (the vertices
+// of the next fragment, the face of the one after, the record of the one after
+// that), at twice the registers.
+template <bool PIPE>
 __device__ __forceinline__ void composite_pixel(
     int px, int py, int W, const u64* __restrict__ offsets, const u64* __restrict__ records,
     const uint4* __restrict__ faces, const VGeo* __restrict__ vgeo, const float4* __restrict__ colors,
@@ -484,10 +503,32 @@ __device__ __forceinline__ void composite_pixel(
     uint32_t i = n;
     if (n >= 2) {
         FragV f1 = load_frag(records[beg], qx, qy, faces, vgeo, colors), f0;
+        const uint32_t last = n - 1u;
+        uint32_t lo1 = 0, lo2 = 0, lo3 = 0;  // records i, i + 1, i + 2 (the last one again past the end)
+        uint4 fc2{};                         // face i + 1
+        FragRaw r1;                          // vertices of fragment i
+        if (PIPE) {
+            lo1 = record_lo(records, beg + 1);
+            lo2 = record_lo(records, beg + min(2u, last));
+            lo3 = record_lo(records, beg + min(3u, last));
+            fc2 = faces[lo2 >> 2];
+            r1 = load_raw(faces[lo1 >> 2], vgeo, colors);
+        }
         for (i = 1; i < n; ++i) {
             if (sh.use_ert && T.hi < sh.ert_thresh) break;
             f0 = f1;
-            f1 = load_frag(records[beg + i], qx, qy, faces, vgeo, colors);
+            if (PIPE) {
+                const FragRaw r = r1;
+                const uint32_t lo = lo1;
+                r1 = load_raw(fc2, vgeo, colors);
+                fc2 = faces[lo3 >> 2];
+                lo1 = lo2;
+                lo2 = lo3;
+                lo3 = record_lo(records, beg + min(i + 3u, last));
+                f1 = frag_of_raw(lo, r, qx, qy);
+            } else {
+                f1 = load_frag(records[beg + i], qx, qy, faces, vgeo, colors);
+            }
             if (skip_pair(f0.bits, f1.bits)) continue;
             segment_composite((f1.z - f0.z) * 0.25f, f0.col, f1.col, sh.atten, C0, C1, C2, T);
         }
