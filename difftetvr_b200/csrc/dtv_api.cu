@@ -97,6 +97,7 @@ struct dtv_renderer {
     // when the lists are stored whole.
     std::vector<std::pair<int, int>> bands;
     bool band_walk = false;       // the bands' lists are walked
+    DevBuf<uint32_t> band_counts; // the pixels' counts of a banded render, for its adjoint
     bool clipped_view = false;    // the last projection clipped a vertex
     bool cells = false;           // last render used per-cell colours
     dtv_tuning tuning{0, 0, dtv::kSortSurrogateDefault, dtv::kSortBucketDefault};
@@ -172,9 +173,9 @@ uint64_t plan_bands(dtv_renderer* r, int W, int H, uint64_t cap, cudaStream_t s)
 // to the end of its range; the walk starts from them.
 void walk_rows(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& cam, int y0, int y1, bool guarded,
                cudaStream_t s) {
-    dtv::launch_raster_fill(mesh->d_bfaces, uint32_t(mesh->bf_global.size()), r->vproj.ptr, r->vfix.ptr, cam.W, cam.H,
-                            r->counts.ptr, r->offsets.ptr, r->records.ptr, s, y0, y1, nullptr, nullptr,
-                            guarded ? &r->info.ptr->ok : nullptr);
+    dtv::launch_boundary_fill(mesh->d_bfaces, uint32_t(mesh->bf_global.size()), r->vproj.ptr, r->vfix.ptr, cam.W, y0,
+                              y1, r->counts.ptr, r->offsets.ptr, r->records.ptr, guarded ? &r->info.ptr->ok : nullptr,
+                              s);
     check_launch("boundary fill");
     dtv::launch_walk_lists(walk_mesh(mesh), r->offsets.ptr, r->records.ptr, r->counts.ptr, r->walk_verts.ptr, cam.W,
                            y0, y1, r->info.ptr, r->redo.ptr, guarded, s);
@@ -196,7 +197,7 @@ void rest_rows(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& cam, in
     } else {
         dtv::launch_raster_fill(mesh->d_faces, F, r->vproj.ptr, r->vfix.ptr, cam.W, cam.H, r->counts.ptr,
                                 r->offsets.ptr, r->records.ptr, s, y0, y1, r->fill_order.ptr, r->wide_list.ptr,
-                                nullptr, /*rest=*/true);
+                                /*rest=*/true);
         dtv::launch_sort(r->offsets.ptr, r->records.ptr, uint32_t(y1 - y0) * uint32_t(cam.W), r->long_list.ptr, s,
                          nullptr, r->tuning.sort_surrogate_classes, r->tuning.sort_bucket_classes, r->redo.ptr,
                          &r->info.ptr->n_redo);
@@ -307,6 +308,9 @@ void render_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors,
     try {
         largest = plan_bands(r, W, H, cap, s);
         r->records.ensure(largest ? largest : 1, s, false, 1.0);
+        const size_t P = size_t(W) * size_t(H);
+        r->band_counts.ensure(P, s);
+        DTV_CK(cudaMemcpyAsync(r->band_counts.ptr, r->counts.ptr, sizeof(uint32_t) * P, cudaMemcpyDeviceToDevice, s));
     } catch (...) {
         r->bands.clear();
         cudaMemsetAsync(r->counts.ptr, 0, uint64_t(W) * H * sizeof(uint32_t), s);
@@ -323,18 +327,14 @@ void render_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors,
     rec_event(r, 6, s);
 }
 
-// Adjoint of a banded render: per band, the lists are rebuilt (count, scan,
-// fill, sort of the band's rows, from the projection kept by the render) and
-// the band's adjoint accumulates into the shared gradient rows.
+// Adjoint of a banded render: per band, the lists are rebuilt (from the counts
+// and the projection kept by the render) and the band's adjoint accumulates
+// into the shared gradient rows.
 void adjoint_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors, const float* d_image_adjoint,
                     const dtv::ShadeDev& sh, float* d_grad_positions, float* d_grad_colors, cudaStream_t s) {
-    const int W = r->cam.W, H = r->cam.H;
     clear_rows(r, mesh, s);
-    r->wide_list.ensure(size_t(mesh->host.num_faces) + 1, s);
+    DTV_CK(cudaMemcpyAsync(r->counts.ptr, r->band_counts.ptr, sizeof(uint32_t) * r->P, cudaMemcpyDeviceToDevice, s));
     for (const auto& b : r->bands) {
-        dtv::launch_raster_count(mesh->d_faces, uint32_t(mesh->host.num_faces), r->vproj.ptr, r->vfix.ptr, W, H,
-                                 r->counts.ptr, s, b.first, b.second, r->wide_list.ptr);
-        check_launch("band count");
         build_band_lists(r, mesh, r->cam, b.first, b.second, s);
         adjoint_rows(r, mesh, d_colors, d_image_adjoint, sh, b.first, b.second, d_grad_colors, s);
         check_launch("band adjoint");
@@ -532,6 +532,7 @@ int32_t dtv_renderer_destroy(dtv_renderer* r) {
     r->long_list.release();
     r->grad_rows.release();
     r->cell_rows.release();
+    r->band_counts.release();
     r->wstate.release();
     r->fill_order.release();
     r->band_scratch.release();
@@ -595,6 +596,7 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
             r->term.ensure(P, s);
         r->long_list.ensure(dtv::sort_scratch_elems(P), s);
 
+        r->wide_list.ensure(size_t(F) + 1, s);
         rec_event(r, 0, s);
         const bool walk = !raytet && mesh->walkable;
         if (walk) {
@@ -603,10 +605,9 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
             r->redo.ensure(P, s);
         }
         dtv::launch_project(d_positions, uint32_t(V), cam, r->vproj.ptr, r->vfix.ptr, r->vgeo.ptr, s,
-                            walk ? r->walk_verts.ptr : nullptr, walk ? r->clipped.ptr : nullptr);
+                            walk ? r->walk_verts.ptr : nullptr, walk ? r->clipped.ptr : nullptr, r->wide_list.ptr);
         check_launch("project");
         rec_event(r, 1, s);
-        r->wide_list.ensure(size_t(F) + 1, s);
         dtv::launch_raster_count(rfaces, uint32_t(F), r->vproj.ptr, r->vfix.ptr, W, H, r->counts.ptr, s, 0, -1,
                                  r->wide_list.ptr);
         check_launch("raster count");
@@ -692,10 +693,15 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         }
         if (!walk) {
             rec_event(r, 3, s);
-            if (!raytet) order_faces();
-            dtv::launch_raster_fill(rfaces, uint32_t(F), r->vproj.ptr, r->vfix.ptr, W, H, r->counts.ptr,
-                                    r->offsets.ptr, r->records.ptr, s, 0, -1, raytet ? nullptr : r->fill_order.ptr,
-                                    raytet ? nullptr : r->wide_list.ptr);
+            if (raytet) {
+                dtv::launch_boundary_fill(rfaces, uint32_t(F), r->vproj.ptr, r->vfix.ptr, W, 0, H, r->counts.ptr,
+                                          r->offsets.ptr, r->records.ptr, nullptr, s);
+            } else {
+                order_faces();
+                dtv::launch_raster_fill(rfaces, uint32_t(F), r->vproj.ptr, r->vfix.ptr, W, H, r->counts.ptr,
+                                        r->offsets.ptr, r->records.ptr, s, 0, -1, r->fill_order.ptr,
+                                        r->wide_list.ptr);
+            }
             check_launch("raster fill");
             rec_event(r, 4, s);
             dtv::launch_sort(r->offsets.ptr, r->records.ptr, uint32_t(P), r->long_list.ptr, s, nullptr,

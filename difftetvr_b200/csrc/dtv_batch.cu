@@ -90,9 +90,10 @@ __device__ __forceinline__ int view_of_item(u64 g, u64 block_first, int n, Gette
 __global__ void __launch_bounds__(256) kb_project(const BatchView* __restrict__ views, int nviews, u64 total,
                                                   float4* __restrict__ vproj, int2* __restrict__ vfix,
                                                   VGeo* __restrict__ vgeo, WalkVertRow* __restrict__ rows,
-                                                  uint32_t* __restrict__ clipped) {
+                                                  uint32_t* __restrict__ clipped, uint32_t* __restrict__ wide_list) {
     const u64 first = u64(blockIdx.x) * blockDim.x;
     const u64 g = first + threadIdx.x;
+    if (g == 0) wide_list[0] = 0u;
     if (g < total) {
         const int v = view_of_item(g, first, nviews, [&](int i) { return views[i].vert_base; });
         const BatchView& bv = views[v];
@@ -169,41 +170,31 @@ __global__ void __launch_bounds__(256) kb_band_scatter(const BatchView* __restri
     if (g < total) order[base[band] + rank] = uint32_t(g);
 }
 
-// Count or fill of every view's faces (kAllFaces), the fill of its boundary
-// faces (kBoundaryFaces: record face field = boundary face index), or the fill
-// of the pixels the walk left to the rasteriser (kRestFaces; see fill_pixels).
-// `ok`: the fill does nothing when *ok is zero.
-enum FaceSet { kAllFaces = 0, kBoundaryFaces = 1, kRestFaces = 2 };
-template <bool FILL, bool WIDE, int kSet = kAllFaces>
+// Count or fill of every view's faces.  REST: the fill of the pixels the walk
+// left to the rasteriser (see fill_pixels).  `ok`: the fill does nothing when
+// *ok is zero.  threads_per_face: of the count (k_raster).
+template <bool FILL, bool WIDE, bool REST = false>
 __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ views, int nviews, u64 total,
                                                  const float4* __restrict__ vproj, const int2* __restrict__ vfix,
                                                  uint32_t* __restrict__ counts, const u64* __restrict__ offsets,
                                                  u64* __restrict__ records, const uint32_t* __restrict__ ok,
                                                  const uint32_t* __restrict__ order,
-                                                 uint32_t* __restrict__ wide_list, uint32_t per_warp) {
+                                                 uint32_t* __restrict__ wide_list, uint32_t threads_per_face) {
     if (FILL && !batch_ok(ok)) return;
     const u64 first = u64(blockIdx.x) * blockDim.x;
-    u64 i = first + threadIdx.x;
-    bool mine = true;
-    // As k_raster: faces per warp of the fill, threads per face of the count.
-    const uint32_t per_face = 32u / per_warp, sub = FILL ? 0u : uint32_t(i) & (per_face - 1u);
-    if (!FILL) {
-        i /= per_face;
-    } else if (per_warp != 32u) {
-        const uint32_t l = threadIdx.x & 31u;
-        i = (i >> 5) * per_warp + l;
-        mine = l < per_warp;
-    }
+    const uint32_t per_face = FILL ? 1u : threads_per_face;
+    const u64 i = (first + threadIdx.x) / per_face;
+    const uint32_t sub = threadIdx.x & (per_face - 1u);
     bool set = false, live = false;
     RasterJob J;
     u64 g = 0;
-    if (mine && i < total) {
+    if (i < total) {
         g = order ? u64(order[i]) : i;
-        auto base = [&](int k) { return kSet == kBoundaryFaces ? views[k].bface_base : views[k].face_base; };
-        const int v = (FILL || order) ? find_index(g, nviews, base) : view_of_item(g, first / per_face, nviews, base);
+        const int v = order ? find_index(g, nviews, [&](int k) { return views[k].face_base; })
+                            : view_of_item(g, first / per_face, nviews, [&](int k) { return views[k].face_base; });
         const BatchView& bv = views[v];
-        set = raster_setup(uint32_t(g - base(v)), kSet == kBoundaryFaces ? bv.walk.bfaces : bv.faces,
-                           vfix + bv.vert_base, uint32_t(bv.vert_base), int(bv.W), 0, int(bv.H), bv.pix_base, J);
+        set = raster_setup(uint32_t(g - bv.face_base), bv.faces, vfix + bv.vert_base, uint32_t(bv.vert_base),
+                           int(bv.W), 0, int(bv.H), bv.pix_base, J);
         live = set && (J.wide != 0) == WIDE;
     }
     if constexpr (!FILL) {
@@ -226,8 +217,8 @@ __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ v
         __shared__ RasterJob jobs[4][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         if (live) jobs[w][lane] = J;
-        raster_warp<FILL, WIDE, kSet == kRestFaces>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts,
-                                                    offsets, records, int(blockIdx.y), int(gridDim.y));
+        raster_warp<FILL, WIDE, REST>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets,
+                                      records);
     }
 }
 
@@ -270,6 +261,34 @@ __global__ void __launch_bounds__(128) kb_raster_listed(const BatchView* __restr
             __syncwarp();  // every lane is done with this step's jobs before the next step writes them
         }
     }
+}
+
+// Fill of every view's boundary faces (k_boundary_fill; record face field =
+// boundary face index).
+__global__ void __launch_bounds__(128) kb_boundary_fill(const BatchView* __restrict__ views, int nviews, u64 total,
+                                                        const float4* __restrict__ vproj,
+                                                        const int2* __restrict__ vfix, uint32_t* __restrict__ counts,
+                                                        const u64* __restrict__ offsets, u64* __restrict__ records,
+                                                        const uint32_t* __restrict__ ok, uint32_t per_warp) {
+    if (!batch_ok(ok)) return;
+    __shared__ RasterJob jobs[4][32];
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const u64 g = (u64(blockIdx.x) * 4 + w) * per_warp + lane;
+    RasterJob J;
+    bool live = false;
+    if (lane < per_warp && g < total) {
+        const int v = find_index(g, nviews, [&](int k) { return views[k].bface_base; });
+        const BatchView& bv = views[v];
+        live = raster_setup(uint32_t(g - bv.bface_base), bv.walk.bfaces, vfix + bv.vert_base, uint32_t(bv.vert_base),
+                            int(bv.W), 0, int(bv.H), bv.pix_base, J);
+    }
+    const bool wide = live && J.wide != 0;
+    if (live) jobs[w][lane] = J;
+    const int part = int(blockIdx.y), parts = int(gridDim.y);
+    raster_warp<true, false>(jobs[w], __ballot_sync(0xffffffffu, live && !wide), int(lane), vproj, counts, offsets,
+                             records, part, parts);
+    raster_warp<true, true>(jobs[w], __ballot_sync(0xffffffffu, wide), int(lane), vproj, counts, offsets, records,
+                            part, parts);
 }
 
 // Fill of the few pixels the walk left to the rasteriser (k_rest_fill).
@@ -738,19 +757,18 @@ void launch_kb_count(dtv_batch* b, cudaStream_t s) {
     using namespace dtv;
     const uint32_t per_face = count_threads_per_face(b->tot_faces);
     const unsigned blocks = grid_for(b->tot_faces * per_face, 128, 0x7fffffffu);
-    DTV_CK(cudaMemsetAsync(b->wide_list.ptr, 0, sizeof(uint32_t), s));
     kb_raster<false, false><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr, b->vfix.ptr,
                                                    b->counts.ptr, nullptr, nullptr, nullptr, nullptr,
-                                                   b->wide_list.ptr, 32u / per_face);
+                                                   b->wide_list.ptr, per_face);
     kb_raster_listed<false><<<148 * 8, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
                                                 nullptr, nullptr, nullptr, b->wide_list.ptr);
     dim3 grid(unsigned(b->max_height + 7) / 8, unsigned(b->nviews));
     kb_row_prefix<<<grid, 256, 0, s>>>(b->d_views.ptr, b->counts.ptr);
 }
 
-// Fill pass over every view's faces in row-band order (kRestFaces: of the
-// pixels the walk left).
-template <int kSet>
+// Fill pass over every view's faces in row-band order (REST: of the pixels the
+// walk left).
+template <bool REST>
 void launch_kb_fill(dtv_batch* b, const uint32_t* okp, cudaStream_t s) {
     using namespace dtv;
     const unsigned blocks = grid_for(b->tot_faces, 128, 0x7fffffffu);
@@ -765,10 +783,10 @@ void launch_kb_fill(dtv_batch* b, const uint32_t* okp, cudaStream_t s) {
                                            b->tot_pixels, b->band_scratch.ptr + kFillBands, b->fill_order.ptr);
         order = b->fill_order.ptr;
     }
-    kb_raster<true, false, kSet><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr,
+    kb_raster<true, false, REST><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr,
                                                   b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr, okp, order, nullptr,
-                                                  32u);
-    kb_raster_listed<true, kSet == kRestFaces><<<148, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
+                                                  1u);
+    kb_raster_listed<true, REST><<<148, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
                                                b->offsets.ptr, b->records.ptr, okp, b->wide_list.ptr);
 }
 
@@ -782,22 +800,15 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
     if (b->walk) {
         if (b->tot_bfaces) {
             const FillSplit sp = fill_split(b->tot_bfaces, b->max_height);
-            const uint32_t per_warp = sp.per_warp;
-            const dim3 bb(grid_for(b->tot_bfaces, 4 * per_warp, 0x7fffffffu), sp.parts);
-            kb_raster<true, false, kBoundaryFaces><<<bb, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_bfaces,
-                                                                      b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
-                                                                      b->offsets.ptr, b->records.ptr, okp, nullptr,
-                                                                      nullptr, per_warp);
-            kb_raster<true, true, kBoundaryFaces><<<bb, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_bfaces,
-                                                                     b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
-                                                                     b->offsets.ptr, b->records.ptr, okp, nullptr,
-                                                                     nullptr, per_warp);
+            const dim3 bb(grid_for(b->tot_bfaces, 4 * sp.per_warp, 0x7fffffffu), sp.parts);
+            kb_boundary_fill<<<bb, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_bfaces, b->vproj.ptr, b->vfix.ptr,
+                                                b->counts.ptr, b->offsets.ptr, b->records.ptr, okp, sp.per_warp);
         }
         kb_walk_lists<<<unsigned(2 * b->tot_tiles), kWalkBatchThreads, 0, s>>>(
             b->d_views.ptr, b->nviews, b->offsets.ptr, b->records.ptr, b->counts.ptr, b->walk_verts.ptr, b->info.ptr,
             b->redo.ptr);
         if (b->many_left) {
-            launch_kb_fill<kRestFaces>(b, okp, s);
+            launch_kb_fill<true>(b, okp, s);
             launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, okp,
                         b->sort_surrogate_classes, b->sort_bucket_classes, b->redo.ptr, &b->info.ptr->n_redo);
         } else {
@@ -806,7 +817,7 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
             launch_rest_sort(b->info.ptr, false, b->redo.ptr, b->offsets.ptr, b->records.ptr, s);
         }
     } else {
-        launch_kb_fill<kAllFaces>(b, okp, s);
+        launch_kb_fill<false>(b, okp, s);
         launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, okp,
                     b->sort_surrogate_classes, b->sort_bucket_classes);
     }
@@ -845,7 +856,8 @@ void enqueue_count(dtv_batch* b, u64 capacity, cudaStream_t s) {
     using namespace dtv;
     kb_project<<<grid_for(b->tot_verts, 256, 0x7fffffffu), 256, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_verts,
                                                                         b->vproj.ptr, b->vfix.ptr, b->vgeo.ptr,
-                                                                        b->walk ? b->walk_verts.ptr : nullptr, b->clipped.ptr);
+                                                                        b->walk ? b->walk_verts.ptr : nullptr, b->clipped.ptr,
+                                                                        b->wide_list.ptr);
     launch_kb_count(b, s);
     launch_scan(b->counts.ptr, b->tot_pixels, b->offsets.ptr, b->scan.ptr, s, b->info.ptr, capacity, b->clipped.ptr);
     check_launch("batch count");

@@ -56,13 +56,14 @@ inline FillSplit fill_split(uint64_t F, uint64_t image_rows) {
 
 // Launch wrappers (dtv_kernels.cu).  All run on `s`.
 // rows (optional): the vertices' walk rows as well; clipped (optional): set to
-// 1 when a vertex is not projected.
+// 1 when a vertex is not projected; wide_list (optional): [0] cleared for the
+// count.
 void launch_project(const float* pos, uint32_t V, const CamDev& cam, float4* vproj, int2* vfix, VGeo* vgeo,
-                    cudaStream_t s, WalkVertRow* rows = nullptr, uint32_t* clipped = nullptr);
-// gate (optional, fill without a wide_list): the kernels do nothing when *gate
-// is zero; rest: the fill takes only pixels whose counter is not zero.
+                    cudaStream_t s, WalkVertRow* rows = nullptr, uint32_t* clipped = nullptr,
+                    uint32_t* wide_list = nullptr);
+// rest: the fill takes only pixels whose counter is not zero.
 // Pixel rows [row0, row1) only (row1 < 0: all rows).  wide_list (u32[F + 1],
-// optional): the count lists the faces of the 64-bit path there, and the
+// optional, [0] zero: launch_project): the count lists the faces of the 64-bit path there, and the
 // 64-bit count and the fill that follows (same rows) walk that list instead of
 // setting up every face again; without it both 64-bit launches cover all F.
 void launch_raster_count(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, int H,
@@ -71,7 +72,11 @@ void launch_raster_count(const uint4* faces, uint32_t F, const float4* vproj, co
 void launch_raster_fill(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, int H,
                         uint32_t* counts, const unsigned long long* offsets, unsigned long long* records,
                         cudaStream_t s, int row0 = 0, int row1 = -1, const uint32_t* order = nullptr,
-                        const uint32_t* wide_list = nullptr, const uint32_t* gate = nullptr, bool rest = false);
+                        const uint32_t* wide_list = nullptr, bool rest = false);
+// Fill of a few faces (the boundary's); nothing is done when *gate is zero.
+void launch_boundary_fill(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, int row0,
+                          int row1, uint32_t* counts, const unsigned long long* offsets, unsigned long long* records,
+                          const uint32_t* gate, cudaStream_t s);
 struct ListInfo;
 // The few pixels the walk left to the rasteriser (nothing is done when there
 // are none, or when clipped vertices make them many: launch_raster_fill with

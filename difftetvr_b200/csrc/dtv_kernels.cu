@@ -19,9 +19,10 @@ constexpr unsigned kFull = 0xffffffffu;
 __global__ void __launch_bounds__(256) k_project(const float* __restrict__ pos, uint32_t V, CamDev cam,
                                                  float4* __restrict__ vproj, int2* __restrict__ vfix,
                                                  VGeo* __restrict__ vgeo, WalkVertRow* __restrict__ rows,
-                                                 uint32_t* __restrict__ clipped) {
+                                                 uint32_t* __restrict__ clipped, uint32_t* __restrict__ wide_list) {
     uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
+    if (wide_list && v == 0) wide_list[0] = 0u;
     float x = pos[3 * size_t(v)], y = pos[3 * size_t(v) + 1], z = pos[3 * size_t(v) + 2];
     int2 fx;
     const float4 pr = project_vertex(cam, x, y, z, fx);
@@ -34,16 +35,21 @@ __global__ void __launch_bounds__(256) k_project(const float* __restrict__ pos, 
 }
 
 void launch_project(const float* pos, uint32_t V, const CamDev& cam, float4* vproj, int2* vfix, VGeo* vgeo,
-                    cudaStream_t s, WalkVertRow* rows, uint32_t* clipped) {
-    if (V == 0) return;
-    k_project<<<(V + 255) / 256, 256, 0, s>>>(pos, V, cam, vproj, vfix, vgeo, rows, clipped);
+                    cudaStream_t s, WalkVertRow* rows, uint32_t* clipped, uint32_t* wide_list) {
+    if (V == 0) {
+        if (wide_list) cudaMemsetAsync(wide_list, 0, sizeof(uint32_t), s);
+        return;
+    }
+    k_project<<<(V + 255) / 256, 256, 0, s>>>(pos, V, cam, vproj, vfix, vgeo, rows, clipped,
+                                                wide_list);
 }
 
 // (a)+(b) face rasterisation: 32 faces per warp, the warp's lanes spread over
 // each face's pixels in turn (raster_warp, dtv_path.cuh).
 constexpr int kRasterWarps = 4;
 
-// `gate` (optional): nothing is done when *gate is zero.  REST: see fill_pixels.
+// REST: see fill_pixels.  threads_per_face: of the count, each every so many
+// rows.
 template <bool FILL, bool WIDE, bool REST = false>
 __global__ void __launch_bounds__(32 * kRasterWarps) k_raster(const uint4* __restrict__ faces, uint32_t F,
                                                               const float4* __restrict__ vproj,
@@ -53,25 +59,12 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster(const uint4* __res
                                                               u64* __restrict__ records,
                                                               const uint32_t* __restrict__ order,
                                                               uint32_t* __restrict__ wide_list,
-                                                              const uint32_t* __restrict__ gate,
-                                                              uint32_t per_warp) {
-    if (gate && *gate == 0u) return;
-    // The fill gives each warp per_warp <= 32 faces, which it takes one at a
-    // time; the count takes 32 / per_warp threads per face (a power of two),
-    // each every so many rows.
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool mine = true;
-    const uint32_t per_face = 32u / per_warp, sub = FILL ? 0u : i & (per_face - 1u);
-    if (!FILL) {
-        i /= per_face;
-    } else if (per_warp != 32u) {
-        const uint32_t l = threadIdx.x & 31u;
-        i = (i >> 5) * per_warp + l;
-        mine = l < per_warp;
-    }
-    const uint32_t f = (order && mine && i < F) ? order[i] : i;
+                                                              uint32_t threads_per_face) {
+    const uint32_t per_face = FILL ? 1u : threads_per_face, t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = t / per_face, sub = t & (per_face - 1u);
+    const uint32_t f = (order && i < F) ? order[i] : i;
     RasterJob J;
-    const bool set = mine && i < F && raster_setup(f, faces, vfix, 0u, W, row0, row1, 0ull, J);
+    const bool set = i < F && raster_setup(f, faces, vfix, 0u, W, row0, row1, 0ull, J);
     const bool live = set && (J.wide != 0) == WIDE;
     if constexpr (!FILL) {
         if (live)
@@ -93,8 +86,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster(const uint4* __res
         __shared__ RasterJob jobs[kRasterWarps][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         if (live) jobs[w][lane] = J;
-        raster_warp<FILL, WIDE, REST>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets, records,
-                                      int(blockIdx.y), int(gridDim.y));
+        raster_warp<FILL, WIDE, REST>(jobs[w], __ballot_sync(kFull, live), lane, vproj, counts, offsets, records);
     }
 }
 
@@ -159,6 +151,41 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_rest_fill(const ListInfo*
     }
 }
 
+// Fill of a few faces (the boundary): fill_split's faces per warp and row
+// groups, 32- and 64-bit faces alike.  Nothing is done when *gate is zero.
+__global__ void __launch_bounds__(32 * kRasterWarps) k_boundary_fill(const uint4* __restrict__ faces, uint32_t F,
+                                                                     const float4* __restrict__ vproj,
+                                                                     const int2* __restrict__ vfix, int W, int row0,
+                                                                     int row1, uint32_t* __restrict__ counts,
+                                                                     const u64* __restrict__ offsets,
+                                                                     u64* __restrict__ records,
+                                                                     const uint32_t* __restrict__ gate,
+                                                                     uint32_t per_warp) {
+    if (gate && *gate == 0u) return;
+    __shared__ RasterJob jobs[kRasterWarps][32];
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const uint32_t f = (blockIdx.x * kRasterWarps + w) * per_warp + lane;
+    RasterJob J;
+    const bool live = lane < per_warp && f < F && raster_setup(f, faces, vfix, 0u, W, row0, row1, 0ull, J);
+    const bool wide = live && J.wide != 0;
+    if (live) jobs[w][lane] = J;
+    const int part = int(blockIdx.y), parts = int(gridDim.y);
+    raster_warp<true, false>(jobs[w], __ballot_sync(kFull, live && !wide), int(lane), vproj, counts, offsets, records,
+                             part, parts);
+    raster_warp<true, true>(jobs[w], __ballot_sync(kFull, wide), int(lane), vproj, counts, offsets, records, part,
+                            parts);
+}
+
+void launch_boundary_fill(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, int row0,
+                          int row1, uint32_t* counts, const u64* offsets, u64* records, const uint32_t* gate,
+                          cudaStream_t s) {
+    if (F == 0 || row1 <= row0) return;
+    const FillSplit sp = fill_split(F, uint64_t(row1 - row0));
+    const dim3 blocks((F + sp.per_warp * kRasterWarps - 1) / (sp.per_warp * kRasterWarps), sp.parts);
+    k_boundary_fill<<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts, offsets,
+                                                         records, gate, sp.per_warp);
+}
+
 void launch_rest_fill(const ListInfo* info, const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W,
                       int row0, int row1, uint32_t* counts, const u64* offsets, u64* records, cudaStream_t s) {
     if (F) k_rest_fill<<<148 * 6, 32 * kRasterWarps, 0, s>>>(info, faces, F, vproj, vfix, W, row0, row1, counts,
@@ -180,17 +207,14 @@ void launch_raster_count(const uint4* faces, uint32_t F, const float4* vproj, co
     if (row1 <= row0) return;
     const uint32_t per_face = count_threads_per_face(F);
     const unsigned blocks = unsigned((uint64_t(F) * per_face + 32 * kRasterWarps - 1) / (32 * kRasterWarps));
-    const uint32_t per_warp = 32u / per_face;
-    if (wide_list) cudaMemsetAsync(wide_list, 0, sizeof(uint32_t), s);
     k_raster<false, false><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts, nullptr,
-                                                                nullptr, nullptr, wide_list, nullptr, per_warp);
+                                                                nullptr, nullptr, wide_list, per_face);
     if (wide_list)
         k_raster_listed<false><<<kListedCountBlocks, 32 * kRasterWarps, 0, s>>>(faces, vproj, vfix, W, row0, row1,
                                                                                 counts, nullptr, nullptr, wide_list);
     else
         k_raster<false, true><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts,
-                                                                   nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                                   per_warp);
+                                                                   nullptr, nullptr, nullptr, nullptr, per_face);
     k_row_prefix<<<unsigned(row1 - row0 + 7) / 8, 256, 0, s>>>(counts, W, row0, row1);
 }
 
@@ -198,30 +222,27 @@ void launch_raster_count(const uint4* faces, uint32_t F, const float4* vproj, co
 template <bool REST>
 static void raster_fill(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, uint32_t* counts,
                         const u64* offsets, u64* records, cudaStream_t s, int row0, int row1, const uint32_t* order,
-                        const uint32_t* wide_list, const uint32_t* gate) {
-    const FillSplit sp = fill_split(F, uint64_t(row1 - row0));
-    const uint32_t per_warp = sp.per_warp;
-    const dim3 blocks((F + per_warp * kRasterWarps - 1) / (per_warp * kRasterWarps), sp.parts);
+                        const uint32_t* wide_list) {
+    const unsigned blocks = (F + 32 * kRasterWarps - 1) / (32 * kRasterWarps);
     k_raster<true, false, REST><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts,
-                                                                     offsets, records, order, nullptr, gate, per_warp);
+                                                                     offsets, records, order, nullptr, 1u);
     if (wide_list)
         k_raster_listed<true, REST><<<kListedBlocks, 32 * kRasterWarps, 0, s>>>(faces, vproj, vfix, W, row0, row1,
                                                                                 counts, offsets, records, wide_list);
     else
         k_raster<true, true, REST><<<blocks, 32 * kRasterWarps, 0, s>>>(faces, F, vproj, vfix, W, row0, row1, counts,
-                                                                        offsets, records, order, nullptr, gate,
-                                                                        per_warp);
+                                                                        offsets, records, order, nullptr, 1u);
 }
 
 void launch_raster_fill(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, int H,
                         uint32_t* counts, const u64* offsets, u64* records, cudaStream_t s, int row0, int row1,
-                        const uint32_t* order, const uint32_t* wide_list, const uint32_t* gate, bool rest) {
+                        const uint32_t* order, const uint32_t* wide_list, bool rest) {
     if (F == 0) return;
     if (row1 < 0) row1 = H;
     if (rest)
-        raster_fill<true>(faces, F, vproj, vfix, W, counts, offsets, records, s, row0, row1, order, wide_list, gate);
+        raster_fill<true>(faces, F, vproj, vfix, W, counts, offsets, records, s, row0, row1, order, wide_list);
     else
-        raster_fill<false>(faces, F, vproj, vfix, W, counts, offsets, records, s, row0, row1, order, wide_list, gate);
+        raster_fill<false>(faces, F, vproj, vfix, W, counts, offsets, records, s, row0, row1, order, wide_list);
 }
 
 // ---------------------------------------------------------------------------
