@@ -336,17 +336,21 @@ __global__ void __launch_bounds__(256) kb_clear_counts(uint32_t* __restrict__ co
     for (u64 i = u64(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += u64(gridDim.x) * blockDim.x) counts[i] = 0;
 }
 
+// Pixel of a thread in the kernels over the views' tiles: two blocks of 16 x 8
+// pixels per tile.
+constexpr int kTileThreads = kTile * kTile / 2;
 __device__ __forceinline__ bool tile_pixel(const BatchView* views, int nviews, int& v, int& px, int& py) {
-    v = find_index(blockIdx.x, nviews, [&](int i) { return views[i].tile_base; });
+    const u64 tile = blockIdx.x >> 1;
+    v = find_index(tile, nviews, [&](int i) { return views[i].tile_base; });
     const BatchView& bv = views[v];
-    const uint32_t t = uint32_t(blockIdx.x - bv.tile_base);
+    const uint32_t t = uint32_t(tile - bv.tile_base);
     px = int((t % bv.tiles_x) * kTile + tile_x<kTile>(threadIdx.x));
-    py = int((t / bv.tiles_x) * kTile + tile_y<kTile>(threadIdx.x));
+    py = int((t / bv.tiles_x) * kTile + (blockIdx.x & 1u) * (kTile / 2) + tile_y<kTile>(threadIdx.x));
     return px < int(bv.W) && py < int(bv.H);
 }
 
 template <bool AHEAD>
-__global__ void __launch_bounds__(kTile * kTile) kb_composite(const BatchView* __restrict__ views, int nviews,
+__global__ void __launch_bounds__(kTileThreads) kb_composite(const BatchView* __restrict__ views, int nviews,
                                                               const u64* __restrict__ offsets,
                                                               const u64* __restrict__ records,
                                                               const VGeo* __restrict__ vgeo, ShadeDev sh,
@@ -363,23 +367,17 @@ __global__ void __launch_bounds__(kTile * kTile) kb_composite(const BatchView* _
 
 // Lists of every view by walking its mesh (walk_pixel), in blocks of 16 x 8
 // pixels (half a tile, four warps of 8 x 4 pixels).
-constexpr int kWalkBatchThreads = 128;
-__global__ void __launch_bounds__(kWalkBatchThreads) kb_walk_lists(
+__global__ void __launch_bounds__(kTileThreads) kb_walk_lists(
     const BatchView* __restrict__ views, int nviews, const u64* __restrict__ offsets, u64* __restrict__ records,
     uint32_t* __restrict__ counts, const WalkVertRow* __restrict__ verts, ListInfo* __restrict__ info,
     uint32_t* __restrict__ redo) {
-    constexpr int N = kWalkBatchThreads;
+    constexpr int N = kTileThreads;
     __shared__ u64 starts[kWalkStarts * N];
     __shared__ u64 recs[4 * N];
     if (info->ok == 0u) return;
-    const u64 tile = blockIdx.x >> 1;
-    const int v = find_index(tile, nviews, [&](int i) { return views[i].tile_base; });
+    int v, px, py;
+    if (!tile_pixel(views, nviews, v, px, py)) return;
     const BatchView& bv = views[v];
-    const uint32_t tl = uint32_t(tile - bv.tile_base);
-    const int lane = int(threadIdx.x & 31u), w = int(threadIdx.x >> 5);
-    const int px = int(tl % bv.tiles_x) * kTile + (w & 1) * 8 + lane % 8;
-    const int py = int(tl / bv.tiles_x) * kTile + int(blockIdx.x & 1u) * 8 + (w >> 1) * 4 + lane / 8;
-    if (px >= int(bv.W) || py >= int(bv.H)) return;
     const size_t p = size_t(py) * bv.W + px;
     walk_pixel(px, py, p, offsets + bv.pix_base, records, counts + bv.pix_base, bv.walk, verts + bv.vert_base,
                WalkSmem{starts + threadIdx.x, recs + threadIdx.x, N}, WalkRedo{&info->n_redo, redo},
@@ -421,7 +419,7 @@ __global__ void __launch_bounds__(256) kb_loss(const BatchView* __restrict__ vie
 // slots' rows; otherwise world-space rows go straight to the slot (views of
 // one mesh share them).
 template <bool SCREEN>
-__global__ void __launch_bounds__(kTile * kTile, 2) kb_adjoint(const BatchView* __restrict__ views, int nviews,
+__global__ void __launch_bounds__(kTileThreads, 4) kb_adjoint(const BatchView* __restrict__ views, int nviews,
                                                             const u64* __restrict__ offsets,
                                                             const u64* __restrict__ records,
                                                             const VGeo* __restrict__ vgeo, ShadeDev sh,
@@ -430,8 +428,8 @@ __global__ void __launch_bounds__(kTile * kTile, 2) kb_adjoint(const BatchView* 
                                                             float4* __restrict__ grad_rows,
                                                             float4* __restrict__ view_rows, size_t copy_stride,
                                                             uint32_t copies, const uint32_t* __restrict__ ok) {
-    __shared__ float4 vcache4[3 * kTile * kTile];
-    __shared__ float vcache1[3 * kTile * kTile];
+    __shared__ float4 vcache4[3 * kTileThreads];
+    __shared__ float vcache1[3 * kTileThreads];
     if (!batch_ok(ok)) return;
     int v, px, py;
     if (!tile_pixel(views, nviews, v, px, py)) return;
@@ -440,12 +438,12 @@ __global__ void __launch_bounds__(kTile * kTile, 2) kb_adjoint(const BatchView* 
     float4* rows = SCREEN ? block_rows(view_rows, copies, copy_stride) + 2 * bv.vert_base
                           : grad_rows + 2 * bv.grad_base;
     if constexpr (SCREEN) {
-        OrderedRowsSmem acc{rows, vcache4 + threadIdx.x, vcache1 + threadIdx.x, kTile * kTile};
+        OrderedRowsSmem acc{rows, vcache4 + threadIdx.x, vcache1 + threadIdx.x, kTileThreads};
         adjoint_pixel<OrderedRowsSmem, SCREEN>(px, py, offsets + bv.pix_base, records, bv.faces, vgeo + bv.vert_base,
                                            bv.colors, int(bv.W), bv.cam, sh, bv.dimage, tfinal + bv.pix_base,
                                            term + bv.pix_base, acc);
     } else {
-        VertCache acc{rows, vcache4 + threadIdx.x, vcache1 + threadIdx.x, kTile * kTile};
+        VertCache acc{rows, vcache4 + threadIdx.x, vcache1 + threadIdx.x, kTileThreads};
         adjoint_pixel<VertCache, SCREEN>(px, py, offsets + bv.pix_base, records, bv.faces, vgeo + bv.vert_base,
                                          bv.colors, int(bv.W), bv.cam, sh, bv.dimage, tfinal + bv.pix_base,
                                          term + bv.pix_base, acc);
@@ -804,7 +802,7 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
             kb_boundary_fill<<<bb, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_bfaces, b->vproj.ptr, b->vfix.ptr,
                                                 b->counts.ptr, b->offsets.ptr, b->records.ptr, okp, sp.per_warp);
         }
-        kb_walk_lists<<<unsigned(2 * b->tot_tiles), kWalkBatchThreads, 0, s>>>(
+        kb_walk_lists<<<unsigned(2 * b->tot_tiles), kTileThreads, 0, s>>>(
             b->d_views.ptr, b->nviews, b->offsets.ptr, b->records.ptr, b->counts.ptr, b->walk_verts.ptr, b->info.ptr,
             b->redo.ptr);
         if (b->many_left) {
@@ -824,7 +822,7 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
     const u64 n = b->nviews > 0 ? u64(b->nviews) : 1;
     const auto composite = composite_ahead(b->tot_verts / n, b->tot_pixels / n, b->tot_pixels) ? kb_composite<true>
                                                                                                : kb_composite<false>;
-    composite<<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(b->d_views.ptr, b->nviews, b->offsets.ptr,
+    composite<<<unsigned(2 * b->tot_tiles), kTileThreads, 0, s>>>(b->d_views.ptr, b->nviews, b->offsets.ptr,
                                                                b->records.ptr, b->vgeo.ptr, sh, b->tfinal.ptr,
                                                                b->term.ptr, okp);
 }
@@ -835,7 +833,7 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
 void enqueue_adjoint(dtv_batch* b, const dtv::ShadeDev& sh, const uint32_t* okp, cudaStream_t s) {
     using namespace dtv;
     if (sh.use_abs_grad) {
-        kb_adjoint<false><<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(
+        kb_adjoint<false><<<unsigned(2 * b->tot_tiles), kTileThreads, 0, s>>>(
             b->d_views.ptr, b->nviews, b->offsets.ptr, b->records.ptr, b->vgeo.ptr, sh, b->tfinal.ptr, b->term.ptr,
             b->grad_rows.ptr, b->view_rows.ptr, 0, 1, okp);
         return;
@@ -843,7 +841,7 @@ void enqueue_adjoint(dtv_batch* b, const dtv::ShadeDev& sh, const uint32_t* okp,
     const uint32_t copies = view_copies(b);
     const size_t stride = 2 * size_t(b->tot_verts);
     DTV_CK(cudaMemsetAsync(b->view_rows.ptr, 0, sizeof(float4) * stride * copies, s));
-    kb_adjoint<true><<<unsigned(b->tot_tiles), kTile * kTile, 0, s>>>(
+    kb_adjoint<true><<<unsigned(2 * b->tot_tiles), kTileThreads, 0, s>>>(
         b->d_views.ptr, b->nviews, b->offsets.ptr, b->records.ptr, b->vgeo.ptr, sh, b->tfinal.ptr, b->term.ptr,
         b->grad_rows.ptr, b->view_rows.ptr, stride, copies, okp);
     kb_view_rows<<<grid_for(b->tot_verts, 256, 0x7fffffffu), 256, 0, s>>>(

@@ -131,7 +131,7 @@ constexpr uint32_t kSortWarpCap = 1024;    // elements per warp list sorted in s
 constexpr uint32_t kSortBlockCap = 16384;  // elements per block-sorted list / chunk of a longer one (128 KiB shared memory)
 
 // gate (optional): nothing is done when *gate is zero.
-// tile: pixel tile of the 256-thread blocks (0: 16 x 16, 1: 32 x 8, 2: 8 x 32).
+// tile: pixel tile of the 128-thread blocks (0: 16 x 8, 1: 32 x 4, 2: 8 x 16).
 // Whether the composite loads ahead (composite_pixel): a pixel's list is a chain
 // of dependent loads, and running ahead of it is worth half the warps when the
 // pixels do not fill the GPU with plain ones anyway, and later only while the

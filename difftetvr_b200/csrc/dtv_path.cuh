@@ -9,7 +9,7 @@
 namespace dtv {
 
 using u64 = unsigned long long;
-constexpr int kTile = 16;  // composite / adjoint pixel tile (16 x 16 threads)
+constexpr int kTile = 16;  // pixel tile width
 
 // Pixel of thread t in a block TX pixels wide: its warps are 8 x 4 pixels.
 template <int TX>
@@ -483,7 +483,7 @@ __device__ __forceinline__ void write_pixel(float4* __restrict__ image, float* _
 }
 
 // ---------------------------------------------------------------------------
-// (d) front-to-back compositing, one thread per pixel (16x16 pixel tiles).
+// (d) front-to-back compositing, one thread per pixel.
 // Forward.glsl:159-211 with early ray termination (:169-173) and the
 // termination index (:256-259); final transmittance is kept for the adjoint.
 // PIPE: the dependent loads record -> face -> vertices run ahead (the vertices
