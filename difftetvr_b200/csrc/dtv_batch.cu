@@ -708,10 +708,24 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
     b->max_height = mh;
 }
 
-// Copies of the views' gradient rows (grad_copies on the mean view).
+// Copies of the views' gradient rows (grad_copies on the mean view), together
+// at most kBatchGradRows rows (64 MiB) beyond the first copy: a batch of many
+// views spreads its atomics over their rows already, and a reserved batch
+// holds the copies from the start.
+constexpr u64 kBatchGradRows = 1u << 21;
 uint32_t view_copies(const dtv_batch* b) {
-    const uint64_t n = b->nviews > 0 ? uint64_t(b->nviews) : 1;
-    return dtv::grad_copies((b->tot_verts + n - 1) / n, b->tot_pixels / n);
+    const u64 n = b->nviews > 0 ? u64(b->nviews) : 1;
+    uint32_t c = dtv::grad_copies((b->tot_verts + n - 1) / n, b->tot_pixels / n);
+    while (c > 1 && c * b->tot_verts > kBatchGradRows) c /= 2;
+    return c;
+}
+
+// Most rows that view_copies gives a batch of up to nv views, V vertices and P
+// pixels.
+u64 most_view_rows(u64 nv, u64 V, u64 P) {
+    const u64 per_view = nv <= kBatchGradRows / dtv::kGradRows ? nv * dtv::kGradRows : kBatchGradRows;
+    const u64 by_pixels = std::min<u64>(P / dtv::kGradCopyPixels, 64);
+    return std::max(V, std::min(per_view, by_pixels * std::min(V, kBatchGradRows)));
 }
 
 void ensure_scratch(dtv_batch* b, cudaStream_t s) {
@@ -921,9 +935,7 @@ int32_t dtv_batch_reserve(dtv_batch* b, uint64_t max_views, uint64_t max_vertice
         b->vproj.ensure(V, s);
         b->vfix.ensure(V, s);
         b->vgeo.ensure(V, s);
-        // Batches of small meshes hold copies of their rows: at most kGradRows
-        // rows per view, grown at the first such batch.
-        b->view_rows.ensure(2 * V, s);
+        b->view_rows.ensure(2 * size_t(most_view_rows(nv, V, P)), s);
         // Fill order: a Kuhn-grid tet mesh has about 12 faces per vertex; a
         // batch with more faces grows it at its first render.
         b->fill_order.ensure(13 * V, s);

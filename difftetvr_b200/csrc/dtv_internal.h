@@ -157,9 +157,10 @@ void launch_composite(const unsigned long long* offsets, const unsigned long lon
 // 983 and 975 at 16^3.  One copy per 8192 pixels at most: a small image has no
 // contention to spread, and clearing and summing 64 copies cost 12 us.
 constexpr uint64_t kGradRows = 1u << 17;
+constexpr uint64_t kGradCopyPixels = 8192;
 inline uint32_t grad_copies(uint64_t rows, uint64_t pixels) {
     uint32_t c = 1;
-    while (c < 64 && 2 * uint64_t(c) * rows <= kGradRows && 2 * uint64_t(c) * 8192 <= pixels) c *= 2;
+    while (c < 64 && 2 * uint64_t(c) * rows <= kGradRows && 2 * uint64_t(c) * kGradCopyPixels <= pixels) c *= 2;
     return c;
 }
 // Adjoint of pixel rows [row0, row1) into the copies of grad_rows ([copies][V][2];
