@@ -710,8 +710,9 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
             rec_event(r, 5, s);
         }
         if (raytet) {
+            const dtv::WalkMesh wm = mesh->walkable ? walk_mesh(mesh) : dtv::WalkMesh{};
             dtv::launch_walk_composite(r->offsets.ptr, r->records.ptr, mesh->d_bf_global, mesh->d_faces,
-                                       mesh->d_face_to_tet, mesh->d_tet_faces, mesh->d_cells, mesh->d_tet_flip,
+                                       mesh->d_face_to_tet, mesh->d_tet_faces, mesh->d_cells, mesh->d_tet_flip, wm,
                                        uint32_t(mesh->host.num_cells),
                                        r->vfix.ptr, r->vgeo.ptr, reinterpret_cast<const float4*>(d_colors), cam, sh,
                                        reinterpret_cast<float4*>(d_image), r->tfinal.ptr, r->wstate.ptr, s);
@@ -756,8 +757,9 @@ int32_t adjoint_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_pos
             adjoint_banded(r, mesh, d_colors, d_image_adjoint, sh, d_grad_positions, d_grad_colors, s);
         } else if (r->type == DTV_RENDERER_INTERSECTION) {
             r->grad_rows.ensure(2 * size_t(r->V ? r->V : 1) * dtv::grad_copies(r->V, r->P), s);
+            const dtv::WalkMesh wm = mesh->walkable ? walk_mesh(mesh) : dtv::WalkMesh{};
             dtv::launch_walk_adjoint(r->offsets.ptr, r->records.ptr, mesh->d_bf_global, mesh->d_faces,
-                                     mesh->d_face_to_tet, mesh->d_tet_faces, mesh->d_cells, mesh->d_tet_flip,
+                                     mesh->d_face_to_tet, mesh->d_tet_faces, mesh->d_cells, mesh->d_tet_flip, wm,
                                      uint32_t(mesh->host.num_cells),
                                      r->vfix.ptr, r->vgeo.ptr, reinterpret_cast<const float4*>(d_colors), r->cam, sh,
                                      reinterpret_cast<const float4*>(d_image_adjoint), r->tfinal.ptr,

@@ -205,13 +205,13 @@ void launch_scatter_positions(const float4* grad_rows, uint32_t V, uint32_t copi
 // Ray-tet path (dtv_raytet.cu).
 void launch_walk_composite(const unsigned long long* b_offsets, const unsigned long long* b_records,
                            const uint32_t* bf_global, const uint4* faces, const uint32_t* face_to_tet,
-                           const uint32_t* tet_faces, const uint32_t* cells, const uint8_t* tet_flip,
+                           const uint32_t* tet_faces, const uint32_t* cells, const uint8_t* tet_flip, const WalkMesh& wm,
                            uint32_t num_tets, const int2* vfix, const VGeo* vgeo,
                            const float4* colors, const CamDev& cam, const ShadeDev& sh, float4* image,
                            float* tfinal, uint4* wstate, cudaStream_t s);
 void launch_walk_adjoint(const unsigned long long* b_offsets, const unsigned long long* b_records,
                          const uint32_t* bf_global, const uint4* faces, const uint32_t* face_to_tet,
-                         const uint32_t* tet_faces, const uint32_t* cells, const uint8_t* tet_flip,
+                         const uint32_t* tet_faces, const uint32_t* cells, const uint8_t* tet_flip, const WalkMesh& wm,
                          uint32_t num_tets, const int2* vfix, const VGeo* vgeo,
                          const float4* colors, const CamDev& cam, const ShadeDev& sh, const float4* dimage,
                          const float* tfinal, const uint4* wstate, uint32_t V, float4* grad_rows, uint32_t copies, float* grad_pos,

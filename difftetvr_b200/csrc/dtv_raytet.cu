@@ -14,13 +14,15 @@
 // count / scan / fill / sort over the boundary faces only); from a tet entered
 // through face fe the ray leaves through the back face that covers the pixel
 // under the rasteriser's exact fixed-point rule, and continues into the tet on
-// the other side of that face until it leaves through a boundary face.  No
+// the other side of that face until it leaves through a boundary face; on a
+// mesh with walk tables the step is taken on its links (ray_step).  No
 // per-fragment storage exists beyond the boundary lists; the adjoint walks the
 // same tets backwards (previous tet = the one across the entry face), so the
 // backward pass needs no stored lists either.  Walks are bounded by the tet
 // count (a malformed mesh cannot loop forever).
 #include "dtv_internal.h"
 #include "dtv_path.cuh"
+#include "dtv_walk.cuh"
 
 namespace dtv {
 
@@ -168,21 +170,157 @@ __device__ __forceinline__ uint32_t other_tet(const uint32_t* __restrict__ f2t, 
     return a == t ? b : a;
 }
 
+// Walk on the mesh's links (meshes with walk tables).  A face search needs the
+// tet's four vertices and table rows; a linked step carries the snapped
+// positions of the face it stands on, so it reads one new vertex (whose row the
+// next face's fragment reads as well) and one 16-byte link, and three edge
+// signs (walk_side, exact) decide which face the ray leaves through.  As a tet's
+// projected faces cover a pixel in pairs of opposite orientation, the one
+// found is the face tet_face_of looks for if it faces the wanted way, and
+// otherwise there is none.  Steps at vertices that are not projected or too far
+// off screen for exact signs, and the rest of such an interval, search.
+// Searched -> linked (us): forward 2,878 -> 2,291 and adjoint 5,264 -> 4,507 at
+// 64^3 / 1024^2, 101 -> 82 and 177 -> 141 at 16^3 / 256^2, 653 -> 263 and 1,002
+// -> 603 at 8^3 / 1000^2, where many steps had vertices beyond 64 px and searched
+// in 64 bits.  What is left is the segment and gradient arithmetic of the lists'
+// composite and adjoint, bound by instruction issue.
+struct RayVert {
+    float sx, sy;   // snapped position relative to the pixel centre
+};
+
+__device__ __forceinline__ RayVert ray_vertex(uint32_t id, float qx, float qy, const VGeo* __restrict__ vgeo) {
+    const float2 q = *reinterpret_cast<const float2*>(vgeo + id);
+    return RayVert{__fsub_rn(q.x, qx), __fsub_rn(q.y, qy)};
+}
+
+// The face a linked walk stands on: three vertex slots, then the tet ahead.
+struct RayFace {
+    RayVert a, b, c;
+    RayVert d;        // the tet's vertex off the face
+    uint32_t t, dn;   // the tet, d's id
+    uint32_t loc;     // local indices in t of the slots' vertices, one byte each, and of d
+    bool rev;         // a, b, c wind counterclockwise on screen
+    bool wound;       // the face winds clockwise in t's own vertex order
+    bool far;         // a vertex without exact signs was met
+};
+
+__device__ __forceinline__ void ray_load(RayFace& r, uint32_t v0, uint32_t v1, uint32_t v2, float qx, float qy,
+                                         const VGeo* __restrict__ vgeo) {
+    r.a = ray_vertex(v0, qx, qy, vgeo);
+    r.b = ray_vertex(v1, qx, qy, vgeo);
+    r.c = ray_vertex(v2, qx, qy, vgeo);
+    r.d = ray_vertex(r.dn, qx, qy, vgeo);
+    r.far = !(walk_usable(r.a) & walk_usable(r.b) & walk_usable(r.c));
+}
+
+// On boundary face bk (bf), looking into the mesh; `front`: it faces the camera.
+__device__ __forceinline__ RayFace ray_boundary(uint32_t bk, const uint4& bf, bool front, float qx, float qy,
+                                                const WalkMesh& wm, const VGeo* __restrict__ vgeo) {
+    const uint4 s0 = wm.start[bk];
+    RayFace r;
+    r.t = s0.x;
+    r.dn = s0.y;
+    r.loc = s0.z;
+    r.rev = !front;
+    r.wound = front;
+    ray_load(r, bf.x, bf.y, bf.z, qx, qy, vgeo);
+    prefetch_links(wm.links + 4 * size_t(r.t));
+    return r;
+}
+
+// On face fx (vertices fc) of tet t, which faces away from the camera as seen
+// from t, looking into t.
+__device__ __forceinline__ RayFace ray_inside(uint32_t t, uint32_t fx, const uint4& fc, const TetRow& tr, float qx,
+                                              float qy, const WalkMesh& wm, const VGeo* __restrict__ vgeo) {
+    const uint32_t k = tr.tf.x == fx ? 3u : (tr.tf.y == fx ? 2u : (tr.tf.z == fx ? 1u : 0u));
+    const uint32_t c[4] = {tr.cv.x, tr.cv.y, tr.cv.z, tr.cv.w}, s[3] = {fc.x, fc.y, fc.z};
+    RayFace r;
+    r.loc = k << 24;
+    r.dn = c[0];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+        if (q == k) r.dn = c[q];
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            if (c[q] == s[j]) r.loc |= q << (8 * j);
+    }
+    const uint4 lk = wm.links[4 * size_t(t) + k];
+    r.t = t;
+    r.wound = ((lk.x >> 30) & 1u) != 0u;
+    r.rev = r.wound == ((lk.y & 1u) != 0u);
+    ray_load(r, fc.x, fc.y, fc.z, qx, qy, vgeo);
+    return r;
+}
+
+// Local vertex opposite the face that tet_face_of finds from r (4: none).
+__device__ __noinline__ uint32_t ray_search(const TetTopo tt, const int2* __restrict__ vfix, uint32_t t, uint32_t skip,
+                                            bool want_front, int px, int py) {
+    const TetRow tr = load_tet(tt, t);
+    const uint32_t f = tet_face_of(tr, vfix, skip, want_front, px, py);
+    if (f == kNoTet) return 4u;
+    return tr.tf.x == f ? 3u : (tr.tf.y == f ? 2u : (tr.tf.z == f ? 1u : 0u));
+}
+
+// Goes on to the other face of r.t that the ray crosses, if it faces the camera
+// as seen from r.t (FRONT) or away from it (else false).  lk: that face's link,
+// slot: the slot whose vertex was replaced, at: r's face before the step.
+template <bool FRONT>
+__device__ __forceinline__ bool ray_step(RayFace& r, uint32_t at, const TetTopo& tt, const int2* __restrict__ vfix,
+                                         const WalkMesh& wm, const VGeo* __restrict__ vgeo, int px, int py, uint4& lk,
+                                         uint32_t& slot) {
+    const float qx = float(px) + 0.5f, qy = float(py) + 0.5f;
+    r.far |= !walk_usable(r.d);
+    bool drop_a, drop_b, drop_c;
+    uint32_t k;
+    if (!r.far) {
+        const bool la = walk_side(r.a, r.d) != r.rev, lb = walk_side(r.b, r.d) != r.rev,
+                   lc = walk_side(r.c, r.d) != r.rev;
+        drop_c = la & !lb;
+        drop_a = !drop_c & lb & !lc;
+        drop_b = !drop_c & !drop_a;
+        k = (drop_a ? r.loc : (drop_b ? r.loc >> 8 : r.loc >> 16)) & 3u;
+    } else {
+        k = ray_search(tt, vfix, r.t, at, FRONT, px, py);
+        if (k == 4u) return false;
+        drop_a = (r.loc & 3u) == k;
+        drop_b = ((r.loc >> 8) & 3u) == k;
+        drop_c = !drop_a & !drop_b;
+    }
+    lk = wm.links[4 * size_t(r.t) + k];
+    if ((r.wound == (((lk.x >> 30) & 1u) != 0u)) != FRONT) return false;
+    if (drop_a) r.a = r.d;
+    if (drop_b) r.b = r.d;
+    if (drop_c) r.c = r.d;
+    slot = drop_a ? 0u : (drop_b ? 1u : 2u);
+    // d takes the slot; the local indices become the next tet's.
+    const uint32_t loc = __byte_perm(r.loc, 0u, drop_a ? 0x4213u : (drop_b ? 0x4230u : 0x4310u));
+    const uint32_t sel = (loc & 0x3u) | ((loc >> 4) & 0x30u) | ((loc >> 8) & 0x300u) | (k << 12);
+    r.loc = __byte_perm(lk.w, 0u, sel);
+    r.t = lk.x & kWalkNoTet;
+    r.wound = r.wound != ((lk.x >> 31) != 0u);
+    r.dn = lk.z;
+    r.d = ray_vertex(lk.z, qx, qy, vgeo);
+    if (!(lk.y & 2u)) prefetch_links(wm.links + 4 * size_t(r.t));
+    return true;
+}
+
 // Length of the pixel ray per unit of view depth (|d| with d.z_view = -1).
 __device__ __forceinline__ float ray_scale(const CamDev& cam, float qx, float qy) {
     const float dx = (qx - cam.cx) / cam.f, dy = (qy - cam.cy) / cam.f;
     return sqrtf(1.f + dx * dx + dy * dy);
 }
 
-// The forward walk in 16 x 8 pixel blocks, five per SM (96 registers): the
-// walk is bound by the latency of its tet -> faces -> vertices chain, and 20
-// warps per SM hide more of it than 16 at 110 registers (3.59 -> 3.22 ms at
-// 64^3 / 1024^2).
+// Both walks in 16 x 8 pixel blocks, as rays differ in length (adjoint at 8^3 /
+// 1000^2: 645 us in 16 x 16 blocks, 603 in these).  The forward walk with five
+// per SM (96 registers): it is bound by the latency of its tet -> vertex chain,
+// which 20 warps per SM hide better than 16 (2,481 -> 2,291 us at 64^3 / 1024^2).
 constexpr int kWalkRows = 8;
 constexpr int kWalkThreads = kTile * kWalkRows;
+template <bool LINKED>
 __global__ void __launch_bounds__(kWalkThreads, 5) k_walk_composite(
     const u64* __restrict__ b_offsets, const u64* __restrict__ b_records, const uint32_t* __restrict__ bf_global,
-    const uint4* __restrict__ faces, const uint32_t* __restrict__ f2t, TetTopo tt, uint32_t num_tets, const int2* __restrict__ vfix, const VGeo* __restrict__ vgeo,
+    const uint4* __restrict__ faces, const uint32_t* __restrict__ f2t, TetTopo tt, WalkMesh wm,
+    uint32_t num_tets, const int2* __restrict__ vfix, const VGeo* __restrict__ vgeo,
     const float4* __restrict__ colors, CamDev cam, ShadeDev sh, float4* __restrict__ image,
     float* __restrict__ tfinal, uint4* __restrict__ wstate) {
     const int px = blockIdx.x * kTile + tile_x<kTile>(threadIdx.x);
@@ -200,6 +338,33 @@ __global__ void __launch_bounds__(kWalkThreads, 5) k_walk_composite(
     for (uint32_t b = 0; b < nb && !stop; ++b) {
         const uint32_t bits = uint32_t(b_records[beg + b]);
         if (!(bits & 1u)) continue;  // intervals start at front-facing boundary faces
+        if constexpr (LINKED) {
+            const uint4 bf = wm.bfaces[bits >> 2];
+            RayFace r = ray_boundary(bits >> 2, bf, true, qx, qy, wm, vgeo);
+            uint32_t fe = bf_global[bits >> 2];
+            FragV f0 = load_frag_face(fe << 2, bf, qx, qy, vgeo, colors);
+            for (uint32_t step = 0; step <= num_tets; ++step) {
+                const uint32_t t = r.t;
+                uint4 lk;
+                uint32_t slot;
+                if (!ray_step<false>(r, fe, tt, vfix, wm, vgeo, px, py, lk, slot)) break;
+                if (sh.use_ert && T.hi < sh.ert_thresh) {
+                    stop = true;
+                    break;
+                }
+                const uint32_t fx = lk.y >> 2;
+                const FragV f1 = load_frag_face(fx << 2, faces[fx], qx, qy, vgeo, colors);
+                segment_composite((f1.z - f0.z) * scale * 0.25f, f0.col, f1.col, sh.atten, C0, C1, C2, T);
+                last_tet = t;
+                last_entry = fe;
+                last_b = b;
+                ++nseg;
+                if (lk.y & 2u) break;  // leaving the mesh
+                fe = fx;
+                f0 = f1;
+            }
+            continue;
+        }
         uint32_t fe = bf_global[bits >> 2];
         uint32_t t = f2t[2 * size_t(fe)];
         FragV f0 = load_frag(u64(fe) << 2, qx, qy, faces, vgeo, colors);
@@ -309,15 +474,77 @@ __device__ __forceinline__ void walk_adjoint_carried(
     acc.flush();
 }
 
-template <bool SCREEN>
-__global__ void __launch_bounds__(kTile * kTile, 2) k_walk_adjoint(
+// The same on the mesh's links: a step's entry face is the exit face with one
+// vertex replaced, so its vertices need neither a face load nor a comparison to
+// come in the row cache's order.
+template <class Acc>
+__device__ __forceinline__ void walk_adjoint_linked(
+    const u64* __restrict__ b_records, u64 beg, const uint32_t* __restrict__ bf_global,
+    const uint4* __restrict__ faces, const TetTopo& tt, const WalkMesh& wm, uint32_t num_tets,
+    const int2* __restrict__ vfix, const VGeo* __restrict__ vgeo, const float4* __restrict__ colors, int px, int py,
+    float scale, float atten, float gC0, float gC1, float gC2, TransBack T, TransF gT, uint32_t t, uint32_t fx, int b,
+    Acc& acc) {
+    const float qx = float(px) + 0.5f, qy = float(py) + 0.5f;
+    const uint4 fcx = faces[fx];
+    RayFace r = ray_inside(t, fx, fcx, load_tet(tt, t), qx, qy, wm, vgeo);
+    FragG fX = load_frag_g(fx << 2, fcx, qx, qy, vgeo, colors, gC0, gC1, gC2);
+    float gz_x = 0.f, wx = 0.f, ax = 0.f;
+    uint32_t open = 0u;
+    for (uint32_t step = 0; step <= num_tets; ++step) {
+        uint4 lk;
+        uint32_t slot;
+        const uint32_t dn = r.dn;
+        if (!ray_step<true>(r, fx, tt, vfix, wm, vgeo, px, py, lk, slot)) break;
+        fx = lk.y >> 2;
+        const uint32_t keep = 7u & ~(1u << slot);
+        const FragG fE = load_frag_g(fx << 2, slot == 0u ? dn : fX.v[0], slot == 1u ? dn : fX.v[1],
+                                     slot == 2u ? dn : fX.v[2], keep, qx, qy, vgeo, colors, gC0, gC1, gC2);
+        const float tSeg = (fX.z - fE.z) * scale * 0.25f;
+        float g_tot = 0.f, we = 0.f, ae = 0.f;
+        segment_adjoint(tSeg, fE.alpha, fX.alpha, fE.pcol, fX.pcol, atten, T, gT, g_tot, we, wx, ae, ax);
+        const float gz_e = -g_tot * scale;
+        gz_x += g_tot * scale;
+        frag_grads_carried(fX, gz_x, wx, ax, keep, acc);
+        if (lk.y & 2u) {
+            frag_grads_carried(fE, gz_e, we, ae, 0u, acc);
+            open = 0u;
+            // Previous interval: its exit is the last back-facing boundary fragment before b.
+            int bb = b - 1;
+            while (bb >= 0 && (uint32_t(b_records[beg + bb]) & 1u)) --bb;
+            if (bb < 0) break;
+            const uint32_t bk = uint32_t(b_records[beg + bb]) >> 2;
+            const uint4 bf = wm.bfaces[bk];
+            r = ray_boundary(bk, bf, false, qx, qy, wm, vgeo);
+            fx = bf_global[bk];
+            int be = bb - 1;
+            while (be >= 0 && !(uint32_t(b_records[beg + be]) & 1u)) --be;
+            b = be < 0 ? 0 : be;
+            fX = load_frag_g(fx << 2, bf, qx, qy, vgeo, colors, gC0, gC1, gC2);
+            gz_x = 0.f;
+            wx = 0.f;
+            ax = 0.f;
+            continue;
+        }
+        open = keep;
+        fX = fE;
+        gz_x = gz_e;
+        wx = we;
+        ax = ae;
+    }
+    acc.close(fX.v, open);
+    acc.flush();
+}
+
+template <bool SCREEN, bool LINKED>
+__global__ void __launch_bounds__(kWalkThreads, 4) k_walk_adjoint(
     const u64* __restrict__ b_offsets, const u64* __restrict__ b_records, const uint32_t* __restrict__ bf_global,
-    const uint4* __restrict__ faces, const uint32_t* __restrict__ f2t, TetTopo tt, uint32_t num_tets, const int2* __restrict__ vfix, const VGeo* __restrict__ vgeo,
+    const uint4* __restrict__ faces, const uint32_t* __restrict__ f2t, TetTopo tt, WalkMesh wm,
+    uint32_t num_tets, const int2* __restrict__ vfix, const VGeo* __restrict__ vgeo,
     const float4* __restrict__ colors, CamDev cam, ShadeDev sh, const float4* __restrict__ dimage,
     const float* __restrict__ tfinal, const uint4* __restrict__ wstate, float4* __restrict__ row_copies, uint32_t V,
     uint32_t copies) {
     const int px = blockIdx.x * kTile + tile_x<kTile>(threadIdx.x);
-    const int py = blockIdx.y * kTile + tile_y<kTile>(threadIdx.x);
+    const int py = blockIdx.y * kWalkRows + tile_y<kTile>(threadIdx.x);
     if (px >= cam.W || py >= cam.H) return;
     const size_t p = size_t(py) * cam.W + px;
     const uint4 ws = wstate[p];
@@ -338,11 +565,15 @@ __global__ void __launch_bounds__(kTile * kTile, 2) k_walk_adjoint(
     if (fx == kNoTet) return;
     float4* grad_rows = block_rows(row_copies, copies, 2 * size_t(V));
     if constexpr (SCREEN) {
-        __shared__ float4 vcache4[3 * kTile * kTile];
-        __shared__ float vcache1[3 * kTile * kTile];
-        OrderedRowsSmem acc{grad_rows, vcache4 + threadIdx.x, vcache1 + threadIdx.x, kTile * kTile};
+        __shared__ float4 vcache4[3 * kWalkThreads];
+        __shared__ float vcache1[3 * kWalkThreads];
+        OrderedRowsSmem acc{grad_rows, vcache4 + threadIdx.x, vcache1 + threadIdx.x, kWalkThreads};
         acc.set_pixel(gC0, gC1, gC2);
-        walk_adjoint_carried(b_records, beg, bf_global, faces, f2t, tt, num_tets, vfix, vgeo, colors, px, py, scale,
+        if constexpr (LINKED)
+            walk_adjoint_linked(b_records, beg, bf_global, faces, tt, wm, num_tets, vfix, vgeo, colors, px, py, scale,
+                                atten, gC0, gC1, gC2, T, gT, t, fx, b, acc);
+        else
+            walk_adjoint_carried(b_records, beg, bf_global, faces, f2t, tt, num_tets, vfix, vgeo, colors, px, py, scale,
                              atten, gC0, gC1, gC2, T, gT, t, fe, fx, b, acc);
         return;
     }
@@ -401,35 +632,33 @@ __global__ void __launch_bounds__(kTile * kTile, 2) k_walk_adjoint(
 
 void launch_walk_composite(const u64* b_offsets, const u64* b_records, const uint32_t* bf_global,
                            const uint4* faces, const uint32_t* face_to_tet, const uint32_t* tet_faces,
-                           const uint32_t* cells, const uint8_t* tet_flip, uint32_t num_tets, const int2* vfix, const VGeo* vgeo, const float4* colors,
+                           const uint32_t* cells, const uint8_t* tet_flip, const WalkMesh& wm,
+                           uint32_t num_tets, const int2* vfix, const VGeo* vgeo, const float4* colors,
                            const CamDev& cam, const ShadeDev& sh, float4* image, float* tfinal, uint4* wstate,
                            cudaStream_t s) {
     dim3 grid((cam.W + kTile - 1) / kTile, (cam.H + kWalkRows - 1) / kWalkRows);
     const TetTopo tt{reinterpret_cast<const uint4*>(tet_faces), reinterpret_cast<const uint4*>(cells), tet_flip};
-    k_walk_composite<<<grid, kWalkThreads, 0, s>>>(b_offsets, b_records, bf_global, faces, face_to_tet, tt,
-                                                    num_tets, vfix, vgeo, colors, cam, sh, image, tfinal, wstate);
+    const auto kernel = wm.links ? k_walk_composite<true> : k_walk_composite<false>;
+    kernel<<<grid, kWalkThreads, 0, s>>>(b_offsets, b_records, bf_global, faces, face_to_tet, tt, wm, num_tets, vfix, vgeo, colors, cam, sh, image, tfinal, wstate);
 }
 
 void launch_walk_adjoint(const u64* b_offsets, const u64* b_records, const uint32_t* bf_global, const uint4* faces,
                          const uint32_t* face_to_tet, const uint32_t* tet_faces, const uint32_t* cells,
-                         const uint8_t* tet_flip, uint32_t num_tets,
+                         const uint8_t* tet_flip, const WalkMesh& wm, uint32_t num_tets,
                          const int2* vfix, const VGeo* vgeo, const float4* colors, const CamDev& cam,
                          const ShadeDev& sh, const float4* dimage, const float* tfinal, const uint4* wstate,
                          uint32_t V, float4* grad_rows, uint32_t copies, float* grad_pos, float4* grad_col,
                          cudaStream_t s) {
     cudaMemsetAsync(grad_rows, 0, sizeof(float4) * 2 * size_t(V) * copies, s);
-    dim3 grid((cam.W + kTile - 1) / kTile, (cam.H + kTile - 1) / kTile);
+    dim3 grid((cam.W + kTile - 1) / kTile, (cam.H + kWalkRows - 1) / kWalkRows);
     const TetTopo tt{reinterpret_cast<const uint4*>(tet_faces), reinterpret_cast<const uint4*>(cells), tet_flip};
     // Screen-space position rows unless absolute gradients are asked for
     // (frag_vertex_grads); the scatter converts them per vertex.
-    if (sh.use_abs_grad)
-        k_walk_adjoint<false><<<grid, kTile * kTile, 0, s>>>(b_offsets, b_records, bf_global, faces, face_to_tet,
-                                                             tt, num_tets, vfix, vgeo, colors, cam, sh, dimage,
-                                                             tfinal, wstate, grad_rows, V, copies);
-    else
-        k_walk_adjoint<true><<<grid, kTile * kTile, 0, s>>>(b_offsets, b_records, bf_global, faces, face_to_tet,
-                                                            tt, num_tets, vfix, vgeo, colors, cam, sh, dimage,
-                                                            tfinal, wstate, grad_rows, V, copies);
+    const auto kernel = sh.use_abs_grad ? k_walk_adjoint<false, false>
+                        : wm.links      ? k_walk_adjoint<true, true>
+                                        : k_walk_adjoint<true, false>;
+    kernel<<<grid, kWalkThreads, 0, s>>>(b_offsets, b_records, bf_global, faces, face_to_tet, tt, wm, num_tets, vfix,
+                                          vgeo, colors, cam, sh, dimage, tfinal, wstate, grad_rows, V, copies);
     launch_scatter_grads(grad_rows, V, copies, grad_pos, grad_col, s, sh.use_abs_grad ? nullptr : vgeo, &cam);
 }
 

@@ -46,8 +46,9 @@ struct alignas(32) WalkVertRow {
 // Walk tables of a mesh.  links[4 t + k] belongs to the face opposite tet t's
 // local vertex k:
 //   x  bits 0..27 the tet across the face (0x0fffffff: none), 28..29 the local
-//      vertex that is the face's third stored vertex, 31 whether the two tets'
-//      vertex orders wind the face alike
+//      vertex that is the face's third stored vertex, 30 the face's bit of the
+//      mesh's tet_flip, 31 whether the two tets' vertex orders wind the face
+//      alike
 //   y  face << 2 | boundary << 1 | whether the stored winding is odd against
 //      the tet's own vertex order
 //   z  the vertex of the tet across that is not on the face

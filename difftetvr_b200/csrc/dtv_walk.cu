@@ -89,7 +89,9 @@ __global__ void __launch_bounds__(256) k_build_walk(const uint4* __restrict__ ce
         } else {
             ok &= bnd;
         }
-        links[4 * size_t(t) + k] = make_uint4((other < T ? other : kWalkNoTet) | (third << 28) | (alike ? 1u << 31 : 0u),
+        const bool flip = ft.x != t && !odd;
+        links[4 * size_t(t) + k] = make_uint4((other < T ? other : kWalkNoTet) | (third << 28) | (flip ? 1u << 30 : 0u) |
+                                                  (alike ? 1u << 31 : 0u),
                                               (f << 2) | (bnd ? 2u : 0u) | (odd ? 1u : 0u), next, map);
     }
     if (!ok) *bad = 1u;

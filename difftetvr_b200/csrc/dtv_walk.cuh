@@ -61,14 +61,16 @@ __device__ __forceinline__ WalkVert walk_vertex(uint32_t id, float qx, float qy,
 
 // False for a vertex that is not projected (sx is NaN there) or so far off
 // screen that its snapped position is not exact in FP32.
-__device__ __forceinline__ bool walk_usable(const WalkVert& v) {
+template <class V>
+__device__ __forceinline__ bool walk_usable(const V& v) {
     return (fabsf(v.sx) < kWalkGuardPx) & (fabsf(v.sy) < kWalkGuardPx);
 }
 
 // Whether the pixel centre is on the inner side of the directed edge a -> b
 // (edge_in on the exact value): the sign of the difference of products with
 // the product's rounding error added back (Kahan) is the exact one.
-__device__ __forceinline__ bool walk_side(const WalkVert& a, const WalkVert& b) {
+template <class V>
+__device__ __forceinline__ bool walk_side(const V& a, const V& b) {
     const float w = __fmul_rn(a.sy, b.sx);
     const float s = __fadd_rn(__fmaf_rn(a.sx, b.sy, -w), __fmaf_rn(-a.sy, b.sx, w));
     bool in = s > 0.f;
