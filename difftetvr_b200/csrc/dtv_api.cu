@@ -112,6 +112,12 @@ struct dtv_renderer {
     DevBuf<uint32_t> clipped;     // [0]: the projection met a vertex it does not project
     cudaEvent_t ev_info = nullptr;  // the record total is on the host
     DevBuf<uint32_t> redo;        // pixels the walk left to the rasteriser
+    // How many they were in the last walked render (pinned, one number per band
+    // up to kLeftSlots, written when its lists are done), and the renders left
+    // that do not walk (many_left).
+    volatile uint32_t* h_left = nullptr;
+    int left_n = 0;
+    int skip_walk = 0;
     dtv::ListInfo* h_info = nullptr;  // pinned
     // State of the last render.
     bool have_render = false;
@@ -127,6 +133,29 @@ struct dtv_renderer {
 };
 
 namespace {
+
+constexpr int kLeftSlots = 64;
+
+// Whether this render walks.
+bool take_walk(dtv_renderer* r, const dtv_mesh* mesh, uint64_t P) {
+    if (r->mesh != mesh) r->left_n = r->skip_walk = 0;
+    if (!mesh->walkable) return false;
+    uint64_t left = 0;
+    for (int i = 0; i < r->left_n; ++i) left += r->h_left[i];
+    if (r->left_n && !r->clipped_view && dtv::many_left(left, P)) {
+        r->left_n = 0;
+        r->skip_walk = dtv::kWalkRetry;
+    }
+    return r->skip_walk == 0 || r->skip_walk-- == 0;
+}
+
+// The number of pixels the walk left, to the host (slot: the band).
+void read_left(dtv_renderer* r, int slot, cudaStream_t s) {
+    if (slot >= kLeftSlots) return;
+    DTV_CK(cudaMemcpyAsync(const_cast<uint32_t*>(r->h_left) + slot, &r->info.ptr->n_redo, sizeof(uint32_t),
+                           cudaMemcpyDeviceToHost, s));
+    r->left_n = slot + 1;
+}
 
 dtv::WalkMesh walk_mesh(const dtv_mesh* m) {
     return dtv::WalkMesh{m->d_walk_links, m->d_walk_start, m->d_bfaces};
@@ -192,7 +221,7 @@ void rest_rows(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& cam, in
     const uint32_t F = uint32_t(mesh->host.num_faces);
     if (few) {
         dtv::launch_rest_fill(r->info.ptr, mesh->d_faces, F, r->vproj.ptr, r->vfix.ptr, cam.W, y0, y1, r->counts.ptr,
-                              r->offsets.ptr, r->records.ptr, s);
+                              r->offsets.ptr, r->records.ptr, r->redo.ptr, s);
         dtv::launch_rest_sort(r->info.ptr, true, r->redo.ptr, r->offsets.ptr, r->records.ptr, s);
     } else {
         dtv::launch_raster_fill(mesh->d_faces, F, r->vproj.ptr, r->vfix.ptr, cam.W, cam.H, r->counts.ptr,
@@ -225,13 +254,15 @@ void composite_rows(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors
 // offsets): scan of the band's counts, then the walk and what it leaves, or
 // fill (faces in the render's fill_order) and per-pixel sort.  The band's
 // counts must hold the rasterised counts; they end at zero.
-void build_band_lists(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& cam, int y0, int y1, cudaStream_t s) {
+void build_band_lists(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& cam, int band, cudaStream_t s) {
+    const int y0 = r->bands[size_t(band)].first, y1 = r->bands[size_t(band)].second;
     const int W = cam.W, H = cam.H;
     const uint64_t p0 = uint64_t(y0) * W, pb = uint64_t(y1 - y0) * W;
     dtv::launch_scan(r->counts.ptr + p0, pb, r->offsets.ptr + p0, r->scan_scratch.ptr, s, r->info.ptr);
     check_launch("band scan");
     if (r->band_walk) {
         walk_rows(r, mesh, cam, y0, y1, false, s);
+        read_left(r, band, s);
         rest_rows(r, mesh, cam, y0, y1, !r->clipped_view, s);
         return;
     }
@@ -317,8 +348,9 @@ void render_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors,
         throw;
     }
     rec_event(r, 3, s);
-    for (const auto& b : r->bands) {
-        build_band_lists(r, mesh, cam, b.first, b.second, s);
+    for (size_t k = 0; k < r->bands.size(); ++k) {
+        const auto& b = r->bands[k];
+        build_band_lists(r, mesh, cam, int(k), s);
         composite_rows(r, mesh, d_colors, cam, sh, d_image, b.first, b.second, s);
         check_launch("band composite");
     }
@@ -334,8 +366,9 @@ void adjoint_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors
                     const dtv::ShadeDev& sh, float* d_grad_positions, float* d_grad_colors, cudaStream_t s) {
     clear_rows(r, mesh, s);
     DTV_CK(cudaMemcpyAsync(r->counts.ptr, r->band_counts.ptr, sizeof(uint32_t) * r->P, cudaMemcpyDeviceToDevice, s));
-    for (const auto& b : r->bands) {
-        build_band_lists(r, mesh, r->cam, b.first, b.second, s);
+    for (size_t k = 0; k < r->bands.size(); ++k) {
+        const auto& b = r->bands[k];
+        build_band_lists(r, mesh, r->cam, int(k), s);
         adjoint_rows(r, mesh, d_colors, d_image_adjoint, sh, b.first, b.second, d_grad_colors, s);
         check_launch("band adjoint");
     }
@@ -507,6 +540,8 @@ int32_t dtv_renderer_create(int32_t type, dtv_renderer** out) {
         r->type = type;
         try {
             DTV_CK(cudaMallocHost(&r->h_info, sizeof(dtv::ListInfo)));
+            DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&r->h_left), sizeof(uint32_t) * kLeftSlots));
+            for (int i = 0; i < kLeftSlots; ++i) r->h_left[i] = 0u;
             for (auto& e : r->ev) DTV_CK(cudaEventCreate(&e));
             DTV_CK(cudaEventCreateWithFlags(&r->ev_info, cudaEventDisableTiming));
         } catch (...) {
@@ -543,6 +578,7 @@ int32_t dtv_renderer_destroy(dtv_renderer* r) {
     if (r->ev_info) cudaEventDestroy(r->ev_info);
     r->walk_verts.release();
     if (r->h_info) cudaFreeHost(r->h_info);
+    if (r->h_left) cudaFreeHost(const_cast<uint32_t*>(r->h_left));
     if (r->h_rowoff) cudaFreeHost(r->h_rowoff);
     for (auto& e : r->ev)
         if (e) cudaEventDestroy(e);
@@ -598,7 +634,7 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
 
         r->wide_list.ensure(size_t(F) + 1, s);
         rec_event(r, 0, s);
-        const bool walk = !raytet && mesh->walkable;
+        const bool walk = !raytet && take_walk(r, mesh, P);
         if (walk) {
             r->walk_verts.ensure(V ? V : 1, s);
             r->clipped.ensure(1, s, /*zero_new=*/true);
@@ -623,13 +659,28 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         check_launch("scan");
         DTV_CK(cudaMemcpyAsync(r->h_info, r->info.ptr, sizeof(dtv::ListInfo), cudaMemcpyDeviceToHost, s));
         DTV_CK(cudaEventRecord(r->ev_info, s));
-        // Lists by the walk (few left), then the composite; events of the
-        // fill, sort and composite stages.
+        // Faces in row-band order for the fill of whole lists.
+        auto order_faces = [&] {
+            r->fill_order.ensure(size_t(F), s);
+            r->band_scratch.ensure(2 * dtv::kFillBands, s);
+            dtv::launch_fill_order(rfaces, uint32_t(F), r->vfix.ptr, H, r->h_info->nf, r->fill_order.ptr, r->band_scratch.ptr, s);
+        };
+        // Lists by the walk, then the composite; events of the fill, sort and
+        // composite stages.  Few pixels are left, as far as the renders before
+        // tell; without one the host waits to know.
         auto lists_and_composite = [&](bool guarded) {
             rec_event(r, 3, s);
             walk_rows(r, mesh, cam, 0, H, guarded, s);
+            const bool known = guarded || r->left_n > 0;
+            read_left(r, 0, s);
+            bool few = true;
+            if (!known) {
+                DTV_CK(cudaStreamSynchronize(s));
+                few = r->h_info->clipped != 0u || !dtv::many_left(r->h_left[0], P);
+                if (!few) order_faces();
+            }
             rec_event(r, 4, s);
-            rest_rows(r, mesh, cam, 0, H, /*few=*/true, s);
+            rest_rows(r, mesh, cam, 0, H, few, s);
             rec_event(r, 5, s);
             composite_rows(r, mesh, d_colors, cam, sh, d_image, 0, H, s, &r->info.ptr->whole);
             check_launch("composite");
@@ -640,12 +691,6 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         const uint64_t nf = r->h_info->nf;
         const bool walked = early && r->h_info->ok != 0u, clipped = walk && r->h_info->clipped != 0u;
         r->clipped_view = clipped;
-        // Faces in row-band order for the fill of whole lists.
-        auto order_faces = [&] {
-            r->fill_order.ensure(size_t(F), s);
-            r->band_scratch.ensure(2 * dtv::kFillBands, s);
-            dtv::launch_fill_order(rfaces, uint32_t(F), r->vfix.ptr, H, nf, r->fill_order.ptr, r->band_scratch.ptr, s);
-        };
         r->bands.clear();
         if (budget && nf * sizeof(u64) > budget) {
             if (params->over_budget != DTV_OVER_BUDGET_RECOMPUTE || raytet) {

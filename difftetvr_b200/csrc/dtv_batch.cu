@@ -296,9 +296,20 @@ __global__ void __launch_bounds__(128) kb_rest_fill(const BatchView* __restrict_
                                                     const ListInfo* __restrict__ info,
                                                     const float4* __restrict__ vproj, const int2* __restrict__ vfix,
                                                     uint32_t* __restrict__ counts, const u64* __restrict__ offsets,
-                                                    u64* __restrict__ records) {
-    if (info->n_redo == 0u) return;
+                                                    u64* __restrict__ records, const uint32_t* __restrict__ redo) {
+    const uint32_t left = info->n_redo;
+    if (left == 0u) return;
     __shared__ RasterJob jobs[4][32];
+    __shared__ uint32_t mask[kRestMaskBits / 32];   // the views' 16 x 16 tiles
+    for (uint32_t i = threadIdx.x; i < kRestMaskBits / 32; i += blockDim.x) mask[i] = 0u;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < left; i += blockDim.x) {
+        const u64 g = redo[i];
+        const BatchView& bv = views[find_index(g, nviews, [&](int k) { return views[k].pix_base; })];
+        const uint32_t p = uint32_t(g - bv.pix_base), y = p / bv.W;
+        rest_mask_set(mask, uint32_t(bv.tile_base) + (y / kTile) * bv.tiles_x + (p - y * bv.W) / kTile);
+    }
+    __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const u64 stride = u64(gridDim.x) * blockDim.x;
     for (u64 base = u64(blockIdx.x) * blockDim.x + u64(w) * 32u; base < total; base += stride) {
@@ -309,7 +320,9 @@ __global__ void __launch_bounds__(128) kb_rest_fill(const BatchView* __restrict_
             const int v = find_index(g, nviews, [&](int k) { return views[k].face_base; });
             const BatchView& bv = views[v];
             live = raster_setup(uint32_t(g - bv.face_base), bv.faces, vfix + bv.vert_base, uint32_t(bv.vert_base),
-                                int(bv.W), 0, int(bv.H), bv.pix_base, J);
+                                int(bv.W), 0, int(bv.H), bv.pix_base, J) &&
+                   rest_mask_hit(mask, uint32_t(bv.tile_base), bv.tiles_x, J.px0 / kTile, (J.px0 + J.bw - 1) / kTile,
+                                 J.py0 / kTile, (J.py0 + J.bh - 1) / kTile);
         }
         const bool wide = live && J.wide != 0;
         if (live) jobs[w][lane] = J;
@@ -605,6 +618,8 @@ struct dtv_batch {
     // the next batch's left-over pixels take the passes for many pixels.  The
     // results do not depend on it.
     bool many_left = false;
+    volatile uint32_t* h_left = nullptr;  // pinned: pixels the last walk left
+    int skip_walk = 0;                    // calls left that do not walk (many_left)
     DevBuf<dtv::WalkVertRow> walk_verts;
     DevBuf<float4> grad_rows;
     DevBuf<uint32_t> fill_order;    // items (view faces) in row-band order for the fill
@@ -620,7 +635,7 @@ struct dtv_batch {
     // shapes of the last render (for the adjoint)
     int nviews = 0;
     u64 tot_verts = 0, tot_faces = 0, tot_bfaces = 0, tot_pixels = 0, tot_tiles = 0, tot_rows = 0;
-    bool walk = false;        // every view's mesh can be walked
+    bool walk = false;        // every view's mesh can be walked, and is
     uint32_t max_height = 0;  // tallest view (grid of the count's row prefix)
     dtv::ShadeDev sh{};
     bool have_render = false;
@@ -652,7 +667,11 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
     ensure_pinned(reinterpret_cast<void**>(&b->h_views), b->h_views_cap, sizeof(BatchView) * size_t(nviews));
     if (b->staging_free) DTV_CK(cudaEventSynchronize(b->staging_free));
     u64 vb = 0, fb = 0, bb = 0, pb = 0, tb = 0;
-    bool walk = true;
+    if (b->h_left && !b->many_left && dtv::many_left(*b->h_left, b->tot_pixels)) {
+        *b->h_left = 0u;
+        b->skip_walk = dtv::kWalkRetry;
+    }
+    bool walk = b->skip_walk == 0 || b->skip_walk-- == 0;
     for (int i = 0; i < nviews; ++i) {
         const dtv_batch_view& in = views[i];
         require(in.mesh >= 0 && in.mesh < int(b->meshes.size()), "view mesh index out of range");
@@ -752,6 +771,8 @@ void ensure_scratch(dtv_batch* b, cudaStream_t s) {
     b->loss.ensure(1, s);
     if (!b->h_info) {
         DTV_CK(cudaMallocHost(&b->h_info, sizeof(dtv::ListInfo)));
+        DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&b->h_left), sizeof(uint32_t)));
+        *b->h_left = 0u;
         DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
     }
 }
@@ -819,13 +840,15 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
         kb_walk_lists<<<unsigned(2 * b->tot_tiles), kTileThreads, 0, s>>>(
             b->d_views.ptr, b->nviews, b->offsets.ptr, b->records.ptr, b->counts.ptr, b->walk_verts.ptr, b->info.ptr,
             b->redo.ptr);
+        DTV_CK(cudaMemcpyAsync(const_cast<uint32_t*>(b->h_left), &b->info.ptr->n_redo, sizeof(uint32_t),
+                               cudaMemcpyDeviceToHost, s));
         if (b->many_left) {
             launch_kb_fill<true>(b, okp, s);
             launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, okp,
                         b->sort_surrogate_classes, b->sort_bucket_classes, b->redo.ptr, &b->info.ptr->n_redo);
         } else {
             kb_rest_fill<<<148 * 6, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->info.ptr, b->vproj.ptr,
-                                                 b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr);
+                                                 b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr, b->redo.ptr);
             launch_rest_sort(b->info.ptr, false, b->redo.ptr, b->offsets.ptr, b->records.ptr, s);
         }
     } else {
@@ -956,6 +979,8 @@ int32_t dtv_batch_reserve(dtv_batch* b, uint64_t max_views, uint64_t max_vertice
         b->loss.ensure(1, s);
         if (!b->h_info) {
             DTV_CK(cudaMallocHost(&b->h_info, sizeof(dtv::ListInfo)));
+        DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&b->h_left), sizeof(uint32_t)));
+        *b->h_left = 0u;
             DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
         }
         DTV_CK(cudaStreamSynchronize(s));
@@ -999,6 +1024,7 @@ int32_t dtv_batch_destroy(dtv_batch* b) {
     if (b->h_views) cudaFreeHost(b->h_views);
     if (b->h_slots) cudaFreeHost(b->h_slots);
     if (b->h_info) cudaFreeHost(b->h_info);
+    if (b->h_left) cudaFreeHost(const_cast<uint32_t*>(b->h_left));
     if (b->staging_free) cudaEventDestroy(b->staging_free);
     delete b;
     return DTV_OK;

@@ -84,7 +84,7 @@ struct ListInfo;
 // listed pixels' lists.
 void launch_rest_fill(const ListInfo* info, const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W,
                       int row0, int row1, uint32_t* counts, const unsigned long long* offsets,
-                      unsigned long long* records, cudaStream_t s);
+                      unsigned long long* records, const uint32_t* redo, cudaStream_t s);
 void launch_rest_sort(const ListInfo* info, bool few, const uint32_t* list, const unsigned long long* offsets,
                       unsigned long long* records, cudaStream_t s);
 // Order of the faces for the fill, grouped by row bands of about
@@ -218,6 +218,17 @@ void launch_walk_adjoint(const unsigned long long* b_offsets, const unsigned lon
                          float4* grad_col, cudaStream_t s);
 
 // Fragment lists by walking the mesh (dtv_walk.cu).
+// A mesh whose tets overlap (many inverted ones, as training without a
+// regularizer leaves them) closes loops of faces over many pixels.  Past one
+// pixel in kManyLeft the rasteriser's passes alone make the next kWalkRetry
+// renders' lists (the same lists); the number is read back without a wait,
+// after the lists.  Walk + rest against fill + sort (us), as training tangles the
+// mesh: 64^3 / 1024^2 with 840 pixels left 1,906 against 3,300, 5,461 left 2,400
+// against 3,340, 19,128 left 4,200 against 3,400; 32^3 / 512^2 with 800 left 540
+// against 550, 1,600 left 670 against 555 (the whole step 1.57 ms either way).
+constexpr uint64_t kManyLeft = 160;
+constexpr int kWalkRetry = 64;
+inline bool many_left(uint64_t left, uint64_t pixels) { return left > pixels / kManyLeft; }
 // Fills the tables (links: 4 T, start: one per boundary face) from the device
 // topology; *bad (device) is set to a non-zero value when the topology cannot
 // be walked (a tet with a vertex twice, a face of more than two tets).

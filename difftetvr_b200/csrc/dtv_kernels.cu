@@ -126,22 +126,38 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_listed(const uint4
 
 // Fill of the few pixels the walk left to the rasteriser (their counters hold
 // the list length, all others zero), 32 faces per warp and step over a fixed
-// grid; nothing is done unless few_left.
+// grid; nothing is done unless few_left.  Faces without such a pixel in the
+// tiles of their box (2^shift px square, the smallest that the mask holds) end
+// after their setup: 2,950 -> 290 us at 64^3 / 1024^2 with 170 pixels left, 530
+// with 840 (fill and sort).
 __global__ void __launch_bounds__(32 * kRasterWarps) k_rest_fill(const ListInfo* __restrict__ info,
                                                                  const uint4* __restrict__ faces, uint32_t F,
                                                                  const float4* __restrict__ vproj,
                                                                  const int2* __restrict__ vfix, int W, int row0,
                                                                  int row1, uint32_t* __restrict__ counts,
                                                                  const u64* __restrict__ offsets,
-                                                                 u64* __restrict__ records) {
-    if (!few_left(info)) return;
+                                                                 u64* __restrict__ records,
+                                                                 const uint32_t* __restrict__ redo, int shift) {
+    const uint32_t left = few_left(info);
+    if (!left) return;
     __shared__ RasterJob jobs[kRasterWarps][32];
+    __shared__ uint32_t mask[kRestMaskBits / 32];
+    const uint32_t pitch = (uint32_t(W) >> shift) + 1u;
+    for (uint32_t i = threadIdx.x; i < kRestMaskBits / 32; i += blockDim.x) mask[i] = 0u;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < left; i += blockDim.x) {
+        const uint32_t p = redo[i], y = p / uint32_t(W);
+        rest_mask_set(mask, ((y - uint32_t(row0)) >> shift) * pitch + ((p - y * uint32_t(W)) >> shift));
+    }
+    __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x + uint32_t(w) * 32u; base < F; base += stride) {
         const uint32_t i = base + uint32_t(lane);
         RasterJob J;
-        const bool live = i < F && raster_setup(i, faces, vfix, 0u, W, row0, row1, 0ull, J);
+        const bool live = i < F && raster_setup(i, faces, vfix, 0u, W, row0, row1, 0ull, J) &&
+                          rest_mask_hit(mask, 0u, pitch, J.px0 >> shift, (J.px0 + J.bw - 1) >> shift,
+                                        (J.py0 - row0) >> shift, (J.py0 + J.bh - 1 - row0) >> shift);
         const bool wide = live && J.wide != 0;
         if (live) jobs[w][lane] = J;
         raster_warp<true, false, true>(jobs[w], __ballot_sync(kFull, live && !wide), lane, vproj, counts, offsets,
@@ -187,9 +203,13 @@ void launch_boundary_fill(const uint4* faces, uint32_t F, const float4* vproj, c
 }
 
 void launch_rest_fill(const ListInfo* info, const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W,
-                      int row0, int row1, uint32_t* counts, const u64* offsets, u64* records, cudaStream_t s) {
-    if (F) k_rest_fill<<<148 * 6, 32 * kRasterWarps, 0, s>>>(info, faces, F, vproj, vfix, W, row0, row1, counts,
-                                                            offsets, records);
+                      int row0, int row1, uint32_t* counts, const u64* offsets, u64* records, const uint32_t* redo,
+                      cudaStream_t s) {
+    if (F == 0 || row1 <= row0) return;
+    int shift = 2;
+    while (((uint64_t(W) >> shift) + 1) * ((uint64_t(row1 - row0) >> shift) + 1) > kRestMaskBits) ++shift;
+    k_rest_fill<<<148 * 6, 32 * kRasterWarps, 0, s>>>(info, faces, F, vproj, vfix, W, row0, row1, counts, offsets,
+                                                      records, redo, shift);
 }
 
 constexpr unsigned kListedBlocks = 148, kListedCountBlocks = 148 * 8;

@@ -336,6 +336,32 @@ __device__ __forceinline__ void raster_warp(const RasterJob* jobs, uint32_t live
 // vertices many pixels' chains are cut: the launches for many pixels follow.
 __device__ __forceinline__ uint32_t few_left(const ListInfo* info) { return info->clipped ? 0u : info->n_redo; }
 
+// Tiles with a pixel left to the rasteriser, one bit each, in a block's shared
+// memory: the rest fills pass over all faces for a few pixels (those that closed
+// loops of faces around inverted tets cover), and a face whose box has none of
+// them ends after its setup.  Bits wrap around (bit_of modulo the mask's size),
+// which only keeps more faces.
+constexpr uint32_t kRestMaskBits = 1u << 16;
+constexpr int kRestTestTiles = 64;   // boxes over more tiles are not tested
+
+__device__ __forceinline__ void rest_mask_set(uint32_t* mask, uint32_t bit) {
+    bit &= kRestMaskBits - 1u;
+    atomicOr(mask + (bit >> 5), 1u << (bit & 31u));
+}
+
+// Whether the tiles (x0..x1) x (y0..y1) of rows `pitch` tiles long from bit
+// `base` have a pixel left.
+__device__ __forceinline__ bool rest_mask_hit(const uint32_t* mask, uint32_t base, uint32_t pitch, int x0, int x1,
+                                              int y0, int y1) {
+    if ((x1 - x0 + 1) * (y1 - y0 + 1) > kRestTestTiles) return true;
+    for (int y = y0; y <= y1; ++y)
+        for (int x = x0; x <= x1; ++x) {
+            const uint32_t bit = (base + uint32_t(y) * pitch + uint32_t(x)) & (kRestMaskBits - 1u);
+            if ((mask[bit >> 5] >> (bit & 31u)) & 1u) return true;
+        }
+    return false;
+}
+
 // ---------------------------------------------------------------------------
 // Fragment evaluation shared by composite and adjoint.
 struct FragV {
