@@ -671,7 +671,7 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         auto lists_and_composite = [&](bool guarded) {
             rec_event(r, 3, s);
             walk_rows(r, mesh, cam, 0, H, guarded, s);
-            const bool known = guarded || r->left_n > 0;
+            const bool known = r->left_n > 0;
             read_left(r, 0, s);
             bool few = true;
             if (!known) {
@@ -685,7 +685,7 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
             composite_rows(r, mesh, d_colors, cam, sh, d_image, 0, H, s, &r->info.ptr->whole);
             check_launch("composite");
         };
-        const bool early = walk && r->records.ptr;
+        const bool early = walk && r->records.ptr && r->left_n > 0;
         if (early) lists_and_composite(true);
         DTV_CK(cudaEventSynchronize(r->ev_info));
         const uint64_t nf = r->h_info->nf;
