@@ -398,12 +398,15 @@ __global__ void __launch_bounds__(kTileThreads) kb_walk_lists(
 }
 
 // Fused L2 loss of every view with a target: dimage = 2 s (image - target),
-// loss += s * sum (image - target)^2 with s = 1 / (4 W H).
-__global__ void __launch_bounds__(256) kb_loss(const BatchView* __restrict__ views, int nviews, u64 total_pixels,
+// loss += s * sum (image - target)^2 with s = 1 / (4 W H).  Two blocks of 512 per
+// SM and carried rounding errors, as k_loss_l2: with 1,184 blocks' additions the
+// loss's rounding reached 1.2e-6, relative.
+constexpr int kLossThreads = 512;
+__global__ void __launch_bounds__(kLossThreads) kb_loss(const BatchView* __restrict__ views, int nviews, u64 total_pixels,
                                                float* __restrict__ loss, const uint32_t* __restrict__ ok) {
     if (!batch_ok(ok)) return;
-    __shared__ float sm[8];
-    float acc = 0.f;
+    __shared__ float sm[kLossThreads / 32];
+    float acc = 0.f, err = 0.f;
     for (u64 g = u64(blockIdx.x) * blockDim.x + threadIdx.x; g < total_pixels; g += u64(gridDim.x) * blockDim.x) {
         const int v = find_index(g, nviews, [&](int i) { return views[i].pix_base; });
         const BatchView& bv = views[v];
@@ -413,8 +416,11 @@ __global__ void __launch_bounds__(256) kb_loss(const BatchView* __restrict__ vie
         const float4 d = make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w);
         const float s2 = 2.f * bv.loss_scale;
         bv.dimage[p] = make_float4(s2 * d.x, s2 * d.y, s2 * d.z, s2 * d.w);
-        acc += bv.loss_scale * (d.x * d.x + d.y * d.y + d.z * d.z + d.w * d.w);
+        const F2 t = two_sum(acc, bv.loss_scale * ((d.x * d.x + d.y * d.y) + (d.z * d.z + d.w * d.w)));
+        acc = t.hi;
+        err += t.lo;
     }
+    acc += err;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
@@ -1217,8 +1223,8 @@ void enqueue_train_body(dtv_batch* b, const dtv::AdamConst& ac, int nslots, cuda
     enqueue_forward(b, b->sh, s);
     const uint32_t* okp = &b->info.ptr->ok;
     DTV_CK(cudaMemsetAsync(b->loss.ptr, 0, sizeof(float), s));
-    kb_loss<<<grid_for(b->tot_pixels, 256, 148 * 8), 256, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_pixels,
-                                                                  b->loss.ptr, okp);
+    kb_loss<<<grid_for(b->tot_pixels, kLossThreads, 148 * 2), kLossThreads, 0, s>>>(b->d_views.ptr, b->nviews,
+                                                                                    b->tot_pixels, b->loss.ptr, okp);
     DTV_CK(cudaMemsetAsync(b->grad_rows.ptr, 0, sizeof(float4) * 2 * size_t(b->tot_rows), s));
     enqueue_adjoint(b, b->sh, okp, s);
     kb_adam_rows<<<grid_for(b->tot_rows, 256, 148 * 16), 256, 0, s>>>(b->d_slots.ptr, nslots, b->tot_rows,
