@@ -643,6 +643,7 @@ struct dtv_batch {
     u64 tot_verts = 0, tot_faces = 0, tot_bfaces = 0, tot_pixels = 0, tot_tiles = 0, tot_rows = 0;
     bool walk = false;        // every view's mesh can be walked, and is
     uint32_t max_height = 0;  // tallest view (grid of the count's row prefix)
+    bool crowded = false;     // a view has many pixels per vertex (view_copies)
     dtv::ShadeDev sh{};
     bool have_render = false;
     u64 last_fragments = 0;
@@ -729,24 +730,31 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
     b->tot_pixels = pb;
     b->tot_tiles = tb;
     uint32_t mh = 0;
-    for (int i = 0; i < nviews; ++i) mh = std::max(mh, b->h_views[i].H);
+    b->crowded = false;
+    for (int i = 0; i < nviews; ++i) {
+        const BatchView& bv = b->h_views[i];
+        mh = std::max(mh, bv.H);
+        b->crowded |= u64(bv.W) * bv.H > 8 * dtv::kGradRowPixels * bv.V;
+    }
     b->max_height = mh;
 }
 
-// Copies of the views' gradient rows (grad_copies on the mean view), together
-// at most kBatchGradRows rows (64 MiB) beyond the first copy: a batch of many
-// views spreads its atomics over their rows already, and a reserved batch
-// holds the copies from the start.
+// Copies of the views' gradient rows (grad_copies on the mean view; one where
+// a view has over eight times the mean's limit of pixels per vertex, 128: sums
+// move by up to 2e-6 there), together at most kBatchGradRows rows (64 MiB)
+// beyond the first copy: a batch of many views spreads its atomics over their
+// rows already, and a reserved batch holds the copies from the start.
 constexpr u64 kBatchGradRows = 1u << 21;
 uint32_t view_copies(const dtv_batch* b) {
+    if (b->crowded) return 1;
     const u64 n = b->nviews > 0 ? u64(b->nviews) : 1;
     uint32_t c = dtv::grad_copies((b->tot_verts + n - 1) / n, b->tot_pixels / n);
     while (c > 1 && c * b->tot_verts > kBatchGradRows) c /= 2;
     return c;
 }
 
-// Most rows that view_copies gives a batch of up to nv views, V vertices and P
-// pixels.
+// Bound on the rows that view_copies gives a batch of up to nv views, V
+// vertices and P pixels.
 u64 most_view_rows(u64 nv, u64 V, u64 P) {
     const u64 per_view = nv <= kBatchGradRows / dtv::kGradRows ? nv * dtv::kGradRows : kBatchGradRows;
     const u64 by_pixels = std::min<u64>(P / dtv::kGradCopyPixels, 64);
@@ -1240,7 +1248,8 @@ std::vector<u64> train_signature(const dtv_batch* b, const dtv::AdamConst& ac, i
                             u64(uintptr_t(b->dimage_internal.ptr)), u64(uintptr_t(b->grad_rows.ptr)),
                             u64(uintptr_t(b->view_rows.ptr)), u64(uintptr_t(b->wide_list.ptr)),
                             u64(uintptr_t(b->counts.ptr)), u64(uintptr_t(b->walk_verts.ptr)),
-                            u64(uintptr_t(b->redo.ptr)), b->tot_bfaces, u64(b->walk), u64(b->many_left)};
+                            u64(uintptr_t(b->redo.ptr)), b->tot_bfaces, u64(b->walk), u64(b->many_left),
+                            u64(view_copies(b))};
     const uint32_t* shw = reinterpret_cast<const uint32_t*>(&b->sh);
     for (size_t i = 0; i < sizeof(b->sh) / 4; ++i) sig.push_back(shw[i]);
     const uint32_t* acw = reinterpret_cast<const uint32_t*>(&ac);

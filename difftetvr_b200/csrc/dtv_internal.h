@@ -151,15 +151,21 @@ void launch_composite(const unsigned long long* offsets, const unsigned long lon
 // Copies of the gradient rows of a mesh with few vertices (or cells): all
 // pixels' atomics on a few thousand rows wait for one another in L2, so the
 // blocks are spread over a power of two of copies with up to kGradRows rows in
-// all, which the scatter sums.  Measured (adjoint, us, one copy -> copies):
-// 8^3 at 800^2 1,326 -> 337, 16^3 at 1000^2 1,890 -> 969, 32^3 at 700^2 992 ->
-// 954, per-cell 10^3 at 600^2 440 -> 207; 2^15, 2^16 and 2^18 rows gave 1,117,
-// 983 and 975 at 16^3.  One copy per 8192 pixels at most: a small image has no
-// contention to spread, and clearing and summing 64 copies cost 12 us.
+// all, which the scatter sums.  One copy per 8192 pixels at most: a small image
+// has no contention to spread, and clearing and summing 64 copies cost 12 us.
+// Past kGradRowPixels pixels per row there is one copy: a row then gets so many
+// terms that the rounding of its one long FP32 sum (relative to the gradient's
+// norm 2e-6 at 200 pixels per vertex, 1.5e-5 to 2.9e-5 at 3,200) shows, and
+// splitting it would move the values by that much; at 16 it moves them by less
+// than another order of the atomics does (1e-6, 2e-6 at attenuation 100).
+// Measured (us per step, one copy -> copies): 16^3 at 256^2 338 -> 321, a
+// training step over 12 views of 12^3 to 36^3 at 384^2 4,308 -> 3,949.
 constexpr uint64_t kGradRows = 1u << 17;
 constexpr uint64_t kGradCopyPixels = 8192;
+constexpr uint64_t kGradRowPixels = 16;
 inline uint32_t grad_copies(uint64_t rows, uint64_t pixels) {
     uint32_t c = 1;
+    if (pixels > kGradRowPixels * rows) return c;
     while (c < 64 && 2 * uint64_t(c) * rows <= kGradRows && 2 * uint64_t(c) * kGradCopyPixels <= pixels) c *= 2;
     return c;
 }
