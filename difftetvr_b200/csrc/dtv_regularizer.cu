@@ -108,6 +108,23 @@ __global__ void __launch_bounds__(256) k_tet_regularizer(const uint4* __restrict
         // Slots whose vertex this tet holds take its gradient; the others are
         // written out and given to the tet's vertices without one.
         uint32_t fresh = 15u;
+        // A corner at an earlier corner's vertex (a tet may hold one twice) adds
+        // to that corner: no two slots ever have one id, so every vertex of a
+        // tet finds a slot.
+        if ((vi[1] == vi[0]) | (vi[2] == vi[0]) | (vi[3] == vi[0]) | (vi[2] == vi[1]) | (vi[3] == vi[1]) |
+            (vi[3] == vi[2])) {
+#pragma unroll
+            for (int j = 1; j < 4; ++j) {
+#pragma unroll
+                for (int i = 0; i < j; ++i) {
+                    if (((fresh >> j) & 1u) && vi[i] == vi[j]) {
+                        g[i] = make_float3(g[i].x + g[j].x, g[i].y + g[j].y, g[i].z + g[j].z);
+                        g[j] = make_float3(0.f, 0.f, 0.f);
+                        fresh &= ~(1u << j);
+                    }
+                }
+            }
+        }
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
             bool keep = false;

@@ -47,3 +47,25 @@ def test_gradient_and_loss(n, order):
         loss = reg.compute_grad_into(g)
         assert rel_err(g.cpu().numpy(), g_ref) < 1e-5
         assert abs(float(loss) - l_ref) < 1e-5 * abs(l_ref)
+
+
+@pytest.mark.parametrize("n", [38, 55])   # runs of 2 and of 6 tets
+@pytest.mark.parametrize("pair", [(0, 1), (0, 2), (0, 3), (1, 2), (1, 3), (2, 3)])
+def test_repeated_vertices_anywhere_in_a_run(n, pair):
+    """Tets with the same vertex at two corners, at every position of a run and
+    followed by the grid's tets, which share the vertex and bring new ones; the
+    sums of test_gradient_and_loss, so its bound."""
+    import difftetvr_b200 as d
+    from difftetvr_b200 import synthetic as S
+    from difftetvr_b200.regularizer import TetRegularizer
+    cells, pos = S.kuhn_mesh(n, seed=n, lo=0.0, hi=float(n))
+    for k in range(6):
+        cells[6 * k + k::90, pair[1]] = cells[6 * k + k::90, pair[0]]
+    mesh = d.TetMesh()
+    mesh.set_use_gradients(True)
+    mesh.set_tet_mesh_data(cells, pos, S.gaussian_colors(pos, seed=1))
+    g_ref, l_ref = reference(cells, pos, np.float64(np.float32(0.1)), 2.0)
+    g = torch.zeros(pos.shape, device="cuda")
+    loss = TetRegularizer(mesh, 0.1, 2.0).compute_grad_into(g)
+    assert rel_err(g.cpu().numpy(), g_ref) < 1e-5
+    assert abs(float(loss) - l_ref) < 1e-5 * abs(l_ref)
