@@ -1241,15 +1241,19 @@ void enqueue_train_body(dtv_batch* b, const dtv::AdamConst& ac, int nslots, cuda
     check_launch("batch train step");
 }
 
+// What a captured step depends on beside the tables it reads: sizes, launch
+// choices and every device buffer its kernels are given (a render in between
+// may have grown any of them).
 std::vector<u64> train_signature(const dtv_batch* b, const dtv::AdamConst& ac, int nslots) {
-    std::vector<u64> sig = {u64(b->nviews), b->tot_verts, b->tot_faces, b->tot_pixels, b->tot_tiles, b->tot_rows,
-                            u64(b->max_height),
-                            b->capacity, u64(nslots), u64(uintptr_t(b->records.ptr)),
-                            u64(uintptr_t(b->dimage_internal.ptr)), u64(uintptr_t(b->grad_rows.ptr)),
-                            u64(uintptr_t(b->view_rows.ptr)), u64(uintptr_t(b->wide_list.ptr)),
-                            u64(uintptr_t(b->counts.ptr)), u64(uintptr_t(b->walk_verts.ptr)),
-                            u64(uintptr_t(b->redo.ptr)), b->tot_bfaces, u64(b->walk), u64(b->many_left),
-                            u64(view_copies(b))};
+    std::vector<u64> sig = {u64(b->nviews), b->tot_verts, b->tot_faces, b->tot_bfaces, b->tot_pixels, b->tot_tiles,
+                            b->tot_rows, u64(b->max_height), b->capacity, u64(nslots), u64(b->walk),
+                            u64(b->many_left), u64(view_copies(b))};
+    const void* buffers[] = {b->d_views.ptr, b->d_slots.ptr, b->vproj.ptr, b->vfix.ptr, b->vgeo.ptr, b->counts.ptr,
+                             b->offsets.ptr, b->records.ptr, b->scan.ptr, b->tfinal.ptr, b->term.ptr,
+                             b->long_list.ptr, b->info.ptr, b->redo.ptr, b->clipped.ptr, b->walk_verts.ptr,
+                             b->grad_rows.ptr, b->fill_order.ptr, b->band_scratch.ptr, b->wide_list.ptr,
+                             b->view_rows.ptr, b->dimage_internal.ptr, b->loss.ptr, b->step.ptr};
+    for (const void* p : buffers) sig.push_back(u64(reinterpret_cast<uintptr_t>(p)));
     const uint32_t* shw = reinterpret_cast<const uint32_t*>(&b->sh);
     for (size_t i = 0; i < sizeof(b->sh) / 4; ++i) sig.push_back(shw[i]);
     const uint32_t* acw = reinterpret_cast<const uint32_t*>(&ac);

@@ -163,3 +163,43 @@ def test_batch_graph_overflow_reruns_step_exactly():
         res.append((m.get_vertex_colors().detach().cpu().numpy(), br.info()))
     assert res[0][1]["steps_rerun"] >= 1
     assert np.abs(res[0][0] - res[1][0]).max() < 1e-6
+
+
+@pytest.mark.parametrize("between", ["many views", "unconnected", "large"])
+def test_captured_step_after_renders_that_grow_buffers(between):
+    """A render between two captured steps grows some of the buffers the step
+    was captured with (the view table alone; the vertices' buffers but not the
+    faces'; the pixels' and records'): the next steps equal uncaptured ones
+    within the order of the atomics (bounds of the plain loop's test)."""
+    train = views_for([0, 0], [(192, 160), (96, 128)])
+    _targets({0: 10}, train)
+    res = []
+    for graph in (True, False):
+        m = make_mesh(10, 1)
+        meshes = [m, make_mesh(2, 3)]
+        if between == "unconnected":
+            cells, pos = S.kuhn_mesh(7, seed=2)
+            soup = d.TetMesh()
+            soup.set_use_gradients(True)
+            p = pos[cells.astype(np.int64)].reshape(-1, 3)
+            soup.set_tet_mesh_data(np.arange(len(p), dtype=np.uint32).reshape(-1, 4), p, S.gaussian_colors(p, seed=2))
+            assert len(p) > 2 * 11 ** 3
+            meshes[1] = soup
+        br = BatchRenderer(meshes, attenuation=1.0)
+        br.set_graph(graph)
+        losses = []
+        for _ in range(3):
+            losses.append(float(br.train_step(train)))
+        if between == "many views":
+            br.render(views_for([1] * 40, [(16, 16)] * 40))
+        elif between == "unconnected":
+            br.render(views_for([1], [(24, 24)]))
+        else:
+            br.render(views_for([0, 0, 0], [(300, 300)] * 3))
+        for _ in range(3):
+            losses.append(float(br.train_step(train)))
+        res.append((m.get_vertex_colors().detach().cpu().numpy(), m.get_vertex_positions().detach().cpu().numpy(), losses,
+                    br.info()))
+    assert res[0][3]["graph"] and not res[1][3]["graph"]
+    assert rel_err(res[0][0], res[1][0]) < 1e-5 and rel_err(res[0][1], res[1][1]) < 1e-6
+    assert np.allclose(res[0][2], res[1][2], rtol=1e-5, atol=0.0)
