@@ -761,6 +761,17 @@ u64 most_view_rows(u64 nv, u64 V, u64 P) {
     return std::max(V, std::min(per_view, by_pixels * std::min(V, kBatchGradRows)));
 }
 
+// Pinned words and the staging event, each by itself: a call that failed half
+// way leaves what it got, and the next one makes the rest.
+void ensure_host(dtv_batch* b) {
+    if (!b->h_info) DTV_CK(cudaMallocHost(&b->h_info, sizeof(dtv::ListInfo)));
+    if (!b->h_left) {
+        DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&b->h_left), sizeof(uint32_t)));
+        *b->h_left = 0u;
+    }
+    if (!b->staging_free) DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
+}
+
 void ensure_scratch(dtv_batch* b, cudaStream_t s) {
     b->d_views.ensure(size_t(b->nviews), s);
     b->vproj.ensure(b->tot_verts ? b->tot_verts : 1, s);
@@ -783,12 +794,7 @@ void ensure_scratch(dtv_batch* b, cudaStream_t s) {
         b->redo.ensure(b->tot_pixels, s);
     }
     b->loss.ensure(1, s);
-    if (!b->h_info) {
-        DTV_CK(cudaMallocHost(&b->h_info, sizeof(dtv::ListInfo)));
-        DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&b->h_left), sizeof(uint32_t)));
-        *b->h_left = 0u;
-        DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
-    }
+    ensure_host(b);
 }
 
 void upload_views(dtv_batch* b, cudaStream_t s) {
@@ -991,12 +997,7 @@ int32_t dtv_batch_reserve(dtv_batch* b, uint64_t max_views, uint64_t max_vertice
         b->walk_verts.ensure(V, s);
         b->redo.ensure(P, s);
         b->loss.ensure(1, s);
-        if (!b->h_info) {
-            DTV_CK(cudaMallocHost(&b->h_info, sizeof(dtv::ListInfo)));
-        DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&b->h_left), sizeof(uint32_t)));
-        *b->h_left = 0u;
-            DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
-        }
+        ensure_host(b);
         DTV_CK(cudaStreamSynchronize(s));
     });
 }
