@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kLossThreads) kb_loss(const BatchView* __restr
         acc = t.hi;
         err += t.lo;
     }
-    acc += err;
+    if (isfinite(acc)) acc += err;  // an infinite sum has no rounding error (two_sum gives NaN)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;

@@ -1430,7 +1430,7 @@ __global__ void __launch_bounds__(512) k_loss_l2(const float* __restrict__ img, 
         if (adj) adj[i] = 2.f * scale * d;
         add(d * d);
     }
-    acc += err;
+    if (isfinite(acc)) acc += err;  // an infinite sum has no rounding error (two_sum gives NaN)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;

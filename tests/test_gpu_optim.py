@@ -64,3 +64,27 @@ def test_adam_fixed_mask_modes():
         assert torch.all(q[~fixed] < 1.0)
         if mode == 2:
             assert torch.all(m[fixed] == 0)
+
+
+@pytest.mark.parametrize("n", [4096, 4099])   # four at a time, with a remainder
+@pytest.mark.parametrize("value,want", [(3e19, float("inf")), (float("inf"), float("inf")), (float("nan"), float("nan"))])
+def test_loss_of_values_beyond_fp32(n, value, want):
+    """A square that overflows, an infinity and a NaN give what FP32 sums give."""
+    from difftetvr_b200.optim import l2_loss
+    x = torch.zeros(n, device="cuda")
+    x[n // 3] = value
+    loss = float(l2_loss(x, torch.zeros_like(x)))
+    assert (np.isnan(want) and np.isnan(loss)) or loss == want
+
+
+@pytest.mark.parametrize("value,want", [(3e19, float("inf")), (float("inf"), float("inf")), (float("nan"), float("nan"))])
+def test_batch_loss_of_values_beyond_fp32(value, want):
+    from difftetvr_b200.batch import BatchRenderer, View
+    from helpers import Scene
+    sc = Scene(3, 48)
+    mesh, _ = sc.make_renderer()
+    target = torch.zeros((48, 48, 4), device="cuda")
+    target[7, 5, 1] = value
+    br = BatchRenderer([mesh])
+    loss = float(br.train_step([View(mesh=0, view_matrix=sc.view, width=48, height=48, fovy=sc.fovy, target=target)]))
+    assert (np.isnan(want) and np.isnan(loss)) or loss == want
