@@ -170,10 +170,9 @@ __global__ void __launch_bounds__(256) kb_band_scatter(const BatchView* __restri
     if (g < total) order[base[band] + rank] = uint32_t(g);
 }
 
-// Count or fill of every view's faces.  REST: the fill of the pixels the walk
-// left to the rasteriser (see fill_pixels).  `ok`: the fill does nothing when
-// *ok is zero.  threads_per_face: of the count (k_raster).
-template <bool FILL, bool WIDE, bool REST = false>
+// Count or fill of every view's faces.  `ok`: the fill does nothing when *ok is
+// zero.  threads_per_face: of the count (k_raster).
+template <bool FILL, bool WIDE>
 __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ views, int nviews, u64 total,
                                                  const float4* __restrict__ vproj, const int2* __restrict__ vfix,
                                                  uint32_t* __restrict__ counts, const u64* __restrict__ offsets,
@@ -217,14 +216,13 @@ __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ v
         __shared__ RasterJob jobs[4][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         if (live) jobs[w][lane] = J;
-        raster_warp<FILL, WIDE, REST>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets,
-                                      records);
+        raster_warp<FILL, WIDE>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets, records);
     }
 }
 
 // The 64-bit items listed by the count (wide_list) over a fixed grid: the count
 // (one item per warp) or the fill (32 per warp and step, raster_warp).
-template <bool FILL, bool REST = false>
+template <bool FILL>
 __global__ void __launch_bounds__(128) kb_raster_listed(const BatchView* __restrict__ views, int nviews,
                                                         const float4* __restrict__ vproj,
                                                         const int2* __restrict__ vfix,
@@ -256,8 +254,8 @@ __global__ void __launch_bounds__(128) kb_raster_listed(const BatchView* __restr
             RasterJob J;
             const bool live = i < n && setup(i, J);
             if (live) jobs[w][lane] = J;
-            raster_warp<FILL, true, REST>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets,
-                                          records);
+            raster_warp<FILL, true>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets,
+                                    records);
             __syncwarp();  // every lane is done with this step's jobs before the next step writes them
         }
     }
@@ -620,10 +618,12 @@ struct dtv_batch {
     DevBuf<dtv::ListInfo> info;     // record total, whether it fits, pixels the walk left
     DevBuf<uint32_t> redo;          // those pixels
     DevBuf<uint32_t> clipped;       // [0]: the projection met a vertex it does not project
-    // The last batch had clipped vertices: they cut many pixels' chains, so
-    // the next batch's left-over pixels take the passes for many pixels.  The
-    // results do not depend on it.
-    bool many_left = false;
+    // The last batch had clipped vertices, and the calls left that, enqueued
+    // before that is known of their own views, do not walk (render_common: a
+    // clipped view is not walked; a walked one is right all the same, its many
+    // left-over pixels are slow).
+    bool clipped_views = false;
+    int skip_clipped = 0;
     volatile uint32_t* h_left = nullptr;  // pinned: pixels the last walk left
     int skip_walk = 0;                    // calls left that do not walk (many_left)
     DevBuf<dtv::WalkVertRow> walk_verts;
@@ -668,17 +668,28 @@ void ensure_pinned(void** p, size_t& cap, size_t bytes) {
     cap = bytes;
 }
 
-// Builds the descriptor table for `views`; returns the totals.
-void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool train, bool internal_dimage) {
+// What the scan of a finished batch found (h_info).
+void note_clipped(dtv_batch* b) {
+    b->clipped_views = b->h_info->clipped != 0u;
+    if (b->clipped_views) b->skip_clipped = dtv::kWalkRetry;
+}
+
+// Builds the descriptor table for `views`; returns the totals.  ahead: the
+// lists are enqueued before the host knows the scan's findings.
+void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool train, bool ahead) {
     require(nviews > 0, "need at least one view");
     ensure_pinned(reinterpret_cast<void**>(&b->h_views), b->h_views_cap, sizeof(BatchView) * size_t(nviews));
     if (b->staging_free) DTV_CK(cudaEventSynchronize(b->staging_free));
     u64 vb = 0, fb = 0, bb = 0, pb = 0, tb = 0;
-    if (b->h_left && !b->many_left && dtv::many_left(*b->h_left, b->tot_pixels)) {
+    if (b->h_left && !b->clipped_views && dtv::many_left(*b->h_left, b->tot_pixels)) {
         *b->h_left = 0u;
         b->skip_walk = dtv::kWalkRetry;
     }
     bool walk = b->skip_walk == 0 || b->skip_walk-- == 0;
+    if (ahead && b->skip_clipped > 0) {
+        --b->skip_clipped;
+        walk = false;
+    }
     for (int i = 0; i < nviews; ++i) {
         const dtv_batch_view& in = views[i];
         require(in.mesh >= 0 && in.mesh < int(b->meshes.size()), "view mesh index out of range");
@@ -719,7 +730,6 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
         tb += u64(bv.tiles_x) * u64((c.height + dtv::kTile - 1) / dtv::kTile);
         b->h_views[i] = bv;
     }
-    (void)internal_dimage;
     require(vb < (u64(1) << 32), "a batch holds fewer than 2^32 vertices in total");
     require(fb < (u64(1) << 32), "a batch holds fewer than 2^32 faces in total");
     b->nviews = nviews;
@@ -819,9 +829,7 @@ void launch_kb_count(dtv_batch* b, cudaStream_t s) {
     kb_row_prefix<<<grid, 256, 0, s>>>(b->d_views.ptr, b->counts.ptr);
 }
 
-// Fill pass over every view's faces in row-band order (REST: of the pixels the
-// walk left).
-template <bool REST>
+// Fill pass over every view's faces in row-band order.
 void launch_kb_fill(dtv_batch* b, const uint32_t* okp, cudaStream_t s) {
     using namespace dtv;
     const unsigned blocks = grid_for(b->tot_faces, 128, 0x7fffffffu);
@@ -836,10 +844,10 @@ void launch_kb_fill(dtv_batch* b, const uint32_t* okp, cudaStream_t s) {
                                            b->tot_pixels, b->band_scratch.ptr + kFillBands, b->fill_order.ptr);
         order = b->fill_order.ptr;
     }
-    kb_raster<true, false, REST><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr,
+    kb_raster<true, false><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr,
                                                   b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr, okp, order, nullptr,
                                                   1u);
-    kb_raster_listed<true, REST><<<148, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
+    kb_raster_listed<true><<<148, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
                                                b->offsets.ptr, b->records.ptr, okp, b->wide_list.ptr);
 }
 
@@ -862,17 +870,11 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
             b->redo.ptr);
         DTV_CK(cudaMemcpyAsync(const_cast<uint32_t*>(b->h_left), &b->info.ptr->n_redo, sizeof(uint32_t),
                                cudaMemcpyDeviceToHost, s));
-        if (b->many_left) {
-            launch_kb_fill<true>(b, okp, s);
-            launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, okp,
-                        b->sort_surrogate_classes, b->sort_bucket_classes, b->redo.ptr, &b->info.ptr->n_redo);
-        } else {
-            kb_rest_fill<<<148 * 6, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->info.ptr, b->vproj.ptr,
-                                                 b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr, b->redo.ptr);
-            launch_rest_sort(b->info.ptr, false, b->redo.ptr, b->offsets.ptr, b->records.ptr, s);
-        }
+        kb_rest_fill<<<148 * 6, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->info.ptr, b->vproj.ptr,
+                                             b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr, b->redo.ptr);
+        launch_rest_sort(b->info.ptr, b->redo.ptr, b->offsets.ptr, b->records.ptr, s);
     } else {
-        launch_kb_fill<false>(b, okp, s);
+        launch_kb_fill(b, okp, s);
         launch_sort(b->offsets.ptr, b->records.ptr, uint32_t(b->tot_pixels), b->long_list.ptr, s, okp,
                     b->sort_surrogate_classes, b->sort_bucket_classes);
     }
@@ -1099,7 +1101,7 @@ int32_t dtv_batch_render(dtv_batch* b, int32_t num_views, const dtv_batch_view* 
         require(b && views && params, "null argument");
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         b->have_render = false;
-        build_views(b, num_views, views, /*train=*/false, false);
+        build_views(b, num_views, views, /*train=*/false, /*ahead=*/false);
         ensure_scratch(b, s);
         b->sh = dtv::shade_constants(*params);
         upload_views(b, s);
@@ -1109,7 +1111,8 @@ int32_t dtv_batch_render(dtv_batch* b, int32_t num_views, const dtv_batch_view* 
         DTV_CK(cudaMemcpyAsync(b->h_info, b->info.ptr, sizeof(ListInfo), cudaMemcpyDeviceToHost, s));
         DTV_CK(cudaStreamSynchronize(s));
         const u64 nf = b->h_info->nf;
-        b->many_left = b->h_info->clipped != 0u;
+        note_clipped(b);
+        b->walk = b->walk && !b->clipped_views;
         if (params->fragment_budget_bytes && nf * sizeof(u64) > params->fragment_budget_bytes) {
             DTV_CK(cudaMemsetAsync(b->counts.ptr, 0, sizeof(uint32_t) * b->tot_pixels, s));
             throw DtvError(DTV_ERR_BUDGET, "batch needs " + std::to_string(nf) + " fragments, over the budget");
@@ -1136,7 +1139,7 @@ int32_t dtv_batch_render_async(dtv_batch* b, int32_t num_views, const dtv_batch_
             throw DtvError(DTV_ERR_STATE, "dtv_batch_render_async needs record capacity (dtv_batch_reserve)");
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         b->have_render = false;
-        build_views(b, num_views, views, /*train=*/false, false);
+        build_views(b, num_views, views, /*train=*/false, /*ahead=*/true);
         ensure_scratch(b, s);
         b->sh = dtv::shade_constants(*params);
         upload_views(b, s);
@@ -1154,7 +1157,7 @@ int32_t dtv_batch_render_status(const dtv_batch* cb, int32_t* fits, uint64_t* nu
         require(b && fits && num_fragments, "null pointer");
         if (!b->have_render || !b->async_render)
             throw DtvError(DTV_ERR_STATE, "no dtv_batch_render_async to report on");
-        b->many_left = b->h_info->clipped != 0u;
+        note_clipped(b);
         *fits = b->h_info->ok != 0u ? 1 : 0;
         *num_fragments = b->h_info->nf;
     });
@@ -1248,7 +1251,7 @@ void enqueue_train_body(dtv_batch* b, const dtv::AdamConst& ac, int nslots, cuda
 std::vector<u64> train_signature(const dtv_batch* b, const dtv::AdamConst& ac, int nslots) {
     std::vector<u64> sig = {u64(b->nviews), b->tot_verts, b->tot_faces, b->tot_bfaces, b->tot_pixels, b->tot_tiles,
                             b->tot_rows, u64(b->max_height), b->capacity, u64(nslots), u64(b->walk),
-                            u64(b->many_left), u64(view_copies(b))};
+                            u64(view_copies(b))};
     const void* buffers[] = {b->d_views.ptr, b->d_slots.ptr, b->vproj.ptr, b->vfix.ptr, b->vgeo.ptr, b->counts.ptr,
                              b->offsets.ptr, b->records.ptr, b->scan.ptr, b->tfinal.ptr, b->term.ptr,
                              b->long_list.ptr, b->info.ptr, b->redo.ptr, b->clipped.ptr, b->walk_verts.ptr,
@@ -1287,7 +1290,7 @@ int32_t dtv_batch_train_step(dtv_batch* b, int32_t num_views, const dtv_batch_vi
         require(opt->fixed_boundary >= 0 && opt->fixed_boundary <= 2, "fixed_boundary must be 0, 1 or 2");
         cudaStream_t user = static_cast<cudaStream_t>(stream);
         b->have_render = false;
-        build_views(b, num_views, views, /*train=*/true, true);
+        build_views(b, num_views, views, /*train=*/true, /*ahead=*/true);
         for (int i = 0; i < num_views; ++i)
             require(views[i].d_target != nullptr, "every view of a training step needs d_target");
         ensure_scratch(b, user);
@@ -1377,7 +1380,7 @@ int32_t dtv_batch_train_step(dtv_batch* b, int32_t num_views, const dtv_batch_vi
             }
             DTV_CK(cudaMemcpyAsync(b->h_info, b->info.ptr, sizeof(dtv::ListInfo), cudaMemcpyDeviceToHost, ws));
             DTV_CK(cudaStreamSynchronize(ws));
-            b->many_left = b->h_info->clipped != 0u;
+            note_clipped(b);
             return b->h_info->ok != 0u;
         };
         bool done = run(true);

@@ -79,13 +79,12 @@ void launch_boundary_fill(const uint4* faces, uint32_t F, const float4* vproj, c
                           const uint32_t* gate, cudaStream_t s);
 struct ListInfo;
 // The few pixels the walk left to the rasteriser (nothing is done when there
-// are none, or when clipped vertices make them many: launch_raster_fill with
-// rest and launch_sort of the list then): fill from all faces, sort of the
-// listed pixels' lists.
+// are none; many: launch_raster_fill with rest and launch_sort of the list):
+// fill from all faces, sort of the listed pixels' lists.
 void launch_rest_fill(const ListInfo* info, const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W,
                       int row0, int row1, uint32_t* counts, const unsigned long long* offsets,
                       unsigned long long* records, const uint32_t* redo, cudaStream_t s);
-void launch_rest_sort(const ListInfo* info, bool few, const uint32_t* list, const unsigned long long* offsets,
+void launch_rest_sort(const ListInfo* info, const uint32_t* list, const unsigned long long* offsets,
                       unsigned long long* records, cudaStream_t s);
 // Order of the faces for the fill, grouped by row bands of about
 // kFillBandBytes of records each (nf records over H rows; order: F entries;
@@ -106,7 +105,7 @@ struct ListInfo {
     unsigned long long nf;  // records of the lists
     uint32_t ok;            // they fit
     uint32_t clipped;
-    uint32_t whole;         // ok and not clipped: the walk and what follows it complete the lists
+    uint32_t whole;         // ok and not clipped: the lists are walked
     uint32_t n_redo;        // pixels the walk left to the rasteriser
 };
 void launch_scan(const uint32_t* counts, uint64_t n, unsigned long long* offsets, unsigned long long* scratch,
@@ -243,7 +242,7 @@ void launch_build_walk(const uint4* cells, uint32_t T, const uint4* tet_faces, c
                        cudaStream_t s);
 // Lists of pixel rows [row0, row1) from the boundary fragments at the end of
 // each pixel's range.  Pixels it cannot finish are appended to `redo`
-// (info->n_redo of them).  guarded: nothing is done when info->ok is zero.
+// (info->n_redo of them).  guarded: nothing is done when info->whole is zero.
 void launch_walk_lists(const WalkMesh& wm, const unsigned long long* offsets, unsigned long long* records,
                        uint32_t* counts, const WalkVertRow* verts, int W, int row0, int row1, ListInfo* info,
                        uint32_t* redo, bool guarded, cudaStream_t s);

@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_raster_listed(const uint4
 
 // Fill of the few pixels the walk left to the rasteriser (their counters hold
 // the list length, all others zero), 32 faces per warp and step over a fixed
-// grid; nothing is done unless few_left.  Faces without such a pixel in the
+// grid; nothing is done when there are none (rounding cannot make any; loops of
+// inverted tets and far vertices do).  Faces without such a pixel in the
 // tiles of their box (2^shift px square, the smallest that the mask holds) end
 // after their setup: 2,950 -> 290 us at 64^3 / 1024^2 with 170 pixels left, 530
 // with 840 (fill and sort).
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps) k_rest_fill(const ListInfo*
                                                                  const u64* __restrict__ offsets,
                                                                  u64* __restrict__ records,
                                                                  const uint32_t* __restrict__ redo, int shift) {
-    const uint32_t left = few_left(info);
+    const uint32_t left = info->n_redo;
     if (!left) return;
     __shared__ RasterJob jobs[kRasterWarps][32];
     __shared__ uint32_t mask[kRestMaskBits / 32];
@@ -1162,11 +1163,11 @@ __global__ void __launch_bounds__(1024) k_sort_class_long(const u64* __restrict_
 // pixels the walk leaves to the rasteriser, whatever their length, in one
 // launch that costs next to nothing when there are none.
 constexpr uint32_t kRestCap = 2048;
-__global__ void __launch_bounds__(256) k_rest_sort(const ListInfo* __restrict__ info, bool few,
+__global__ void __launch_bounds__(256) k_rest_sort(const ListInfo* __restrict__ info,
                                                    const uint32_t* __restrict__ list,
                                                    const u64* __restrict__ offsets, u64* records) {
     __shared__ u64 sm[kRestCap];
-    const uint32_t num = few ? few_left(info) : info->n_redo;
+    const uint32_t num = info->n_redo;
     for (uint32_t i = blockIdx.x; i < num; i += gridDim.x) {
         const uint32_t p = list[i];
         const u64 beg = offsets[p], n = offsets[p + 1] - beg;
@@ -1185,8 +1186,8 @@ __global__ void __launch_bounds__(256) k_rest_sort(const ListInfo* __restrict__ 
     }
 }
 
-void launch_rest_sort(const ListInfo* info, bool few, const uint32_t* list, const u64* offsets, u64* records, cudaStream_t s) {
-    k_rest_sort<<<148 * 8, 256, 0, s>>>(info, few, list, offsets, records);
+void launch_rest_sort(const ListInfo* info, const uint32_t* list, const u64* offsets, u64* records, cudaStream_t s) {
+    k_rest_sort<<<148 * 8, 256, 0, s>>>(info, list, offsets, records);
 }
 
 static_assert(kSortClasses == 9, "k_sort_classify assigns classes 0..8");

@@ -331,11 +331,6 @@ __device__ __forceinline__ void raster_warp(const RasterJob* jobs, uint32_t live
     }
 }
 
-// Pixels the walk left to the rasteriser when that are few (rounding cannot
-// make any; loops of inverted tets and far vertices do).  With clipped
-// vertices many pixels' chains are cut: the launches for many pixels follow.
-__device__ __forceinline__ uint32_t few_left(const ListInfo* info) { return info->clipped ? 0u : info->n_redo; }
-
 // Tiles with a pixel left to the rasteriser, one bit each, in a block's shared
 // memory: the rest fills pass over all faces for a few pixels (those that closed
 // loops of faces around inverted tets cover), and a face whose box has none of

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kWalkListThreads) k_walk_lists(
     constexpr int N = kWalkListThreads;
     __shared__ u64 starts[kWalkStarts * N];
     __shared__ u64 recs[4 * N];
-    if (guarded && info->ok == 0u) return;
+    if (guarded && info->whole == 0u) return;
     const int lane = int(threadIdx.x & 31u), w = int(threadIdx.x >> 5);
     const int px = blockIdx.x * 16 + (w & 1) * 8 + lane % 8;
     const int py = row0 + int(blockIdx.y) * 8 + (w >> 1) * 4 + lane / 8;

@@ -114,3 +114,50 @@ def test_batch_matches_plain_views(kinds):
              for i, sc in enumerate(scs)]
     for img, (_, r) in zip(br.render(views), made):
         assert float((img - r.render()).abs().max()) <= 1e-6
+
+
+NEAR, WHOLE, FAR_OFF = [0.31, 0.22, 0.43], [1.6, 1.1, 2.3], [0.1, 0.2, 1.02]
+
+
+def test_lists_of_clipped_and_whole_views_in_turn(oracle):
+    """Views with and without clipped vertices from one renderer, in every
+    order of two; small and large ones (the record buffer grows in between)."""
+    from difftetvr_b200 import synthetic as S
+    sc = Scene(6, 93, seed=7)
+    mesh, r = sc.make_renderer()
+    fa = oracle.Faces(sc.cells, sc.pos.shape[0])
+    for at, res in [(WHOLE, 40), (NEAR, 93), (NEAR, 40), (WHOLE, 93), (WHOLE, 93), (FAR_OFF, 93), (WHOLE, 150),
+                    (NEAR, 150), (WHOLE, 40)]:
+        sc.view, sc.res = S.look_at_view(at), res
+        off_o, rec_o = oracle.fragments(fa, sc.pos, sc.oracle_camera(oracle))
+        r.set_view_matrix(sc.view)
+        r.set_viewport_size(res, res)
+        r.render()
+        off_g, rec_g = r.get_fragment_lists()
+        assert np.array_equal(off_g.astype(np.int64), off_o) and np.array_equal(rec_g, rec_o)
+
+
+@pytest.mark.parametrize("how", ["render", "async", "train"])
+def test_batches_of_clipped_and_whole_views_in_turn(how):
+    from difftetvr_b200 import synthetic as S
+    from difftetvr_b200.batch import BatchRenderer, View
+    sc = Scene(6, 93, seed=7)
+    mesh, r = sc.make_renderer()
+    br = BatchRenderer([mesh], attenuation=1.0, use_early_ray_termination=False)
+    br.reserve(4, 4 * len(sc.pos), 4 * 93 * 93, 4 * 93 * 93 * 200, len(sc.pos))
+    br.set_graph(how == "train")
+    for cams in [[WHOLE, WHOLE], [WHOLE, NEAR], [NEAR, FAR_OFF], [WHOLE, WHOLE], [WHOLE, WHOLE], [FAR_OFF, WHOLE]]:
+        views = [View(mesh=0, view_matrix=S.look_at_view(c), width=93, height=93, fovy=sc.fovy) for c in cams]
+        if how == "render":
+            br.render(views)
+        elif how == "async":
+            br.render_async(views)
+            torch.cuda.synchronize()
+            assert br.render_status()[0]
+        else:
+            for v in views:
+                v.target = torch.zeros((93, 93, 4), device="cuda")
+            br.train_step(views, lr_positions=0.0, lr_colors=0.0)  # the mesh stays
+        for v in views:
+            r.set_view_matrix(v.view_matrix)
+            assert float((v.image - r.render()).abs().max()) <= 1e-6
