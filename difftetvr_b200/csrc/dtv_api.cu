@@ -112,11 +112,18 @@ struct dtv_renderer {
     DevBuf<uint32_t> clipped;     // [0]: the projection met a vertex it does not project
     cudaEvent_t ev_info = nullptr;  // the record total is on the host
     DevBuf<uint32_t> redo;        // pixels the walk left to the rasteriser
-    // How many they were in the last walked render (pinned, one number per band
-    // up to kLeftSlots, written when its lists are done), and the renders left
-    // that do not walk (many_left).
-    volatile uint32_t* h_left = nullptr;
-    int left_n = 0;
+    // How many they were in the last two walked renders in turn (pinned, one
+    // number per band up to kLeftSlots, there when `done` is) and the pixels they
+    // were left of; whether a walk of this mesh was counted; and the renders
+    // left that do not walk (many_left).
+    struct Left {
+        volatile uint32_t* n = nullptr;
+        int slots = 0;
+        uint64_t pixels = 0;
+        cudaEvent_t done = nullptr;
+    } left[2];
+    int left_now = 0;
+    bool left_known = false;
     int skip_walk = 0;
     dtv::ListInfo* h_info = nullptr;  // pinned
     // State of the last render.
@@ -136,25 +143,51 @@ namespace {
 
 constexpr int kLeftSlots = 64;
 
-// Whether this render walks.
-bool take_walk(dtv_renderer* r, const dtv_mesh* mesh, uint64_t P) {
-    if (r->mesh != mesh) r->left_n = r->skip_walk = 0;
-    if (!mesh->walkable) return false;
-    uint64_t left = 0;
-    for (int i = 0; i < r->left_n; ++i) left += r->h_left[i];
-    if (r->left_n && dtv::many_left(left, P)) {
-        r->left_n = 0;
-        r->skip_walk = dtv::kWalkRetry;
+// What a walked render left decides on the next ones, once its numbers are there.
+void judge_left(dtv_renderer* r, int which) {
+    auto& l = r->left[which];
+    if (l.slots == 0) return;
+    if (cudaEventQuery(l.done) != cudaSuccess) {
+        cudaGetLastError();
+        return;
     }
-    return r->skip_walk == 0 || r->skip_walk-- == 0;
+    uint64_t n = 0;
+    for (int i = 0; i < l.slots; ++i) n += l.n[i];
+    l.slots = 0;
+    if (dtv::many_left(n, l.pixels)) r->skip_walk = dtv::kWalkRetry;
 }
 
-// The number of pixels the walk left, to the host (slot: the band).
-void read_left(dtv_renderer* r, int slot, cudaStream_t s) {
+// Whether this render walks.  (The render before it is judged here if it is
+// done, else when this one's scan is.)
+bool take_walk(dtv_renderer* r, const dtv_mesh* mesh) {
+    if (r->mesh != mesh) {
+        r->left[0].slots = r->left[1].slots = r->skip_walk = 0;
+        r->left_known = false;
+    }
+    if (!mesh->walkable) return false;
+    judge_left(r, r->left_now);
+    if (r->skip_walk > 0) {
+        --r->skip_walk;
+        r->left[0].slots = r->left[1].slots = 0;
+        r->left_known = false;
+        return false;
+    }
+    r->left_now ^= 1;
+    r->left[r->left_now].slots = 0;
+    return true;
+}
+
+// The number of pixels that the walk of `pixels` pixels left, to the host
+// (slot: the band).
+void read_left(dtv_renderer* r, int slot, uint64_t pixels, cudaStream_t s) {
     if (slot >= kLeftSlots) return;
-    DTV_CK(cudaMemcpyAsync(const_cast<uint32_t*>(r->h_left) + slot, &r->info.ptr->n_redo, sizeof(uint32_t),
+    auto& l = r->left[r->left_now];
+    DTV_CK(cudaMemcpyAsync(const_cast<uint32_t*>(l.n) + slot, &r->info.ptr->n_redo, sizeof(uint32_t),
                            cudaMemcpyDeviceToHost, s));
-    r->left_n = slot + 1;
+    DTV_CK(cudaEventRecord(l.done, s));
+    l.pixels = slot == 0 ? pixels : l.pixels + pixels;
+    l.slots = slot + 1;
+    r->left_known = true;
 }
 
 dtv::WalkMesh walk_mesh(const dtv_mesh* m) {
@@ -262,7 +295,7 @@ void build_band_lists(dtv_renderer* r, const dtv_mesh* mesh, const dtv::CamDev& 
     check_launch("band scan");
     if (r->band_walk) {
         walk_rows(r, mesh, cam, y0, y1, false, s);
-        read_left(r, band, s);
+        read_left(r, band, pb, s);
         rest_rows(r, mesh, cam, y0, y1, /*few=*/true, s);
         return;
     }
@@ -540,8 +573,10 @@ int32_t dtv_renderer_create(int32_t type, dtv_renderer** out) {
         r->type = type;
         try {
             DTV_CK(cudaMallocHost(&r->h_info, sizeof(dtv::ListInfo)));
-            DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&r->h_left), sizeof(uint32_t) * kLeftSlots));
-            for (int i = 0; i < kLeftSlots; ++i) r->h_left[i] = 0u;
+            for (auto& l : r->left) {
+                DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&l.n), sizeof(uint32_t) * kLeftSlots));
+                DTV_CK(cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming));
+            }
             for (auto& e : r->ev) DTV_CK(cudaEventCreate(&e));
             DTV_CK(cudaEventCreateWithFlags(&r->ev_info, cudaEventDisableTiming));
         } catch (...) {
@@ -578,7 +613,10 @@ int32_t dtv_renderer_destroy(dtv_renderer* r) {
     if (r->ev_info) cudaEventDestroy(r->ev_info);
     r->walk_verts.release();
     if (r->h_info) cudaFreeHost(r->h_info);
-    if (r->h_left) cudaFreeHost(const_cast<uint32_t*>(r->h_left));
+    for (auto& l : r->left) {
+        if (l.n) cudaFreeHost(const_cast<uint32_t*>(l.n));
+        if (l.done) cudaEventDestroy(l.done);
+    }
     if (r->h_rowoff) cudaFreeHost(r->h_rowoff);
     for (auto& e : r->ev)
         if (e) cudaEventDestroy(e);
@@ -634,7 +672,7 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
 
         r->wide_list.ensure(size_t(F) + 1, s);
         rec_event(r, 0, s);
-        const bool walk = !raytet && take_walk(r, mesh, P);
+        const bool walk = !raytet && take_walk(r, mesh);
         if (walk) {
             r->walk_verts.ensure(V ? V : 1, s);
             r->clipped.ensure(1, s, /*zero_new=*/true);
@@ -677,12 +715,13 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         auto lists_and_composite = [&](bool guarded) {
             rec_event(r, 3, s);
             walk_rows(r, mesh, cam, 0, H, guarded, s);
-            const bool known = r->left_n > 0;
-            read_left(r, 0, s);
+            const bool known = r->left_known;
+            read_left(r, 0, P, s);
             bool few = true;
             if (!known) {
                 DTV_CK(cudaStreamSynchronize(s));
-                few = !dtv::many_left(r->h_left[0], P);
+                judge_left(r, r->left_now);
+                few = r->skip_walk == 0;
                 if (!few) order_faces();
             }
             rec_event(r, 4, s);
@@ -691,9 +730,10 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
             composite_rows(r, mesh, d_colors, cam, sh, d_image, 0, H, s, &r->info.ptr->whole);
             check_launch("composite");
         };
-        const bool early = walk && r->records.ptr && r->left_n > 0 && !r->clipped_view;
+        const bool early = walk && r->records.ptr && r->left_known && !r->clipped_view;
         if (early) lists_and_composite(true);
         DTV_CK(cudaEventSynchronize(r->ev_info));
+        if (walk) judge_left(r, r->left_now ^ 1);
         const uint64_t nf = r->h_info->nf;
         const bool walked = early && r->h_info->whole != 0u;
         r->clipped_view = walk && r->h_info->clipped != 0u;

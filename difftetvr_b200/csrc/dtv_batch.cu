@@ -593,6 +593,7 @@ struct dtv_batch {
         dtv::WalkMesh walk{};        // links null: the mesh cannot be walked
         uint32_t Nb = 0;
         const uint32_t* boundary = nullptr;
+        int skip_walk = 0;           // batches with this mesh left that do not walk (many_left)
         // training state (allocated on the first train step)
         DevBuf<float> m_pos, v_pos;
         DevBuf<float4> m_col, v_col;
@@ -618,14 +619,18 @@ struct dtv_batch {
     DevBuf<dtv::ListInfo> info;     // record total, whether it fits, pixels the walk left
     DevBuf<uint32_t> redo;          // those pixels
     DevBuf<uint32_t> clipped;       // [0]: the projection met a vertex it does not project
-    // The last batch had clipped vertices, and the calls left that, enqueued
-    // before that is known of their own views, do not walk (render_common: a
-    // clipped view is not walked; a walked one is right all the same, its many
-    // left-over pixels are slow).
-    bool clipped_views = false;
+    // Calls left that, enqueued before it is known whether their views clip
+    // vertices, do not walk, after one that did (render_common: a clipped view
+    // is not walked; a walked one is right all the same, its many left-over
+    // pixels are slow).
     int skip_clipped = 0;
-    volatile uint32_t* h_left = nullptr;  // pinned: pixels the last walk left
-    int skip_walk = 0;                    // calls left that do not walk (many_left)
+    // What the last call found and left (pinned, there when `done` is), of how
+    // many pixels and which meshes.
+    dtv::ListInfo* h_done = nullptr;
+    cudaEvent_t done = nullptr;
+    bool done_pending = false, done_walk = false;
+    u64 done_pixels = 0;
+    std::vector<char> used, done_used;   // by mesh: of this call, of the last one
     DevBuf<dtv::WalkVertRow> walk_verts;
     DevBuf<float4> grad_rows;
     DevBuf<uint32_t> fill_order;    // items (view faces) in row-band order for the fill
@@ -637,7 +642,7 @@ struct dtv_batch {
     DevBuf<float4> dimage_internal;
     DevBuf<float> loss;
     DevBuf<int> step;
-    dtv::ListInfo* h_info = nullptr;  // pinned
+    dtv::ListInfo* h_info = nullptr;  // pinned: what the scan of render() found
     // shapes of the last render (for the adjoint)
     int nviews = 0;
     u64 tot_verts = 0, tot_faces = 0, tot_bfaces = 0, tot_pixels = 0, tot_tiles = 0, tot_rows = 0;
@@ -668,10 +673,29 @@ void ensure_pinned(void** p, size_t& cap, size_t bytes) {
     cap = bytes;
 }
 
-// What the scan of a finished batch found (h_info).
-void note_clipped(dtv_batch* b) {
-    b->clipped_views = b->h_info->clipped != 0u;
-    if (b->clipped_views) b->skip_clipped = dtv::kWalkRetry;
+// What this call found and left, to the host.
+void read_done(dtv_batch* b, cudaStream_t s) {
+    DTV_CK(cudaMemcpyAsync(b->h_done, b->info.ptr, sizeof(dtv::ListInfo), cudaMemcpyDeviceToHost, s));
+    DTV_CK(cudaEventRecord(b->done, s));
+    b->done_pending = true;
+    b->done_walk = b->walk;
+    b->done_pixels = b->tot_pixels;
+    b->done_used = b->used;
+}
+
+// What it decides on the next calls, once it is there.
+void judge_done(dtv_batch* b) {
+    if (!b->done_pending) return;
+    if (cudaEventQuery(b->done) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    b->done_pending = false;
+    if (b->h_done->clipped != 0u)
+        b->skip_clipped = dtv::kWalkRetry;
+    else if (b->done_walk && dtv::many_left(b->h_done->n_redo, b->done_pixels))
+        for (size_t m = 0; m < b->meshes.size() && m < b->done_used.size(); ++m)
+            if (b->done_used[m]) b->meshes[m].skip_walk = dtv::kWalkRetry;
 }
 
 // Builds the descriptor table for `views`; returns the totals.  ahead: the
@@ -681,19 +705,14 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
     ensure_pinned(reinterpret_cast<void**>(&b->h_views), b->h_views_cap, sizeof(BatchView) * size_t(nviews));
     if (b->staging_free) DTV_CK(cudaEventSynchronize(b->staging_free));
     u64 vb = 0, fb = 0, bb = 0, pb = 0, tb = 0;
-    if (b->h_left && !b->clipped_views && dtv::many_left(*b->h_left, b->tot_pixels)) {
-        *b->h_left = 0u;
-        b->skip_walk = dtv::kWalkRetry;
-    }
-    bool walk = b->skip_walk == 0 || b->skip_walk-- == 0;
-    if (ahead && b->skip_clipped > 0) {
-        --b->skip_clipped;
-        walk = false;
-    }
+    judge_done(b);
+    bool walk = true;
+    b->used.assign(b->meshes.size(), 0);
     for (int i = 0; i < nviews; ++i) {
         const dtv_batch_view& in = views[i];
         require(in.mesh >= 0 && in.mesh < int(b->meshes.size()), "view mesh index out of range");
         const auto& me = b->meshes[size_t(in.mesh)];
+        b->used[size_t(in.mesh)] = 1;
         const dtv_camera& c = in.camera;
         require(c.width > 0 && c.height > 0 && c.width <= 16384 && c.height <= 16384, "viewport size out of range");
         require(c.znear > 0.f && c.zfar > c.znear, "need 0 < znear < zfar");
@@ -732,6 +751,15 @@ void build_views(dtv_batch* b, int nviews, const dtv_batch_view* views, bool tra
     }
     require(vb < (u64(1) << 32), "a batch holds fewer than 2^32 vertices in total");
     require(fb < (u64(1) << 32), "a batch holds fewer than 2^32 faces in total");
+    for (size_t m = 0; m < b->meshes.size(); ++m)
+        if (b->used[m] && b->meshes[m].skip_walk > 0) {
+            --b->meshes[m].skip_walk;
+            walk = false;
+        }
+    if (ahead && b->skip_clipped > 0) {
+        --b->skip_clipped;
+        walk = false;
+    }
     b->nviews = nviews;
     b->tot_verts = vb;
     b->tot_faces = fb;
@@ -771,14 +799,12 @@ u64 most_view_rows(u64 nv, u64 V, u64 P) {
     return std::max(V, std::min(per_view, by_pixels * std::min(V, kBatchGradRows)));
 }
 
-// Pinned words and the staging event, each by itself: a call that failed half
+// Pinned words and the events, each by itself: a call that failed half
 // way leaves what it got, and the next one makes the rest.
 void ensure_host(dtv_batch* b) {
     if (!b->h_info) DTV_CK(cudaMallocHost(&b->h_info, sizeof(dtv::ListInfo)));
-    if (!b->h_left) {
-        DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&b->h_left), sizeof(uint32_t)));
-        *b->h_left = 0u;
-    }
+    if (!b->h_done) DTV_CK(cudaMallocHost(&b->h_done, sizeof(dtv::ListInfo)));
+    if (!b->done) DTV_CK(cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming));
     if (!b->staging_free) DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
 }
 
@@ -868,8 +894,6 @@ void launch_kb_lists(dtv_batch* b, const dtv::ShadeDev& sh, bool guarded, cudaSt
         kb_walk_lists<<<unsigned(2 * b->tot_tiles), kTileThreads, 0, s>>>(
             b->d_views.ptr, b->nviews, b->offsets.ptr, b->records.ptr, b->counts.ptr, b->walk_verts.ptr, b->info.ptr,
             b->redo.ptr);
-        DTV_CK(cudaMemcpyAsync(const_cast<uint32_t*>(b->h_left), &b->info.ptr->n_redo, sizeof(uint32_t),
-                               cudaMemcpyDeviceToHost, s));
         kb_rest_fill<<<148 * 6, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->info.ptr, b->vproj.ptr,
                                              b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr, b->redo.ptr);
         launch_rest_sort(b->info.ptr, b->redo.ptr, b->offsets.ptr, b->records.ptr, s);
@@ -1041,7 +1065,8 @@ int32_t dtv_batch_destroy(dtv_batch* b) {
     if (b->h_views) cudaFreeHost(b->h_views);
     if (b->h_slots) cudaFreeHost(b->h_slots);
     if (b->h_info) cudaFreeHost(b->h_info);
-    if (b->h_left) cudaFreeHost(const_cast<uint32_t*>(b->h_left));
+    if (b->h_done) cudaFreeHost(b->h_done);
+    if (b->done) cudaEventDestroy(b->done);
     if (b->staging_free) cudaEventDestroy(b->staging_free);
     delete b;
     return DTV_OK;
@@ -1077,8 +1102,10 @@ int32_t dtv_batch_set_meshes(dtv_batch* b, int32_t num_meshes, const dtv_mesh* c
                 std::swap(me[i].v_pos, old.v_pos);
                 std::swap(me[i].m_col, old.m_col);
                 std::swap(me[i].v_col, old.v_col);
+                me[i].skip_walk = old.skip_walk;
             }
         }
+        b->done_pending = false;
         for (auto& old : b->meshes) {
             old.m_pos.release();
             old.v_pos.release();
@@ -1111,8 +1138,8 @@ int32_t dtv_batch_render(dtv_batch* b, int32_t num_views, const dtv_batch_view* 
         DTV_CK(cudaMemcpyAsync(b->h_info, b->info.ptr, sizeof(ListInfo), cudaMemcpyDeviceToHost, s));
         DTV_CK(cudaStreamSynchronize(s));
         const u64 nf = b->h_info->nf;
-        note_clipped(b);
-        b->walk = b->walk && !b->clipped_views;
+        judge_done(b);  // the call before this one
+        b->walk = b->walk && b->h_info->clipped == 0u;
         if (params->fragment_budget_bytes && nf * sizeof(u64) > params->fragment_budget_bytes) {
             DTV_CK(cudaMemsetAsync(b->counts.ptr, 0, sizeof(uint32_t) * b->tot_pixels, s));
             throw DtvError(DTV_ERR_BUDGET, "batch needs " + std::to_string(nf) + " fragments, over the budget");
@@ -1125,6 +1152,7 @@ int32_t dtv_batch_render(dtv_batch* b, int32_t num_views, const dtv_batch_view* 
         }
         launch_kb_lists(b, b->sh, /*guarded=*/false, s);
         check_launch("batch render");
+        read_done(b, s);
         b->last_fragments = nf;
         b->have_render = true;
         b->async_render = false;
@@ -1145,7 +1173,7 @@ int32_t dtv_batch_render_async(dtv_batch* b, int32_t num_views, const dtv_batch_
         upload_views(b, s);
         b->capacity = b->records.cap;
         enqueue_forward(b, b->sh, s);
-        DTV_CK(cudaMemcpyAsync(b->h_info, b->info.ptr, sizeof(dtv::ListInfo), cudaMemcpyDeviceToHost, s));
+        read_done(b, s);
         b->have_render = true;
         b->async_render = true;
     });
@@ -1157,9 +1185,9 @@ int32_t dtv_batch_render_status(const dtv_batch* cb, int32_t* fits, uint64_t* nu
         require(b && fits && num_fragments, "null pointer");
         if (!b->have_render || !b->async_render)
             throw DtvError(DTV_ERR_STATE, "no dtv_batch_render_async to report on");
-        note_clipped(b);
-        *fits = b->h_info->ok != 0u ? 1 : 0;
-        *num_fragments = b->h_info->nf;
+        judge_done(b);
+        *fits = b->h_done->ok != 0u ? 1 : 0;
+        *num_fragments = b->h_done->nf;
     });
 }
 
@@ -1378,15 +1406,14 @@ int32_t dtv_batch_train_step(dtv_batch* b, int32_t num_views, const dtv_batch_vi
             } else {
                 enqueue_train_body(b, ac, nslots, ws);
             }
-            DTV_CK(cudaMemcpyAsync(b->h_info, b->info.ptr, sizeof(dtv::ListInfo), cudaMemcpyDeviceToHost, ws));
+            read_done(b, ws);
             DTV_CK(cudaStreamSynchronize(ws));
-            note_clipped(b);
-            return b->h_info->ok != 0u;
+            return b->h_done->ok != 0u;
         };
         bool done = run(true);
         if (!done) {
             // Records did not fit: grow, rerun this step uncaptured, recapture next time.
-            const u64 need = b->h_info->nf;
+            const u64 need = b->h_done->nf;
             b->capacity = u64(double(need) * 1.25) + 1024;
             b->records.ensure(b->capacity, ws);
             b->capacity = b->records.cap;
@@ -1399,7 +1426,7 @@ int32_t dtv_batch_train_step(dtv_batch* b, int32_t num_views, const dtv_batch_vi
             done = run(false);
             if (!done) throw DtvError(DTV_ERR_STATE, "batch records overflowed after resizing");
         }
-        b->last_fragments = b->h_info->nf;
+        b->last_fragments = b->h_done->nf;
         if (d_loss) DTV_CK(cudaMemcpyAsync(d_loss, b->loss.ptr, sizeof(float), cudaMemcpyDeviceToDevice, ws));
         DTV_CK(cudaEventRecord(ev_out, ws));
         DTV_CK(cudaStreamWaitEvent(user, ev_out, 0));

@@ -50,3 +50,33 @@ def test_batches_of_tangled_meshes(jitter):
     for _ in range(4):
         for out in br.render(views):
             assert float((out - img).abs().max()) <= 1e-6
+
+
+def test_lists_of_tangled_and_plain_meshes_in_turn_at_two_sizes(oracle):
+    """What one render left decides on others: of another mesh, at another size."""
+    made = []
+    for jitter in (3.0, 0.2):
+        sc = Scene(7, 101, seed=12, jitter=jitter)
+        made.append((sc, sc.make_renderer()[0], oracle.Faces(sc.cells, sc.pos.shape[0])))
+    r = made[0][0].make_renderer()[1]
+    for k, res in [(0, 101), (0, 33), (1, 33), (1, 101), (0, 101), (0, 101), (0, 33), (0, 33), (1, 101)]:
+        sc, mesh, fa = made[k]
+        sc.res = res
+        r.set_tet_mesh(mesh)
+        r.set_viewport_size(res, res)
+        r.render()
+        off, rec = r.get_fragment_lists()
+        off_o, rec_o = oracle.fragments(fa, sc.pos, sc.oracle_camera(oracle))
+        assert np.array_equal(off.astype(np.int64), off_o.astype(np.int64)) and np.array_equal(rec, rec_o)
+
+
+def test_batches_of_tangled_and_plain_meshes_in_turn():
+    from difftetvr_b200.batch import BatchRenderer, View
+    scs = [Scene(7, 101, seed=12, jitter=j) for j in (3.0, 0.2)]
+    made = [sc.make_renderer() for sc in scs]
+    imgs = [r.render().clone() for _, r in made]
+    br = BatchRenderer([m for m, _ in made], attenuation=scs[0].attenuation, use_early_ray_termination=False)
+    for idx in [(0, 0), (1, 1), (0, 1), (1, 1), (0,), (1,), (0, 0)]:
+        views = [View(mesh=i, view_matrix=scs[i].view, width=101, height=101, fovy=scs[i].fovy) for i in idx]
+        for i, out in zip(idx, br.render(views)):
+            assert float((out - imgs[i]).abs().max()) <= 1e-6
