@@ -777,7 +777,7 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         }
         if (!walk_now) {
             rec_event(r, 3, s);
-            if (raytet) {
+            if (raytet && !dtv::many_boundary_faces(F)) {
                 dtv::launch_boundary_fill(rfaces, uint32_t(F), r->vproj.ptr, r->vfix.ptr, W, 0, H, r->counts.ptr,
                                           r->offsets.ptr, r->records.ptr, nullptr, s);
             } else {

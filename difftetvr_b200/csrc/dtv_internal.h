@@ -54,6 +54,13 @@ inline FillSplit fill_split(uint64_t F, uint64_t image_rows) {
     return FillSplit{uint32_t(w < 1 ? 1 : (w > 32 ? 32 : w)), uint32_t(p < 1 ? 1 : (p > 16 ? 16 : p))};
 }
 
+// Whether boundary faces are so many (unconnected tets) that their fill in
+// row-band order (launch_raster_fill) is worth ordering them: past 64 per warp
+// slot of the GPU.  Boundary fill against fill in bands (us): 331 k faces at
+// 512^2 495 and 527, at 1024^2 3,011 and 3,026; 786 k at 512^2 713 and 583, at
+// 1024^2 3,798 and 3,388; 1.5 M at 1024^2 4,679 and 3,030.
+inline bool many_boundary_faces(uint64_t F) { return F > 64 * 148 * 64; }
+
 // Launch wrappers (dtv_kernels.cu).  All run on `s`.
 // rows (optional): the vertices' walk rows as well; clipped (optional): set to
 // 1 when a vertex is not projected; wide_list (optional): [0] cleared for the

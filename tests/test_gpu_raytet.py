@@ -211,3 +211,20 @@ def test_walk_is_deterministic_and_differs_from_list_path_off_axis():
     c = rl.render()
     covered = c[..., 3] > 1e-3
     assert bool((a[..., 3][covered] >= c[..., 3][covered] - 1e-6).all())
+
+
+@pytest.mark.parametrize("n", [29, 30])   # 585 k and 648 k faces: filled as they come, and in row-band order
+def test_lists_of_many_unconnected_tets(oracle, n):
+    sc = Scene(n, 64, seed=4)
+    p = sc.pos[sc.cells.astype(np.int64)]
+    centre = p.mean(axis=1, keepdims=True)
+    sc.pos = ((p - centre) * np.float32(0.95) + centre).reshape(-1, 3).astype(np.float32)
+    sc.col = np.repeat(sc.col[:1], len(sc.pos), axis=0)
+    sc.cells = np.arange(len(sc.pos), dtype=np.uint32).reshape(-1, 4)
+    mesh, r = sc.make_renderer(_intersection())
+    fa = oracle.Faces(sc.cells, sc.pos.shape[0])
+    off_o, rec_o = oracle.fragments(fa, sc.pos, sc.oracle_camera(oracle))
+    for _ in range(2):
+        r.render()
+        off_g, rec_g = r.get_fragment_lists()
+        assert np.array_equal(off_g.astype(np.int64), off_o.astype(np.int64)) and np.array_equal(rec_g, rec_o)
