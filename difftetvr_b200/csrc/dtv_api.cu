@@ -69,10 +69,11 @@ struct dtv_mesh {
     uint4* d_bfaces = nullptr;         // Nb
     uint32_t* d_bf_global = nullptr;   // Nb
     std::vector<uint32_t> bf_global;   // host copy
-    // Tables of the list walk; `walkable`: the topology can be walked and at
-    // most three quarters of the faces are boundary faces (else the lists are
-    // filled by the rasteriser and sorted: with unconnected tets every face is
-    // the start or end of a chain of its own).
+    // Tables of the list walk (64 bytes per tet), held where `walkable`: there
+    // is memory for them, the topology can be walked and at most three quarters
+    // of the faces are boundary faces (else the lists are filled by the
+    // rasteriser and sorted: with unconnected tets every face is the start or
+    // end of a chain of its own).
     uint4* d_walk_links = nullptr;
     uint4* d_walk_start = nullptr;
     bool walkable = false;
@@ -409,6 +410,40 @@ void adjoint_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors
     check_launch("scatter gradients");
 }
 
+// The mesh's walk tables, if they can be had (walkable); a mesh without them
+// renders all the same.
+void build_walk_tables(dtv_mesh* m) {
+    const uint64_t T = m->host.num_cells, Nb = m->bf_global.size();
+    DevBuf<uint32_t> bad;
+    uint32_t h_bad = 1;
+    if (cudaMalloc(&m->d_walk_links, sizeof(uint4) * 4 * T) == cudaSuccess &&
+        cudaMalloc(&m->d_walk_start, sizeof(uint4) * (Nb ? Nb : 1)) == cudaSuccess) {
+        try {
+            bad.ensure(1, nullptr, /*zero_new=*/true);
+            dtv::launch_build_walk(reinterpret_cast<const uint4*>(m->d_cells), uint32_t(T),
+                                   reinterpret_cast<const uint4*>(m->d_tet_faces), m->d_faces,
+                                   reinterpret_cast<const uint2*>(m->d_face_to_tet), m->d_bf_global, uint32_t(Nb),
+                                   m->d_walk_links, m->d_walk_start, bad.ptr, nullptr);
+            check_launch("walk tables");
+            DTV_CK(cudaMemcpy(&h_bad, bad.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+        } catch (const DtvError& e) {
+            if (e.code != DTV_ERR_BUDGET) {
+                bad.release();
+                throw;
+            }
+        }
+        bad.release();
+    } else {
+        cudaGetLastError();
+    }
+    m->walkable = h_bad == 0;
+    if (!m->walkable) {
+        cudaFree(m->d_walk_links);
+        cudaFree(m->d_walk_start);
+        m->d_walk_links = m->d_walk_start = nullptr;
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -493,24 +528,7 @@ int32_t dtv_mesh_create(const uint32_t* h_cells, uint64_t num_cells, uint64_t nu
                                   sizeof(uint32_t) * num_vertices, cudaMemcpyHostToDevice));
             if (num_cells) {
                 DTV_CK(cudaMemcpy(m->d_cells, h_cells, sizeof(uint32_t) * 4 * num_cells, cudaMemcpyHostToDevice));
-                DTV_CK(cudaMalloc(&m->d_walk_links, sizeof(uint4) * 4 * num_cells));
-                DTV_CK(cudaMalloc(&m->d_walk_start, sizeof(uint4) * (Nb ? Nb : 1)));
-                DevBuf<uint32_t> bad;
-                uint32_t h_bad = 1;
-                try {
-                    bad.ensure(1, nullptr, /*zero_new=*/true);
-                    dtv::launch_build_walk(reinterpret_cast<const uint4*>(m->d_cells), uint32_t(num_cells),
-                                           reinterpret_cast<const uint4*>(m->d_tet_faces), m->d_faces,
-                                           reinterpret_cast<const uint2*>(m->d_face_to_tet), m->d_bf_global,
-                                           uint32_t(Nb), m->d_walk_links, m->d_walk_start, bad.ptr, nullptr);
-                    check_launch("walk tables");
-                    DTV_CK(cudaMemcpy(&h_bad, bad.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-                } catch (...) {
-                    bad.release();
-                    throw;
-                }
-                bad.release();
-                m->walkable = h_bad == 0 && 4 * Nb <= 3 * F;
+                if (4 * Nb <= 3 * F) build_walk_tables(m);
             }
         } catch (...) {
             dtv_mesh_destroy(m);
@@ -672,11 +690,16 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
 
         r->wide_list.ensure(size_t(F) + 1, s);
         rec_event(r, 0, s);
-        const bool walk = !raytet && take_walk(r, mesh);
+        bool walk = !raytet && take_walk(r, mesh);
         if (walk) {
-            r->walk_verts.ensure(V ? V : 1, s);
-            r->clipped.ensure(1, s, /*zero_new=*/true);
-            r->redo.ensure(P, s);
+            try {
+                r->walk_verts.ensure(V ? V : 1, s);
+                r->clipped.ensure(1, s, /*zero_new=*/true);
+                r->redo.ensure(P, s);
+            } catch (const DtvError& e) {
+                if (e.code != DTV_ERR_BUDGET) throw;
+                walk = false;  // no memory for the walk: fill and sort
+            }
         }
         dtv::launch_project(d_positions, uint32_t(V), cam, r->vproj.ptr, r->vfix.ptr, r->vgeo.ptr, s,
                             walk ? r->walk_verts.ptr : nullptr, walk ? r->clipped.ptr : nullptr, r->wide_list.ptr);

@@ -808,6 +808,19 @@ void ensure_host(dtv_batch* b) {
     if (!b->staging_free) DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
 }
 
+// Buffers of the walk of V vertices and P pixels; false: no memory for them (the
+// batch does not walk).
+bool ensure_walk(dtv_batch* b, u64 V, u64 P, cudaStream_t s) {
+    try {
+        b->walk_verts.ensure(V ? V : 1, s);
+        b->redo.ensure(P, s);
+        return true;
+    } catch (const DtvError& e) {
+        if (e.code != DTV_ERR_BUDGET) throw;
+        return false;
+    }
+}
+
 void ensure_scratch(dtv_batch* b, cudaStream_t s) {
     b->d_views.ensure(size_t(b->nviews), s);
     b->vproj.ensure(b->tot_verts ? b->tot_verts : 1, s);
@@ -825,10 +838,7 @@ void ensure_scratch(dtv_batch* b, cudaStream_t s) {
     b->long_list.ensure(dtv::sort_scratch_elems(b->tot_pixels), s);
     b->info.ensure(1, s);
     b->clipped.ensure(1, s, /*zero_new=*/true);
-    if (b->walk) {
-        b->walk_verts.ensure(b->tot_verts ? b->tot_verts : 1, s);
-        b->redo.ensure(b->tot_pixels, s);
-    }
+    b->walk = b->walk && ensure_walk(b, b->tot_verts, b->tot_pixels, s);
     b->loss.ensure(1, s);
     ensure_host(b);
 }
@@ -1020,8 +1030,7 @@ int32_t dtv_batch_reserve(dtv_batch* b, uint64_t max_views, uint64_t max_vertice
         b->grad_rows.ensure(2 * (max_grad_vertices ? max_grad_vertices : 1), s);
         b->info.ensure(1, s);
         b->clipped.ensure(1, s, /*zero_new=*/true);
-        b->walk_verts.ensure(V, s);
-        b->redo.ensure(P, s);
+        ensure_walk(b, V, P, s);
         b->loss.ensure(1, s);
         ensure_host(b);
         DTV_CK(cudaStreamSynchronize(s));

@@ -80,3 +80,20 @@ def test_batches_of_tangled_and_plain_meshes_in_turn():
         views = [View(mesh=i, view_matrix=scs[i].view, width=101, height=101, fovy=scs[i].fovy) for i in idx]
         for i, out in zip(idx, br.render(views)):
             assert float((out - imgs[i]).abs().max()) <= 1e-6
+
+
+def test_a_mesh_that_is_not_walked_holds_no_walk_tables():
+    """Unconnected tets: device memory for faces, tets and boundary faces alone
+    (225 bytes per tet; the walk's tables would be 128 more)."""
+    from difftetvr_b200.tet_mesh import NativeMesh
+    T = 300_000
+    cells = np.arange(4 * T, dtype=np.uint32).reshape(-1, 4)
+    NativeMesh(cells[:100], 400)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    mesh = NativeMesh(cells, 4 * T)
+    used = free - torch.cuda.mem_get_info()[0]
+    assert mesh.num_faces == 4 * T
+    # face rows 64, face tets 32, boundary flags 16, tets 32 + 1, boundary faces 64 + 16, 225 in all; each
+    # allocation in whole 2 MiB pages
+    assert used <= 225 * T + 8 * (2 << 20)
