@@ -109,8 +109,9 @@ struct dtv_renderer {
     DevBuf<uint32_t> wide_list;     // [0] = n, then the faces of the 64-bit raster path (count -> fill)
     DevBuf<uint4> wstate;         // ray-tet path: (last tet, its entry face, boundary entry index, segments)
     DevBuf<dtv::WalkVertRow> walk_verts;  // per-view vertex rows of the list walk
-    DevBuf<dtv::ListInfo> info;   // record total and redo counters of the lists
-    DevBuf<uint32_t> clipped;     // [0]: the projection met a vertex it does not project
+    // [0]: what the scan found and the walk left; [1].clipped: the projection met
+    // a vertex it does not project.
+    DevBuf<dtv::ListInfo> info;
     cudaEvent_t ev_info = nullptr;  // the record total is on the host
     DevBuf<uint32_t> redo;        // pixels the walk left to the rasteriser
     // How many they were in the last two walked renders in turn (pinned, one
@@ -627,7 +628,6 @@ int32_t dtv_renderer_destroy(dtv_renderer* r) {
     r->wide_list.release();
     r->info.release();
     r->redo.release();
-    r->clipped.release();
     if (r->ev_info) cudaEventDestroy(r->ev_info);
     r->walk_verts.release();
     if (r->h_info) cudaFreeHost(r->h_info);
@@ -686,23 +686,24 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
             r->wstate.ensure(P, s);
         else
             r->term.ensure(P, s);
-        r->long_list.ensure(dtv::sort_scratch_elems(P), s);
-
         r->wide_list.ensure(size_t(F) + 1, s);
+        r->info.ensure(2, s, /*zero_new=*/true);
+        uint32_t* d_clipped = &r->info.ptr[1].clipped;
         rec_event(r, 0, s);
         bool walk = !raytet && take_walk(r, mesh);
         if (walk) {
             try {
                 r->walk_verts.ensure(V ? V : 1, s);
-                r->clipped.ensure(1, s, /*zero_new=*/true);
                 r->redo.ensure(P, s);
             } catch (const DtvError& e) {
                 if (e.code != DTV_ERR_BUDGET) throw;
                 walk = false;  // no memory for the walk: fill and sort
             }
         }
+        // Sort scratch (36 bytes per pixel) only where lists are sorted.
+        if (!walk) r->long_list.ensure(dtv::sort_scratch_elems(P), s);
         dtv::launch_project(d_positions, uint32_t(V), cam, r->vproj.ptr, r->vfix.ptr, r->vgeo.ptr, s,
-                            walk ? r->walk_verts.ptr : nullptr, walk ? r->clipped.ptr : nullptr, r->wide_list.ptr);
+                            walk ? r->walk_verts.ptr : nullptr, walk ? d_clipped : nullptr, r->wide_list.ptr);
         check_launch("project");
         rec_event(r, 1, s);
         dtv::launch_raster_count(rfaces, uint32_t(F), r->vproj.ptr, r->vfix.ptr, W, H, r->counts.ptr, s, 0, -1,
@@ -710,7 +711,6 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         check_launch("raster count");
         rec_event(r, 2, s);
         const uint64_t budget = params->fragment_budget_bytes;
-        r->info.ensure(1, s);
         // The walk and the composite are enqueued before the host knows the
         // record total: they run if the records fit what is allocated already
         // (and the budget) and no vertex is clipped.  The host waits for the
@@ -722,14 +722,21 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
         // against 747).
         const uint64_t room = std::min<uint64_t>(r->records.cap, budget ? budget / sizeof(u64) : ~0ull);
         dtv::launch_scan(r->counts.ptr, P, r->offsets.ptr, r->scan_scratch.ptr, s, r->info.ptr, room,
-                         walk ? r->clipped.ptr : nullptr);
+                         walk ? d_clipped : nullptr);
         check_launch("scan");
         DTV_CK(cudaMemcpyAsync(r->h_info, r->info.ptr, sizeof(dtv::ListInfo), cudaMemcpyDeviceToHost, s));
         DTV_CK(cudaEventRecord(r->ev_info, s));
-        // Faces in row-band order for the fill of whole lists.
+        // Faces in row-band order for the fill of whole lists, and the sort's
+        // scratch.
         auto order_faces = [&] {
-            r->fill_order.ensure(size_t(F), s);
-            r->band_scratch.ensure(2 * dtv::kFillBands, s);
+            try {
+                r->fill_order.ensure(size_t(F), s);
+                r->band_scratch.ensure(2 * dtv::kFillBands, s);
+                r->long_list.ensure(dtv::sort_scratch_elems(P), s);
+            } catch (...) {
+                cudaMemsetAsync(r->counts.ptr, 0, P * sizeof(uint32_t), s);
+                throw;
+            }
             dtv::launch_fill_order(rfaces, uint32_t(F), r->vfix.ptr, H, r->h_info->nf, r->fill_order.ptr, r->band_scratch.ptr, s);
         };
         // Lists by the walk, then the composite; events of the fill, sort and
