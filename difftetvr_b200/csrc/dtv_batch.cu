@@ -170,9 +170,10 @@ __global__ void __launch_bounds__(256) kb_band_scatter(const BatchView* __restri
     if (g < total) order[base[band] + rank] = uint32_t(g);
 }
 
-// Count or fill of every view's faces.  `ok`: the fill does nothing when *ok is
-// zero.  threads_per_face: of the count (k_raster).
-template <bool FILL, bool WIDE>
+// Count or fill of every view's 32-bit faces; the count lists the 64-bit ones
+// (wide_list[0] = how many, then the items) for kb_raster_listed.  `ok`: the fill
+// does nothing when *ok is zero.  threads_per_face: of the count (k_raster).
+template <bool FILL>
 __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ views, int nviews, u64 total,
                                                  const float4* __restrict__ vproj, const int2* __restrict__ vfix,
                                                  uint32_t* __restrict__ counts, const u64* __restrict__ offsets,
@@ -194,29 +195,25 @@ __global__ void __launch_bounds__(128) kb_raster(const BatchView* __restrict__ v
         const BatchView& bv = views[v];
         set = raster_setup(uint32_t(g - bv.face_base), bv.faces, vfix + bv.vert_base, uint32_t(bv.vert_base),
                            int(bv.W), 0, int(bv.H), bv.pix_base, J);
-        live = set && (J.wide != 0) == WIDE;
+        live = set && J.wide == 0;
     }
     if constexpr (!FILL) {
         if (live)
-            count_face<typename std::conditional<WIDE, long long, int>::type>(J, counts, int(sub), int(per_face));
-        if (!WIDE && wide_list) {
-            // The items of the 64-bit path, for its count and fill launches
-            // (wide_list[0] = how many, then the items).
-            const bool wide = set && J.wide != 0 && sub == 0u;
-            const unsigned m = __ballot_sync(0xffffffffu, wide);
-            if (m) {
-                const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-                uint32_t base = 0;
-                if (lane == leader) base = atomicAdd(wide_list, uint32_t(__popc(m)));
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (wide) wide_list[1 + base + __popc(m & ((1u << lane) - 1u))] = uint32_t(g);
-            }
+            count_face<int>(J, counts, int(sub), int(per_face));
+        const bool wide = set && J.wide != 0 && sub == 0u;
+        const unsigned m = __ballot_sync(0xffffffffu, wide);
+        if (m) {
+            const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+            uint32_t base = 0;
+            if (lane == leader) base = atomicAdd(wide_list, uint32_t(__popc(m)));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (wide) wide_list[1 + base + __popc(m & ((1u << lane) - 1u))] = uint32_t(g);
         }
     } else {
         __shared__ RasterJob jobs[4][32];
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         if (live) jobs[w][lane] = J;
-        raster_warp<FILL, WIDE>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets, records);
+        raster_warp<FILL, false>(jobs[w], __ballot_sync(0xffffffffu, live), lane, vproj, counts, offsets, records);
     }
 }
 
@@ -856,7 +853,7 @@ void launch_kb_count(dtv_batch* b, cudaStream_t s) {
     using namespace dtv;
     const uint32_t per_face = count_threads_per_face(b->tot_faces);
     const unsigned blocks = grid_for(b->tot_faces * per_face, 128, 0x7fffffffu);
-    kb_raster<false, false><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr, b->vfix.ptr,
+    kb_raster<false><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr, b->vfix.ptr,
                                                    b->counts.ptr, nullptr, nullptr, nullptr, nullptr,
                                                    b->wide_list.ptr, per_face);
     kb_raster_listed<false><<<148 * 8, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,
@@ -880,7 +877,7 @@ void launch_kb_fill(dtv_batch* b, const uint32_t* okp, cudaStream_t s) {
                                            b->tot_pixels, b->band_scratch.ptr + kFillBands, b->fill_order.ptr);
         order = b->fill_order.ptr;
     }
-    kb_raster<true, false><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr,
+    kb_raster<true><<<blocks, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->tot_faces, b->vproj.ptr,
                                                   b->vfix.ptr, b->counts.ptr, b->offsets.ptr, b->records.ptr, okp, order, nullptr,
                                                   1u);
     kb_raster_listed<true><<<148, 128, 0, s>>>(b->d_views.ptr, b->nviews, b->vproj.ptr, b->vfix.ptr, b->counts.ptr,

@@ -68,11 +68,11 @@ inline bool many_boundary_faces(uint64_t F) { return F > 64 * 148 * 64; }
 void launch_project(const float* pos, uint32_t V, const CamDev& cam, float4* vproj, int2* vfix, VGeo* vgeo,
                     cudaStream_t s, WalkVertRow* rows = nullptr, uint32_t* clipped = nullptr,
                     uint32_t* wide_list = nullptr);
-// rest: the fill takes only pixels whose counter is not zero.
 // Pixel rows [row0, row1) only (row1 < 0: all rows).  wide_list (u32[F + 1],
 // optional, [0] zero: launch_project): the count lists the faces of the 64-bit path there, and the
 // 64-bit count and the fill that follows (same rows) walk that list instead of
 // setting up every face again; without it both 64-bit launches cover all F.
+// rest (the fill): only pixels whose counter is not zero.
 void launch_raster_count(const uint4* faces, uint32_t F, const float4* vproj, const int2* vfix, int W, int H,
                          uint32_t* counts, cudaStream_t s, int row0 = 0, int row1 = -1,
                          uint32_t* wide_list = nullptr);
@@ -136,8 +136,6 @@ void launch_sort(const unsigned long long* offsets, unsigned long long* records,
 constexpr uint32_t kSortWarpCap = 1024;    // elements per warp list sorted in shared memory
 constexpr uint32_t kSortBlockCap = 16384;  // elements per block-sorted list / chunk of a longer one (128 KiB shared memory)
 
-// gate (optional): nothing is done when *gate is zero.
-// tile: pixel tile of the 128-thread blocks (0: 16 x 8, 1: 32 x 4, 2: 8 x 16).
 // Whether the composite loads ahead (composite_pixel): a pixel's list is a chain
 // of dependent loads, and running ahead of it is worth half the warps when the
 // pixels do not fill the GPU with plain ones anyway, and later only while the
@@ -150,6 +148,8 @@ inline bool composite_ahead(uint64_t V, uint64_t pixels, uint64_t all) {
     if (all < 148 * 1280) return true;
     return pixels < (pixels < 148 * 2560 ? 64 : 6) * V;
 }
+// gate (optional): nothing is done when *gate is zero.
+// tile: pixel tile of the 128-thread blocks (0: 16 x 8, 1: 32 x 4, 2: 8 x 16).
 void launch_composite(const unsigned long long* offsets, const unsigned long long* records, const uint4* faces,
                       const VGeo* vgeo, const float4* colors, uint32_t V, int W, int H, const ShadeDev& sh,
                       float4* image, float* tfinal, uint32_t* term, cudaStream_t s, int row0 = 0, int row1 = -1, int tile = 0,
