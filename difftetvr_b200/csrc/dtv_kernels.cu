@@ -1426,7 +1426,26 @@ __global__ void __launch_bounds__(512) k_loss_l2(const float* __restrict__ img, 
                 make_float4(2.f * scale * d.x, 2.f * scale * d.y, 2.f * scale * d.z, 2.f * scale * d.w);
         add((d.x * d.x + d.y * d.y) + (d.z * d.z + d.w * d.w));
     }
-    for (uint64_t i = 4 * n4 + first; i < n; i += stride) {
+    // One at a time: pointers that are not 16-byte aligned, and the remainder.
+    // Four loads of each array in flight, as with float4 (16 M unaligned values:
+    // 77 us with one, 39 with four; aligned 33).
+    uint64_t i = 4 * n4 + first;
+    for (; i + 3 * stride < n; i += 4 * stride) {
+        float a[4], b[4], q = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            a[k] = img[i + k * stride];
+            b[k] = tgt[i + k * stride];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float d = a[k] - b[k];
+            if (adj) adj[i + k * stride] = 2.f * scale * d;
+            q += d * d;
+        }
+        add(q);
+    }
+    for (; i < n; i += stride) {
         const float d = img[i] - tgt[i];
         if (adj) adj[i] = 2.f * scale * d;
         add(d * d);

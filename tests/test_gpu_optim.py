@@ -88,3 +88,20 @@ def test_batch_loss_of_values_beyond_fp32(value, want):
     br = BatchRenderer([mesh])
     loss = float(br.train_step([View(mesh=0, view_matrix=sc.view, width=48, height=48, fovy=sc.fovy, target=target)]))
     assert (np.isnan(want) and np.isnan(loss)) or loss == want
+
+
+@pytest.mark.parametrize("n", [1, 151552, 3 * 151552, 4 * 151552, 4 * 151552 + 5])   # around whole passes of the grid
+@pytest.mark.parametrize("shift", [0, 1])                                           # 16- and 4-byte aligned
+def test_l2_loss_lengths_and_alignments(n, shift):
+    """Loss within the rounding of 296 FP32 additions of carried sums (1e-5);
+    at this scale the adjoint is the difference itself."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.rand(n + 1, device="cuda", generator=g)[shift:shift + n]
+    y = torch.rand(n + 1, device="cuda", generator=g)[shift:shift + n]
+    adj = torch.empty(n + 1, device="cuda")[shift:shift + n]
+    loss = torch.zeros(1, device="cuda")
+    _lib.call("dtv_loss_l2", x.data_ptr(), y.data_ptr(), n, 0.5, adj.data_ptr(), loss.data_ptr(),
+              torch.cuda.current_stream().cuda_stream)
+    d = x.double() - y.double()
+    assert abs(float(loss) - 0.5 * float((d * d).sum())) <= 1e-5 * 0.5 * float((d * d).sum())
+    assert torch.equal(adj, x - y)
