@@ -778,8 +778,8 @@ int32_t render_common(dtv_renderer* r, const dtv_mesh* mesh, const float* d_posi
                                                    " bytes), over the budget of " + std::to_string(budget) +
                                                    " bytes");
             }
-            r->band_walk = walk_now;
-            if (!walk_now) order_faces();
+            r->band_walk = walk_now && dtv::walk_bands(nf, P, budget / sizeof(u64));
+            if (!r->band_walk) order_faces();
             render_banded(r, mesh, d_colors, cam, sh, d_image, budget / sizeof(u64), s);
             r->adjoint_timed = false;
             r->have_render = true;

@@ -241,6 +241,17 @@ void launch_walk_adjoint(const unsigned long long* b_offsets, const unsigned lon
 constexpr uint64_t kManyLeft = 160;
 constexpr int kWalkRetry = 64;
 inline bool many_left(uint64_t left, uint64_t pixels) { return left > pixels / kManyLeft; }
+// Whether the row bands of a render over its fragment budget are walked: a
+// band of few pixels takes as long as its longest chain of steps (1.4 us each),
+// while fill and sort of few records cost one pass over the faces.  Per list
+// build, walk against fill + sort (us): lists of 97 records on average and bands
+// of 580 pixels +33, of 9,200 -8; 151 records and 600 pixels +85, 9,200 +18,
+// 37,000 -46; 193 records and 570 pixels +226, 3,100 +116, 9,200 -28, 12,300
+// +32, 49,000 -46; 49 records and 640 pixels -11, 25 records -38.
+inline bool walk_bands(uint64_t records, uint64_t pixels, uint64_t band_records) {
+    return double(records) <= 64.0 * double(pixels) ||
+           double(band_records) * double(pixels) >= 12288.0 * double(records);
+}
 // Fills the tables (links: 4 T, start: one per boundary face) from the device
 // topology; *bad (device) is set to a non-zero value when the topology cannot
 // be walked (a tet with a vertex twice, a face of more than two tets).

@@ -80,3 +80,24 @@ def test_autograd_under_budget_matches_fp64_oracle(oracle):
     gp_o, gc_o = oracle.adjoint(fa, sc.pos, sc.col, sc.oracle_camera(oracle), sc.oracle_params(oracle), w)
     assert rel_err(pos.grad.cpu().numpy(), gp_o) < 1e-4
     assert rel_err(col.grad.cpu().numpy(), gc_o) < 1e-4
+
+
+@pytest.mark.parametrize("n,res,bands", [(26, 64, 3), (26, 64, 9), (26, 208, 3), (10, 96, 9)])
+def test_bands_on_both_sides_of_the_walk_rule(n, res, bands):
+    """Long lists in bands of few pixels (filled and sorted), of more than
+    12,288 (walked), and short lists in small bands (walked): the image of the
+    whole lists to the bit, gradients within the order of the atomics."""
+    sc = Scene(n, res, seed=5)
+    mesh, r = sc.make_renderer()
+    w = torch.from_numpy(np.random.default_rng(3).normal(size=(res, res, 4)).astype(np.float32)).cuda()
+    out = []
+    for budget in (0, 1):
+        r.set_fragment_budget_bytes(budget * 8 * (r.get_num_fragments() // bands + 40 * n * res))
+        img = r.render().clone()
+        gp = torch.zeros_like(mesh.get_vertex_positions()).detach()
+        gc = torch.zeros_like(mesh.get_vertex_colors()).detach()
+        r.render_adjoint_into(w, gp, gc)
+        out.append((img, gp.cpu().numpy(), gc.cpu().numpy()))
+    assert r.get_num_bands() > 1
+    assert torch.equal(out[0][0], out[1][0])
+    assert rel_err(out[1][1], out[0][1]) < 1e-5 and rel_err(out[1][2], out[0][2]) < 1e-5
