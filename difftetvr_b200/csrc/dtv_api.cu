@@ -411,36 +411,29 @@ void adjoint_banded(dtv_renderer* r, const dtv_mesh* mesh, const float* d_colors
     check_launch("scatter gradients");
 }
 
-// The mesh's walk tables, if they can be had (walkable); a mesh without them
-// renders all the same.
+// The mesh's walk tables, if they can be had (walkable), in one allocation: the
+// links, the starts, and the word that says whether the topology can be walked.
+// A mesh without them renders all the same.
 void build_walk_tables(dtv_mesh* m) {
     const uint64_t T = m->host.num_cells, Nb = m->bf_global.size();
-    DevBuf<uint32_t> bad;
-    uint32_t h_bad = 1;
-    if (cudaMalloc(&m->d_walk_links, sizeof(uint4) * 4 * T) == cudaSuccess &&
-        cudaMalloc(&m->d_walk_start, sizeof(uint4) * (Nb ? Nb : 1)) == cudaSuccess) {
-        try {
-            bad.ensure(1, nullptr, /*zero_new=*/true);
-            dtv::launch_build_walk(reinterpret_cast<const uint4*>(m->d_cells), uint32_t(T),
-                                   reinterpret_cast<const uint4*>(m->d_tet_faces), m->d_faces,
-                                   reinterpret_cast<const uint2*>(m->d_face_to_tet), m->d_bf_global, uint32_t(Nb),
-                                   m->d_walk_links, m->d_walk_start, bad.ptr, nullptr);
-            check_launch("walk tables");
-            DTV_CK(cudaMemcpy(&h_bad, bad.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-        } catch (const DtvError& e) {
-            if (e.code != DTV_ERR_BUDGET) {
-                bad.release();
-                throw;
-            }
-        }
-        bad.release();
-    } else {
+    if (cudaMalloc(&m->d_walk_links, sizeof(uint4) * (4 * T + Nb + 1)) != cudaSuccess) {
         cudaGetLastError();
+        m->d_walk_links = nullptr;
+        return;
     }
+    m->d_walk_start = m->d_walk_links + 4 * T;
+    uint32_t* bad = &m->d_walk_start[Nb].x;
+    uint32_t h_bad = 1;
+    DTV_CK(cudaMemsetAsync(bad, 0, sizeof(uint32_t), nullptr));
+    dtv::launch_build_walk(reinterpret_cast<const uint4*>(m->d_cells), uint32_t(T),
+                           reinterpret_cast<const uint4*>(m->d_tet_faces), m->d_faces,
+                           reinterpret_cast<const uint2*>(m->d_face_to_tet), m->d_bf_global, uint32_t(Nb),
+                           m->d_walk_links, m->d_walk_start, bad, nullptr);
+    check_launch("walk tables");
+    DTV_CK(cudaMemcpy(&h_bad, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost));
     m->walkable = h_bad == 0;
     if (!m->walkable) {
         cudaFree(m->d_walk_links);
-        cudaFree(m->d_walk_start);
         m->d_walk_links = m->d_walk_start = nullptr;
     }
 }
@@ -549,8 +542,7 @@ int32_t dtv_mesh_destroy(dtv_mesh* m) {
     cudaFree(m->d_tet_flip);
     cudaFree(m->d_bfaces);
     cudaFree(m->d_bf_global);
-    cudaFree(m->d_walk_links);
-    cudaFree(m->d_walk_start);
+    cudaFree(m->d_walk_links);  // the starts lie behind them
     delete m;
     return DTV_OK;
 }
@@ -591,10 +583,11 @@ int32_t dtv_renderer_create(int32_t type, dtv_renderer** out) {
         auto* r = new dtv_renderer();
         r->type = type;
         try {
-            DTV_CK(cudaMallocHost(&r->h_info, sizeof(dtv::ListInfo)));
-            for (auto& l : r->left) {
-                DTV_CK(cudaMallocHost(const_cast<uint32_t**>(&l.n), sizeof(uint32_t) * kLeftSlots));
-                DTV_CK(cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming));
+            // One pinned block: h_info, then the numbers of pixels left.
+            DTV_CK(cudaMallocHost(&r->h_info, sizeof(dtv::ListInfo) + 2 * kLeftSlots * sizeof(uint32_t)));
+            for (int i = 0; i < 2; ++i) {
+                r->left[i].n = reinterpret_cast<uint32_t*>(r->h_info + 1) + i * kLeftSlots;
+                DTV_CK(cudaEventCreateWithFlags(&r->left[i].done, cudaEventDisableTiming));
             }
             for (auto& e : r->ev) DTV_CK(cudaEventCreate(&e));
             DTV_CK(cudaEventCreateWithFlags(&r->ev_info, cudaEventDisableTiming));
@@ -631,10 +624,8 @@ int32_t dtv_renderer_destroy(dtv_renderer* r) {
     if (r->ev_info) cudaEventDestroy(r->ev_info);
     r->walk_verts.release();
     if (r->h_info) cudaFreeHost(r->h_info);
-    for (auto& l : r->left) {
-        if (l.n) cudaFreeHost(const_cast<uint32_t*>(l.n));
+    for (auto& l : r->left)
         if (l.done) cudaEventDestroy(l.done);
-    }
     if (r->h_rowoff) cudaFreeHost(r->h_rowoff);
     for (auto& e : r->ev)
         if (e) cudaEventDestroy(e);

@@ -799,8 +799,8 @@ u64 most_view_rows(u64 nv, u64 V, u64 P) {
 // Pinned words and the events, each by itself: a call that failed half
 // way leaves what it got, and the next one makes the rest.
 void ensure_host(dtv_batch* b) {
-    if (!b->h_info) DTV_CK(cudaMallocHost(&b->h_info, sizeof(dtv::ListInfo)));
-    if (!b->h_done) DTV_CK(cudaMallocHost(&b->h_done, sizeof(dtv::ListInfo)));
+    if (!b->h_info) DTV_CK(cudaMallocHost(&b->h_info, 2 * sizeof(dtv::ListInfo)));
+    b->h_done = b->h_info + 1;
     if (!b->done) DTV_CK(cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming));
     if (!b->staging_free) DTV_CK(cudaEventCreateWithFlags(&b->staging_free, cudaEventDisableTiming));
 }
@@ -1071,7 +1071,6 @@ int32_t dtv_batch_destroy(dtv_batch* b) {
     if (b->h_views) cudaFreeHost(b->h_views);
     if (b->h_slots) cudaFreeHost(b->h_slots);
     if (b->h_info) cudaFreeHost(b->h_info);
-    if (b->h_done) cudaFreeHost(b->h_done);
     if (b->done) cudaEventDestroy(b->done);
     if (b->staging_free) cudaEventDestroy(b->staging_free);
     delete b;
